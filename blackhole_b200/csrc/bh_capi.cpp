@@ -335,7 +335,6 @@ int plan_launch(bh_ctx* ctx, std::vector<FrameParams>& frames, bh_xyz* d_pixels,
     // with long serial step chains, so it runs the spill-free (wide) register
     // variant in small blocks.
     tl.block_resume = 64;
-    tl.reg_variant_resume = 1;
     {
         int bps64 = trace_blocks_per_sm(BH_PRECISION_FP64, tl.block_resume, true);
         tl.grid_resume = ctx->sm_count * (bps64 < 1 ? 1 : bps64);

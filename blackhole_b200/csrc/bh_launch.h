@@ -27,7 +27,6 @@ struct TraceLaunch {
     void* deferred;                  // mixed precision: total_rays deferred records
     int grid_resume;                 // blocks of the binary64 resume launch
     int block_resume;                // its threads per block
-    int reg_variant_resume;          // its register cap (0 tight, 1 wide)
     cudaEvent_t resume_event;        // recorded between the two launches (optional)
     double* jet;                     // jet emission per ray (total_rays), or null when no
                                      // frame of the launch has a jet

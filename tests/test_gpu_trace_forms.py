@@ -1,0 +1,99 @@
+"""The forms of an integration attempt on the GPU.
+
+  - the binary64 right-hand side against Hamilton's equations written out in
+    numpy, for spins on both sides of a = 1 (Delta in factors or not), at
+    ordinary angles and where the metric clamps sin(th);
+  - frames whose rays pass close to the poles, where a stage can move the angle
+    further than angle addition reaches and the attempt takes its general form,
+    against the CPU oracle, in both precisions.
+"""
+import math
+
+import numpy as np
+import pytest
+
+
+from blackhole_b200 import abi  # noqa: E402
+from blackhole_b200.config import M_SUN, Camera, RenderConfig  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+def _rates(a, y):
+    """dy/dlambda of 2 Sigma H = Delta p_r^2 + p_th^2 + (L - a E sin^2)^2 / sin^2 - ((r^2 + a^2) E - a L)^2 / Delta, and
+    the sum of the absolute values of each component's terms."""
+    r, th, pr, pth, E, L = y[:, 1], y[:, 2], y[:, 5], y[:, 6], -y[:, 4], y[:, 7]
+    sn, cs = np.sin(th), np.cos(th)
+    sn = np.where(np.abs(sn) < 1e-9, np.where(sn < 0, -1e-9, 1e-9), sn)
+    s2 = sn * sn
+    S, D = r * r + a * a * cs * cs, r * r - 2 * r + a * a
+    w = r * r + a * a
+    K, P = w * E - a * L, L - a * E * s2
+    B = [D * pr * pr, pth * pth, P * P / s2, -K * K / D]
+    Bs, Ba = sum(B), sum(np.abs(b) for b in B)
+    rows = [[a * P / S, w * K / (D * S)], [D * pr / S], [pth / S], [P / (s2 * S), a * K / (D * S)],
+            [-(r - 1) * pr * pr / S, 2 * r * E * K / (D * S), -(r - 1) * (K / D) ** 2 / S, r * Bs / (S * S)],
+            [-sn * cs * a * a * E * E / S, sn * cs * (L / s2) ** 2 / S, -sn * cs * a * a * Bs / (S * S)]]
+    value = [sum(t) for t in rows]
+    size = [sum(np.abs(t) for t in q) for q in rows]
+    size[4] = size[4] + r * Ba / (S * S)
+    size[5] = size[5] + np.abs(sn * cs) * a * a * Ba / (S * S)
+    return np.stack(value, 1), np.stack(size, 1)
+
+
+@pytest.mark.parametrize("spin", [0.0, 0.9, -0.7, 0.998, 1.0, 1.2])
+def test_binary64_right_hand_side(renderer, spin):
+    rng = np.random.default_rng(11)
+    n = 257
+    y = np.zeros((n, 8))
+    y[:, 1] = 2.5 + np.exp(rng.uniform(-2.0, 6.0, n))
+    y[:, 2] = rng.uniform(0.05, math.pi - 0.05, n)
+    y[:8, 2] = [0.0, 1e-12, math.pi, 1e-4, math.pi - 1e-4, 0.5 * math.pi, 3.0, 0.01]
+    y[:, 4] = -rng.uniform(0.5, 1.5, n)
+    y[:, 5] = rng.normal(0.0, 1.0, n)
+    y[:, 6] = rng.normal(0.0, 6.0, n)
+    y[:, 7] = rng.normal(0.0, 6.0, n)
+    y[:4, 7] = 0.0
+    cfg = RenderConfig(spin=spin, cam=Camera(r=50.0, theta=1.0), width=4, height=4, disc_enabled=False, star_count=0,
+                       quiet=True)
+    got = renderer.eval(cfg, abi.EVAL_RHS, y)[:, [0, 1, 2, 3, 5, 6]]
+    want, size = _rates(spin, y)
+    # each term is a product of at most a dozen rounded factors; Delta in the
+    # expanded form loses (r^2 + 1) / Delta <= 20 roundings at r >= 2.6, and
+    # sin(th) at pi - 1e-4 one part in 1e-4 of an ulp of pi per factor
+    tol = 64 * 2.0 ** -53 * (20.0 + np.pi / np.maximum(np.abs(np.sin(y[:, 2])), 1e-9))
+    ok = np.abs(got - want) <= tol[:, None] * size
+    ok |= np.abs(np.sin(y[:, 2]))[:, None] < 1e-9      # there sin is the clamp's: compared below
+    assert ok.all(), np.argwhere(~ok)[:5]
+    # where sin(th) is clamped the value is finite (and sign and size are the clamp's)
+    clamped = np.abs(np.sin(y[:, 2])) < 1e-9
+    assert clamped.sum() >= 3 and np.isfinite(got[clamped]).all()
+    assert np.allclose(got[clamped][:, :3], want[clamped][:, :3], rtol=1e-9, atol=0.0)
+
+
+@pytest.mark.parametrize("theta_deg,spin,precision", [
+    (theta, spin, p) for theta, spin in ((0.3, 0.9), (179.6, 0.998), (2.0, 0.0), (90.0, 1.0))
+    for p in (abi.PRECISION_FP64, abi.PRECISION_MIXED)
+    # at a = 1 the mixed path's captured rays run out of steps: Delta has a
+    # double root there, and no hand-over radius
+    if not (spin == 1.0 and p == abi.PRECISION_MIXED)])
+def test_rays_past_the_poles(renderer, orc, theta_deg, spin, precision):
+    cfg = RenderConfig(
+        M_kg=4.3e6 * M_SUN, spin=spin,
+        cam=Camera(r=40.0, theta=math.radians(theta_deg), phi=0.7, fov=0.9), width=37, height=29, sqrt_spp=1,
+        disc_r_out=20.0, rtol=1e-8, atol=1e-10, r_escape=220.0, star_count=0, quiet=True,
+    )
+    chk, _ = orc.trace_rays(cfg)
+    cfg.precision = precision
+    got = renderer.trace_rays(cfg)
+    same = got["what"] == chk["what"]
+    # the suite's bounds for a scene against the oracle: at most two rays of
+    # another class; g and direction to 1e-6 (binary64) or the mixed targets
+    assert (~same).sum() <= 2
+    g_tol, d_tol = (1e-6, 1e-6) if precision == abi.PRECISION_FP64 else (1e-3, 1e-4)
+    disc = same & (chk["what"] == abi.HIT_DISC) & (chk["g"] > 0)
+    sky = same & (chk["what"] == abi.HIT_SKY)
+    assert disc.sum() + sky.sum() > 500
+    assert np.quantile(np.abs(got["g"][disc] / chk["g"][disc] - 1.0), 0.95) <= g_tol
+    d = np.linalg.norm(got["dir"][sky] - chk["dir"][sky], axis=1)
+    assert np.quantile(d, 0.95) <= d_tol
