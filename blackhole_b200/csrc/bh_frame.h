@@ -98,6 +98,12 @@ struct FrameParams {
     double jet_z_base, jet_z_top, jet_R_base, jet_k, jet_gamma_max, jet_z_sat;
     double jet_alpha, jet_u_peak, jet_u_wid, jet_spine, jet_spine_wid, jet_zeta;
     double jet_Omega_F, jet_j_nu0, jet_r_bound;
+    double jet_inv_zb;               // 1 / z_base
+    double jet_ck;                   // (z_base / z_sat)^k
+    double jet_inv_gb;               // 1 / Gamma(z_base)
+    float jet_f_cut;                 // u_cut R_base / z_base^k: times z^k, the radius beyond which the
+                                     // profile is below its cut-off for certain; < 0: not known
+    float jet_pad;
     double jet_col[3];               // powerlaw_xyz(alpha) (spectrum.cpp:77-92)
 };
 

@@ -150,6 +150,7 @@ struct Lane {
     int steps, tries, attempts;
     int att0;                // attempts already counted against the budget
     double jet;              // jet emission picked up so far (jet kernels only)
+    float jet_z, jet_rho;    // cylindrical z and radius at y, binary32 (jet kernels only)
     int gid, frame;
     int mirror;              // mixed: the state holds pi - th and -p_th
     int factored;
@@ -180,6 +181,13 @@ __device__ __forceinline__ void set_horizons(const FrameParams& F, Lane<P>& L) {
 __device__ __forceinline__ unsigned abs_hi(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
 constexpr unsigned kMaxShiftHi = 0x3fd00000u;   // of kMaxShift = 1/4
 constexpr unsigned kMinSinHi = 0x3e112e0bu;     // of the metric's clamp 1e-9
+
+// Cylindrical (z, rho) of (r, th), for the test of a step against the jet.
+template <class P>
+__device__ __forceinline__ void cylindrical(const Lane<P>& L, float r, float sn, float cs, float* z, float* rho) {
+    *z = r * cs;
+    *rho = sqrtf(fmaf(r, r, (float)L.a2R)) * fabsf(sn);
+}
 
 template <class P>
 struct Aux {
@@ -773,6 +781,7 @@ __device__ bool start_ray(const TraceArgs& A, Lane<P>& L, long long id) {
     }
     L.c0 = ax.cs;
     L.sn0 = ax.sn;
+    if constexpr (JET) cylindrical(L, (float)L.y[1], (float)L.sn0, (float)L.c0, &L.jet_z, &L.jet_rho);
     return true;
 }
 
@@ -1127,19 +1136,33 @@ __device__ bool attempt(const TraceArgs& A, Lane<P>& L) {
             }
         }
     }
+    float jet_z1 = 0.f, jet_rho1 = 0.f;
+    if constexpr (JET) cylindrical(L, (float)yn[1], (float)ax7.sn, (float)ax7.cs, &jet_z1, &jet_rho1);
     if (JET && s_jet > 0.0) {
         // Optically thin jet emission along the step (render.cpp:150-152,
-        // 107-122): skipped unless the chord passes within r_bound of the hole.
-        double q0[3], q1[3];
-        bl_cartesian(F.a, (double)L.y[1], (double)L.y[2], (double)L.y[3], q0);
-        bl_cartesian(F.a, rn, (double)yn[2], (double)yn[3], q1);
-        if (segment_distance_to_origin(q0, q1) < F.jet_r_bound) {
-            const DenseC cr = coef(1);
-            const DenseC ct = coef(2);
-            const DenseC cpr = coef(4);
-            const DenseC cpt = coef(5);
-            L.jet += jet_step_integral(F, cr, ct, cpr, cpt, (double)L.E, (double)L.Lz, hd, s_jet);
+        // 107-122): skipped unless the chord passes within r_bound of the hole
+        // (certainly so where an end of it does).
+        if (jet_may_touch(F, L.jet_z, L.jet_rho, jet_z1, jet_rho1, (float)(yn[3] - L.y[3]))) {
+            const double r_near = dminr((double)L.y[1], rn);
+            bool near = r_near * r_near + F.a2 < F.jet_r_bound * F.jet_r_bound;
+            if (!near) {
+                double q0[3], q1[3];
+                bl_cartesian(F.a, (double)L.y[1], (double)L.y[2], (double)L.y[3], q0);
+                bl_cartesian(F.a, rn, (double)yn[2], (double)yn[3], q1);
+                near = segment_distance_to_origin(q0, q1) < F.jet_r_bound;
+            }
+            if (near) {
+                const DenseC cr = coef(1);
+                const DenseC ct = coef(2);
+                const DenseC cpr = coef(4);
+                const DenseC cpt = coef(5);
+                L.jet += jet_step_integral(F, cr, ct, cpr, cpt, (double)L.E, (double)L.Lz, hd, s_jet);
+            }
         }
+    }
+    if constexpr (JET) {
+        L.jet_z = jet_z1;
+        L.jet_rho = jet_rho1;
     }
     if (what < 0 && (P::kMixed ? yn[1] > r_escape_f : rn > F.r_escape)) what = BH_HIT_SKY;   // render.cpp:247-251
 
