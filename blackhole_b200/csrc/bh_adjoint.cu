@@ -1,8 +1,13 @@
-// bh_adjoint.cu - The discrete-adjoint kernel and its reductions (sm_100a).
+// bh_adjoint.cu - The discrete-adjoint kernels and reductions (sm_100a).
 //
-// adjoint_kernel: one thread per job at a time, jobs handed out by a global
-// atomic counter; each thread owns `checkpoint_slots` checkpoint states in
-// global memory for the job it is working on (bh_adjoint.cuh has the per-ray
+// adjoint_select_kernel: one thread per ray.  The render's hit record says
+// which rays have a gradient at all: those that ended on the disc or saw a sky
+// that varies at their direction.  A captured ray, or one that met the uniform
+// background, is done here; the others are listed.
+//
+// adjoint_kernel: a warp takes 32 jobs at a time from a global atomic counter;
+// each lane owns `checkpoint_slots` stored states in global memory, interleaved
+// over the warp, for the job it is working on (bh_adjoint.cuh has the per-ray
 // algorithm).  A ray's loss weight is 2 (Y_pixel - target) / S^2 for
 // Loss = sum over pixels of (Y_pixel - target)^2, Y_pixel being the sample
 // mean of the rendered frame (bh_gpu_render's output).
@@ -36,14 +41,19 @@ namespace bhg {
 
 namespace {
 
-constexpr int kAdjBlock = 128;
+using adj::kAdjBlock;
+constexpr size_t kAdjShared = sizeof(double) * adj::kScratch * kAdjBlock;
+// 8 warps per SM with 255 registers; 10 and 12 with 200 and 168 took 5 and 9% longer
+// per 512^2 gradient, 6 the same.
+constexpr int kAdjBlocksPerSm = 4;
 constexpr int kReduceThreads = 1024;
+static_assert(adj::kCkWords == kAdjSlotWords, "kAdjSlotWords is stale");
 
 // Candidate selection: one thread per sample (work order); each of its first
 // two equatorial crossings, as the render recorded them, is compared with the
 // same crossing of its four neighbours in the W S x H S sample grid
 // (adj::edge_mask).
-__global__ void __launch_bounds__(256) edge_candidates_kernel(const AdjointLaunch L) {
+__global__ void __launch_bounds__(256) edge_candidates_kernel(const __grid_constant__ AdjointLaunch L) {
     const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= L.n_rays) return;
     const int S = L.frame.S;
@@ -57,7 +67,7 @@ __global__ void __launch_bounds__(256) edge_candidates_kernel(const AdjointLaunc
     const int gy = py * S + k / S;
     const int GW = W * S, GH = H * S;
     for (int j = 0; j < 2; ++j) {
-        const double rc = L.xing_r[2 * id + j];
+        const double rc = fabs(L.xing_r[2 * id + j]);
         if (rc == 0.0) break;
         double dmax = 0.0;
         #pragma unroll
@@ -66,7 +76,7 @@ __global__ void __launch_bounds__(256) edge_candidates_kernel(const AdjointLaunc
             const int ny = gy + (n == 2) - (n == 3);
             if (nx < 0 || nx >= GW || ny < 0 || ny >= GH) continue;
             const long long nid = pixel_index(W, H, nx / S, ny / S) * SS + (ny % S) * S + nx % S;
-            const double rn = L.xing_r[2 * nid + j];
+            const double rn = fabs(L.xing_r[2 * nid + j]);
             if (rn == 0.0) continue;
             const double d = fabs(rc - rn);
             if (d > dmax) dmax = d;
@@ -79,79 +89,125 @@ __global__ void __launch_bounds__(256) edge_candidates_kernel(const AdjointLaunc
     }
 }
 
+// The pixel (index, row-major) and sample of a ray (work order).
+__device__ __forceinline__ long long ray_pixel(const AdjointLaunch& L, long long id, int* px, int* py, int* k) {
+    const int SS = L.frame.S * L.frame.S;
+    const long long pixel = id / SS;
+    *k = (int)(id - pixel * SS);
+    pixel_xy(L.frame.width, L.frame.height, pixel, px, py);
+    return (long long)*py * L.frame.width + *px;
+}
+
+// What the render's hit record says of each ray: its class counts, whether
+// its image is of order three or higher, and whether it has a gradient.
+// Rays without one get their (zero) gradient and their luminance here; the
+// rest are listed, 32 consecutive rays at a time.
+__global__ void __launch_bounds__(256) adjoint_select_kernel(const __grid_constant__ AdjointLaunch L) {
+    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int SS = L.frame.S * L.frame.S;
+    bool listed = false;
+    unsigned steps = 0;
+    int what = BH_HIT_EXHAUSTED;
+    bool high = false;
+    if (id < L.n_rays) {
+        int px, py, k;
+        const long long pix = ray_pixel(L, id, &px, &py, &k);
+        const long long o = pix * SS + k;
+        const HitRecord& h = L.hits[id];
+        what = h.what;
+        steps = (unsigned)h.steps;
+        const bool event = what == BH_HIT_DISC || what == BH_HIT_SKY;
+        high = event && L.xing_r[2 * id + 1] < 0.0;
+        const double w = 2.0 * (L.pixels[pix].y - (double)L.target[pix]) / (double)SS;
+        double Y = 0.0;
+        if (what == BH_HIT_DISC) {
+            listed = w != 0.0;
+            if (!listed && L.ray_Y)
+                Y = adj::disc_luminance(L.frame, L.X, L.sky.table, h.y[1], -h.y[4], h.y[7]).v;
+        } else if (what == BH_HIT_SKY) {
+            const double y6[6] = {h.y[0], h.y[1], h.y[2], h.y[3], h.y[5], h.y[6]};
+            double d[3], gY[3];
+            if (adj::escape_direction_value(y6, -h.y[4], h.y[7], L.frame.a, d)) {
+                Y = adj::sky_luminance(L.sky, L.frame, d, gY);
+                listed = w != 0.0 && (gY[0] != 0.0 || gY[1] != 0.0 || gY[2] != 0.0);
+            }
+        }
+        L.high_order[o] = high ? 1 : 0;
+        if (!listed) {
+            #pragma unroll
+            for (int q = 0; q < 4; ++q) L.ray_grad[o * 4 + q] = 0.0;
+            if (L.ray_Y) L.ray_Y[o] = Y;
+        }
+    }
+    const unsigned lane = threadIdx.x & 31;
+    const unsigned m = __ballot_sync(kFull, listed);
+    const unsigned nd = __popc(__ballot_sync(kFull, what == BH_HIT_DISC));
+    const unsigned ns = __popc(__ballot_sync(kFull, what == BH_HIT_SKY));
+    const unsigned nh = __popc(__ballot_sync(kFull, high));
+    const unsigned st = __reduce_add_sync(kFull, steps);
+    unsigned long long base = 0;
+    if (lane == 0) {
+        if (m) base = atomicAdd(&L.counters[10], (unsigned long long)__popc(m));
+        if (st) atomicAdd(&L.counters[1], (unsigned long long)st);
+        if (nd) atomicAdd(&L.counters[3], (unsigned long long)nd);
+        if (ns) atomicAdd(&L.counters[4], (unsigned long long)ns);
+        if (nh) atomicAdd(&L.counters[9], (unsigned long long)nh);
+    }
+    base = __shfl_sync(kFull, base, 0);
+    if (listed) L.rays[base + __popc(m & ((1u << lane) - 1u))] = (int)id;
+}
+
 // One queue of jobs: first the edge candidates (each a forward pass to its
 // crossing, the continuation past it and a reverse sweep: the longest jobs),
-// then the rays.  Each thread owns `checkpoint_slots` checkpoint states for
-// the job it is working on; results go to per-ray and per-crossing slots, so
-// the sums do not depend on which thread took which job.
-__global__ void __launch_bounds__(kAdjBlock) adjoint_kernel(const AdjointLaunch L) {
-    const long long slot = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// then the listed rays.  Results go to per-ray and per-crossing slots, so the
+// sums do not depend on which lane took which job.
+__global__ void __launch_bounds__(kAdjBlock, kAdjBlocksPerSm) adjoint_kernel(const __grid_constant__ AdjointLaunch L) {
+    const int lane = threadIdx.x & 31;
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int slots = L.X.checkpoint_slots;
-    double* ck = L.ckpt + slot * slots * 8;
-    const int S = L.frame.S;
-    const int SS = S * S;
-    const int W = L.frame.width, H = L.frame.height;
-    const unsigned long long n_cand = L.counters[6];
-    unsigned long long steps = 0, replay = 0, disc = 0, sky = 0, max_int = 0, n_high = 0;
-    unsigned long long edge_steps = 0, edge_cells = 0;
+    double* ck = L.ckpt + warp * slots * adj::kCkWords * 32 + lane;
+    const int SS = L.frame.S * L.frame.S;
+    const unsigned long long n_cand = L.counters[6], n_jobs = n_cand + L.counters[10];
+    unsigned long long replay = 0, max_int = 0, edge_steps = 0, edge_cells = 0;
     for (;;) {
-        const unsigned long long job = atomicAdd(&L.counters[0], 1ull);
+        unsigned long long job = 0;
+        if (lane == 0) job = atomicAdd(&L.counters[0], 32ull);
+        job = __shfl_sync(kFull, job, 0);
+        if (job >= n_jobs) break;
+        job += lane;
+        int px, py, k;
         if (job < n_cand) {
             const unsigned long long c = L.cand[job];
             const long long xs = (long long)(c >> 2);     // 2 * ray + crossing
-            const long long id = xs >> 1;
-            const long long pixel = id / SS;
-            const int k = (int)(id - pixel * SS);
-            int px, py;
-            pixel_xy(W, H, pixel, &px, &py);
-            const long long pix = (long long)py * W + px;
+            const long long pix = ray_pixel(L, xs >> 1, &px, &py, &k);
             const double w = 2.0 * (L.pixels[pix].y - (double)L.target[pix]);
             double out[3];
             int n_cells = 0;
             edge_steps += (unsigned long long)adj::edge_sample(L.frame, L.X, L.sky, px, py, k, (int)(xs & 1) + 1,
-                                                               (int)(c & 3ull), w, ck, slots, out, &n_cells);
+                                                               (int)(c & 3ull), w, ck, slots, 32, out, &n_cells);
             edge_cells += (unsigned long long)n_cells;
             L.edge_out[3 * xs] = out[0];
             L.edge_out[3 * xs + 1] = out[1];
             L.edge_out[3 * xs + 2] = out[2];
-            continue;
+        } else if (job < n_jobs) {
+            const long long id = L.rays[job - n_cand];
+            const long long pix = ray_pixel(L, id, &px, &py, &k);
+            const double w = 2.0 * (L.pixels[pix].y - (double)L.target[pix]) / (double)SS;
+            adj::RayResult res;
+            adj::adjoint_ray(L.frame, L.X, L.sky, id, w, ck, slots, 32, false, &res);
+            const long long o = pix * SS + k;
+            #pragma unroll
+            for (int q = 0; q < 4; ++q) L.ray_grad[o * 4 + q] = res.grad[q];
+            if (L.ray_Y) L.ray_Y[o] = res.Y;
+            replay += (unsigned long long)res.replay;
+            if ((unsigned long long)res.interval > max_int) max_int = (unsigned long long)res.interval;
         }
-        const long long id = (long long)(job - n_cand);
-        if (id >= L.n_rays) break;
-        const long long pixel = id / SS;
-        const int k = (int)(id - pixel * SS);
-        int px, py;
-        pixel_xy(W, H, pixel, &px, &py);
-        const long long pix = (long long)py * W + px;
-        const double w = 2.0 * (L.pixels[pix].y - (double)L.target[pix]) / (double)SS;
-        adj::RayResult res;
-        adj::Crossings xr;
-        xr.n = 0;
-        xr.count = 0;
-        xr.r[0] = xr.r[1] = 0.0;
-        xr.step[0] = xr.step[1] = 0;
-        adj::adjoint_ray(L.frame, L.X, L.sky, id, w, ck, slots, false, &res, &xr);
-        const long long o = pix * SS + k;
-        const bool high = xr.count >= 3 && (res.what == BH_HIT_DISC || res.what == BH_HIT_SKY);
-        L.high_order[o] = high ? 1 : 0;
-        n_high += high ? 1ull : 0ull;
-        #pragma unroll
-        for (int q = 0; q < 4; ++q) L.ray_grad[o * 4 + q] = res.grad[q];
-        if (L.ray_Y) L.ray_Y[o] = res.Y;
-        steps += (unsigned long long)res.steps;
-        replay += (unsigned long long)res.replay;
-        disc += (res.what == BH_HIT_DISC) ? 1ull : 0ull;
-        sky += (res.what == BH_HIT_SKY) ? 1ull : 0ull;
-        if ((unsigned long long)res.interval > max_int) max_int = (unsigned long long)res.interval;
+        __syncwarp();
     }
-    atomicAdd(&L.counters[1], steps);
-    atomicAdd(&L.counters[2], replay);
-    atomicAdd(&L.counters[3], disc);
-    atomicAdd(&L.counters[4], sky);
-    atomicMax(&L.counters[5], max_int);
-    atomicAdd(&L.counters[7], edge_steps);
-    atomicAdd(&L.counters[8], edge_cells);
-    atomicAdd(&L.counters[9], n_high);
+    if (replay) atomicAdd(&L.counters[2], replay);
+    if (max_int) atomicMax(&L.counters[5], max_int);
+    if (edge_steps) atomicAdd(&L.counters[7], edge_steps);
+    if (edge_cells) atomicAdd(&L.counters[8], edge_cells);
 }
 
 __global__ void __launch_bounds__(kReduceThreads)
@@ -188,10 +244,12 @@ adjoint_reduce_kernel(const double* __restrict__ grad, const double* __restrict_
 
 }  // namespace
 
+int adjoint_block_size() { return kAdjBlock; }
+
 int adjoint_blocks_per_sm(int block_size) {
     int n = 0;
     if (block_size != kAdjBlock) return 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, adjoint_kernel, block_size, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, adjoint_kernel, block_size, kAdjShared);
     return n;
 }
 
@@ -199,7 +257,8 @@ cudaError_t launch_adjoint(const AdjointLaunch& L, cudaStream_t stream) {
     if (L.block != kAdjBlock) return cudaErrorInvalidValue;
     if (L.n_rays > 0) {
         edge_candidates_kernel<<<(unsigned)((L.n_rays + 255) / 256), 256, 0, stream>>>(L);
-        adjoint_kernel<<<L.grid, L.block, 0, stream>>>(L);
+        adjoint_select_kernel<<<(unsigned)((L.n_rays + 255) / 256), 256, 0, stream>>>(L);
+        adjoint_kernel<<<L.grid, L.block, kAdjShared, stream>>>(L);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;

@@ -6,17 +6,18 @@
 //
 //   1. forward: the ray is integrated with the render path's DP5(4) scheme,
 //      PI controller, step limiter and events (render.cpp:69-260,
-//      geodesic.h:123-204); the state (y, h, controller memory) after every
-//      `interval` accepted steps is stored in the ray's checkpoint slots.
-//      When the slots are full every second checkpoint is dropped and the
-//      interval doubles, so memory stays bounded for any step count;
+//      geodesic.h:123-204); the state (y, h, controller memory) before each
+//      accepted step and the step's size are stored in the ray's slots.
+//      When the slots are full every second state is dropped and the interval
+//      between the stored ones doubles, so memory stays bounded for any step
+//      count;
 //   2. seed: the shading of the hit (disc: Novikov-Thorne temperature,
 //      Keplerian redshift, blackbody table, disc.h:94-126, render.cpp:31-34,
 //      spectrum.cpp:123-134; sky: the escape direction and the star field,
 //      render.cpp:15-26, scene.h:111-158) is differentiated in forward mode
 //      (dual numbers) with respect to the hit state and the parameters;
-//   3. reverse: segment by segment from the last, the accepted steps are
-//      replayed from their checkpoint and the adjoint state is carried back
+//   3. reverse: step by step from the last (replayed from the stored states
+//      where those were thinned), the adjoint state is carried back
 //      through each DP5 step in reverse (the vector-Jacobian products of its
 //      six stages), with the accepted step sizes held fixed: the discrete
 //      adjoint of the step sequence the forward pass took.  The disc-crossing
@@ -41,6 +42,7 @@
 
 #include <cmath>
 #include <cstdint>
+#include <type_traits>
 
 #include "../../include/bh_gpu.h"
 #include "bh_adjoint.h"
@@ -122,27 +124,55 @@ struct RayC {
 //   2 Sigma H = Delta p_r^2 + p_th^2 + (L_z - a E sin^2)^2 / sin^2
 //               - ((r^2 + a^2) E - a L_z)^2 / Delta,
 // at sin(th) = sn, cos(th) = cs, with one reciprocal (of Sigma Delta sin^2)
-// for the three quotients.  d = (dt, dr, dth, dphi, dp_r, dp_th) / dlambda.
-__host__ __device__ BHA_NOINLINE void rhs6(const RayC& c, double r, double sn, double cs, double pr, double pth,
-                                           double d[6]) {
+// for the three quotients.  RhsMid holds what the derivatives and their
+// vector-Jacobian products share.
+struct RhsMid {
+    double sn, sn2, D, iS, iD, isn2, r2a2, K, Lp, KiD, B;
+};
+__host__ __device__ __forceinline__ RhsMid rhs_mid(const RayC& c, double r, double sn, double cs, double pr,
+                                                   double pth) {
+    RhsMid m;
     if (fabs(sn) < 1e-9) sn = (sn < 0.0) ? -1e-9 : 1e-9;   // kerr.h:51
-    const double sn2 = sn * sn, cs2 = cs * cs, r2 = r * r;
+    m.sn = sn;
+    m.sn2 = sn * sn;
+    const double cs2 = cs * cs, r2 = r * r;
     const double S = r2 + c.a2 * cs2;
-    const double D = c.factored ? (r - c.rp) * (r - c.rm) : (r2 - 2.0 * r + c.a2);
-    const double inv = rcp_nr(S * D * sn2);
-    const double iS = inv * D * sn2, iD = inv * S * sn2, isn2 = inv * S * D;
-    const double r2a2 = r2 + c.a2;
-    const double K = r2a2 * c.E - c.a * c.Lz;
-    const double Lp = c.Lz - c.a * c.E * sn2;
-    const double KiD = K * iD;
-    const double B = D * pr * pr + pth * pth + Lp * Lp * isn2 - K * KiD;
+    m.D = c.factored ? (r - c.rp) * (r - c.rm) : (r2 - 2.0 * r + c.a2);
+    const double SD = S * m.D;
+    const double inv = rcp_nr(SD * m.sn2);
+    m.iS = inv * m.D * m.sn2;
+    m.iD = inv * S * m.sn2;
+    m.isn2 = inv * SD;
+    m.r2a2 = r2 + c.a2;
+    m.K = m.r2a2 * c.E - c.a * c.Lz;
+    m.Lp = c.Lz - c.a * c.E * m.sn2;
+    m.KiD = m.K * m.iD;
+    m.B = m.D * pr * pr + pth * pth + m.Lp * m.Lp * m.isn2 - m.K * m.KiD;
+    return m;
+}
+// (dr, dth, dp_r, dp_th) / dlambda: the components the stages depend on.
+__host__ __device__ __forceinline__ void rhs4(const RayC& c, double r, double sn, double cs, double pr, double pth,
+                                              double d[4]) {
+    const RhsMid m = rhs_mid(c, r, sn, cs, pr, pth);
     const double Dr = 2.0 * r - 2.0;
-    d[0] = iS * (c.a * Lp + r2a2 * KiD);
-    d[1] = D * pr * iS;
-    d[2] = pth * iS;
-    d[3] = iS * (Lp * isn2 + c.a * KiD);
-    d[4] = -0.5 * iS * (Dr * pr * pr - 4.0 * r * c.E * KiD + Dr * KiD * KiD - 2.0 * r * B * iS);
-    d[5] = -sn * cs * iS * (c.a2 * c.E * c.E - c.Lz * c.Lz * isn2 * isn2 + c.a2 * B * iS);
+    d[0] = m.D * pr * m.iS;
+    d[1] = pth * m.iS;
+    d[2] = -0.5 * m.iS * (Dr * (pr * pr + m.KiD * m.KiD) - 2.0 * r * (2.0 * c.E * m.KiD + m.B * m.iS));
+    const double q = c.Lz * m.isn2;
+    d[3] = -m.sn * cs * m.iS * (c.a2 * (c.E * c.E + m.B * m.iS) - q * q);
+}
+// d = (dt, dr, dth, dphi, dp_r, dp_th) / dlambda.
+__host__ __device__ __forceinline__ void rhs6(const RayC& c, double r, double sn, double cs, double pr, double pth,
+                                              double d[6]) {
+    const RhsMid m = rhs_mid(c, r, sn, cs, pr, pth);
+    const double Dr = 2.0 * r - 2.0;
+    d[0] = m.iS * (c.a * m.Lp + m.r2a2 * m.KiD);
+    d[1] = m.D * pr * m.iS;
+    d[2] = pth * m.iS;
+    d[3] = m.iS * (m.Lp * m.isn2 + c.a * m.KiD);
+    d[4] = -0.5 * m.iS * (Dr * (pr * pr + m.KiD * m.KiD) - 2.0 * r * (2.0 * c.E * m.KiD + m.B * m.iS));
+    const double q = c.Lz * m.isn2;
+    d[5] = -m.sn * cs * m.iS * (c.a2 * (c.E * c.E + m.B * m.iS) - q * q);
 }
 
 // The right-hand side at angle th; *sn_out, *cs_out receive sin(th), cos(th).
@@ -158,34 +188,27 @@ __host__ __device__ __forceinline__ void rhs6_th(const RayC& c, double r, double
 // Vector-Jacobian product of rhs6 at (r, th, p_r, p_th) given sin(th) = sn
 // and cos(th) = cs: for db = dLoss/d(d), adds dLoss/d(r, th, p_r, p_th) into
 // g[0..3] and dLoss/d(E, L_z, a) into *Eb, *Lzb, *ab.  Reverse-mode
-// differentiation of the expressions of rhs6, written out.
-__host__ __device__ BHA_NOINLINE void rhs6_vjp(const RayC& c, double r, double sn, double cs, double pr, double pth,
-                                               const double db[6], double g[4], double* Eb, double* Lzb,
-                                               double* ab) {
-    const double sn_true = sn;
-    const bool clamped = fabs(sn) < 1e-9;
-    if (clamped) sn = (sn < 0.0) ? -1e-9 : 1e-9;
+// differentiation of the expressions of rhs6, written out.  TIME: whether
+// db[0] can be non-zero; nothing the loss sees depends on t, so the reverse
+// sweep runs without.
+template <bool TIME>
+__host__ __device__ __forceinline__ void rhs_vjp(const RayC& c, double r, double sn_true, double cs, double pr,
+                                                 double pth, const double db[6], double g[4], double* Eb,
+                                                 double* Lzb, double* ab) {
+    const RhsMid m = rhs_mid(c, r, sn_true, cs, pr, pth);
+    const bool clamped = fabs(sn_true) < 1e-9;
     const double a = c.a, a2 = c.a2, E = c.E, Lz = c.Lz;
-    const double sn2 = sn * sn, cs2 = cs * cs, r2 = r * r;
-    const double S = r2 + a2 * cs2;
-    const double D = c.factored ? (r - c.rp) * (r - c.rm) : (r2 - 2.0 * r + a2);
-    const double inv = rcp_nr(S * D * sn2);
-    const double iS = inv * D * sn2, iD = inv * S * sn2, isn2 = inv * S * D;
-    const double r2a2 = r2 + a2;
-    const double K = r2a2 * E - a * Lz;
-    const double Lp = Lz - a * E * sn2;
-    const double KiD = K * iD;
-    const double B = D * pr * pr + pth * pth + Lp * Lp * isn2 - K * KiD;
+    const double sn = m.sn, sn2 = m.sn2, cs2 = cs * cs, D = m.D, iS = m.iS, iD = m.iD, isn2 = m.isn2;
+    const double r2a2 = m.r2a2, K = m.K, Lp = m.Lp, KiD = m.KiD, B = m.B;
     const double Dr = 2.0 * r - 2.0;
-    const double X0 = a * Lp + r2a2 * KiD;
+    const double BiS = B * iS, q = Lz * isn2, pk = pr * pr + KiD * KiD;
     const double X3 = Lp * isn2 + a * KiD;
-    const double X4 = Dr * pr * pr - 4.0 * r * E * KiD + Dr * KiD * KiD - 2.0 * r * B * iS;
-    const double X5 = a2 * E * E - Lz * Lz * isn2 * isn2 + a2 * B * iS;
+    const double X4 = Dr * pk - 2.0 * r * (2.0 * E * KiD + BiS);
+    const double X5 = a2 * (E * E + BiS) - q * q;
     const double P5 = -sn * cs;
 
     // outputs
-    double b_iS = db[0] * X0 + db[1] * D * pr + db[2] * pth + db[3] * X3 - 0.5 * db[4] * X4 + db[5] * P5 * X5;
-    const double bX0 = db[0] * iS;
+    double b_iS = db[1] * D * pr + db[2] * pth + db[3] * X3 - 0.5 * db[4] * X4 + db[5] * P5 * X5;
     double bD = db[1] * pr * iS;
     double bpr = db[1] * D * iS;
     double bpth = db[2] * iS;
@@ -193,74 +216,74 @@ __host__ __device__ BHA_NOINLINE void rhs6_vjp(const RayC& c, double r, double s
     const double bX4 = -0.5 * db[4] * iS;
     const double bP5 = db[5] * iS * X5;
     const double bX5 = db[5] * P5 * iS;
-    // X0 = a Lp + r2a2 KiD
-    double ba = bX0 * Lp;
-    double bLp = bX0 * a;
-    double br2a2 = bX0 * KiD;
-    double bKiD = bX0 * r2a2;
     // X3 = Lp isn2 + a KiD
-    bLp += bX3 * isn2;
+    double bLp = bX3 * isn2;
     double bisn2 = bX3 * Lp;
-    ba += bX3 * KiD;
-    bKiD += bX3 * a;
-    // X4 = Dr pr^2 - 4 r E KiD + Dr KiD^2 - 2 r B iS
-    const double bDr = bX4 * (pr * pr + KiD * KiD);
-    bpr += bX4 * 2.0 * Dr * pr;
-    double br = bX4 * (-4.0 * E * KiD - 2.0 * B * iS);
-    double bE = bX4 * (-4.0 * r * KiD);
-    bKiD += bX4 * (-4.0 * r * E + 2.0 * Dr * KiD);
-    double bB = bX4 * (-2.0 * r * iS);
-    b_iS += bX4 * (-2.0 * r * B);
-    // X5 = a2 E^2 - Lz^2 isn2^2 + a2 B iS
-    double ba2 = bX5 * (E * E + B * iS);
-    bE += bX5 * 2.0 * a2 * E;
-    double bLz = bX5 * (-2.0 * Lz * isn2 * isn2);
-    bisn2 += bX5 * (-2.0 * Lz * Lz * isn2);
-    bB += bX5 * a2 * iS;
-    b_iS += bX5 * a2 * B;
+    double ba = bX3 * KiD;
+    double bKiD = bX3 * a;
+    double br2a2 = 0.0;
+    if (TIME) {
+        // X0 = a Lp + r2a2 KiD
+        b_iS += db[0] * (a * Lp + r2a2 * KiD);
+        const double bX0 = db[0] * iS;
+        ba += bX0 * Lp;
+        bLp += bX0 * a;
+        br2a2 += bX0 * KiD;
+        bKiD += bX0 * r2a2;
+    }
+    // X4 = Dr (pr^2 + KiD^2) - 2 r (2 E KiD + B iS)
+    const double bDr = bX4 * pk;
+    bpr += 2.0 * bX4 * Dr * pr;
+    const double br4 = -2.0 * bX4;
+    double br = br4 * (2.0 * E * KiD + BiS) + 2.0 * bDr;
+    const double rb4 = r * br4;
+    double bE = 2.0 * rb4 * KiD;
+    bKiD += 2.0 * (rb4 * E + bX4 * Dr * KiD);
+    // X5 = a2 (E^2 + B iS) - (Lz isn2)^2
+    double ba2 = bX5 * (E * E + BiS);
+    const double a2b5 = a2 * bX5;
+    bE += 2.0 * a2b5 * E;
+    const double bq = -2.0 * bX5 * q;
+    double bLz = bq * isn2;
+    bisn2 += bq * Lz;
+    // B iS in both
+    const double bBiS = rb4 + a2b5;
+    const double bB = bBiS * iS;
+    b_iS += bBiS * B;
     // P5 = -sn cs
     double bsn = -bP5 * cs;
     double bcs = -bP5 * sn;
-    // Dr = 2 r - 2
-    br += 2.0 * bDr;
     // B = D pr^2 + pth^2 + Lp^2 isn2 - K KiD
     bD += bB * pr * pr;
-    bpr += bB * 2.0 * D * pr;
-    bpth += bB * 2.0 * pth;
-    bLp += bB * 2.0 * Lp * isn2;
-    bisn2 += bB * Lp * Lp;
-    double bK = -bB * KiD;
-    bKiD += -bB * K;
+    bpr += 2.0 * bB * D * pr;
+    bpth += 2.0 * bB * pth;
+    const double bLp2 = bB * Lp;
+    bLp += 2.0 * bLp2 * isn2;
+    bisn2 += bLp2 * Lp;
+    bKiD -= bB * K;
     // KiD = K iD
-    bK += bKiD * iD;
+    const double bK = bKiD * iD - bB * KiD;
     const double biD = bKiD * K;
     // Lp = Lz - a E sn2
-    bLz += bLp;
-    ba += -bLp * E * sn2;
-    bE += -bLp * a * sn2;
-    double bsn2 = -bLp * a * E;
-    // K = r2a2 E - a Lz
+    bLz += bLp - bK * a;
+    const double bLps = bLp * sn2;
+    ba -= bLps * E + bK * Lz;
+    bE += bK * r2a2 - bLps * a;
+    // K = r2a2 E - a Lz; r2a2 = r2 + a2
     br2a2 += bK * E;
-    bE += bK * r2a2;
-    ba += -bK * Lz;
-    bLz += -bK * a;
-    // r2a2 = r2 + a2
-    double br2 = br2a2;
     ba2 += br2a2;
     // the reciprocals
     const double bS = -b_iS * iS * iS;
-    bD += -biD * iD * iD;
-    bsn2 += -bisn2 * isn2 * isn2;
+    bD -= biD * iD * iD;
+    const double bsn2 = -bLp * a * E - bisn2 * isn2 * isn2;
     // Delta = r^2 - 2 r + a^2 (the factored form has the same value)
-    br += bD * (2.0 * r - 2.0);
+    br += bD * Dr;
     ba2 += bD;
     // Sigma = r2 + a2 cs2
-    br2 += bS;
     ba2 += bS * cs2;
-    const double bcs2 = bS * a2;
-    br += 2.0 * r * br2;
+    br += 2.0 * r * (br2a2 + bS);
     bsn += 2.0 * sn * bsn2;
-    bcs += 2.0 * cs * bcs2;
+    bcs += 2.0 * cs * (bS * a2);
     ba += 2.0 * a * ba2;
     const double bth = (clamped ? 0.0 : cs * bsn) - sn_true * bcs;
     g[0] += br;
@@ -271,6 +294,72 @@ __host__ __device__ BHA_NOINLINE void rhs6_vjp(const RayC& c, double r, double s
     *Lzb += bLz;
     *ab += ba;
 }
+__host__ __device__ BHA_NOINLINE void rhs6_vjp(const RayC& c, double r, double sn, double cs, double pr, double pth,
+                                               const double db[6], double g[4], double* Eb, double* Lzb,
+                                               double* ab) {
+    rhs_vjp<true>(c, r, sn, cs, pr, pth, db, g, Eb, Lzb, ab);
+}
+
+// sin and cos of a stage's angle th from those of the step's base angle th0.
+__host__ __device__ __forceinline__ bool near_angle(double dth) { return fabs(dth) <= kMaxShift; }
+// The full form for an angle that moved further: out of line on the device.
+__host__ __device__ BHA_NOINLINE void far_sincos(double th, double* s, double* c) { sc(th, s, c); }
+__host__ __device__ __forceinline__ void stage_sincos(double th, double th0, double sn0, double cs0, double* s,
+                                                      double* c) {
+    const double dth = th - th0;
+    if (near_angle(dth)) shift_sincos(sn0, cs0, dth, s, c);
+    else far_sincos(th, s, c);
+}
+
+// The Runge-Kutta tableau for the stage loops (row j: stage j + 1), the
+// fifth-order weights (row 6) and the error weights (row 7).
+__host__ __device__ constexpr double tableau(int row, int col) {
+    const double t[8][7] = {
+        {0, 0, 0, 0, 0, 0, 0}, {A21, 0, 0, 0, 0, 0, 0}, {A31, A32, 0, 0, 0, 0, 0},
+        {A41, A42, A43, 0, 0, 0, 0}, {A51, A52, A53, A54, 0, 0, 0}, {A61, A62, A63, A64, A65, 0, 0},
+        {B1, 0, B3, B4, B5, B6, 0}, {E1, 0, E3, E4, E5, E6, E7}};
+    return t[row][col];
+}
+// f(std::integral_constant<int, j>) for a stage number 1 <= j <= 6 that is not
+// known before the loop runs.
+template <class Fn>
+__host__ __device__ __forceinline__ void by_stage(int j, Fn&& f) {
+    switch (j) {
+    case 1: f(std::integral_constant<int, 1>{}); break;
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: f(std::integral_constant<int, 3>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 5: f(std::integral_constant<int, 5>{}); break;
+    default: f(std::integral_constant<int, 6>{}); break;
+    }
+}
+__host__ __device__ __forceinline__ double weight5(int j) {
+    return (j == 0) ? B1 : (j == 2) ? B3 : (j == 3) ? B4 : (j == 4) ? B5 : (j == 5) ? B6 : 0.0;
+}
+
+// A ray's stage values live in shared memory on the device (kScratch doubles
+// per thread, threads side by side: no bank conflicts) and the stage loops
+// stay rolled around one copy of the right-hand side and of its
+// vector-Jacobian product.  Unrolled, with the stages in registers, the forward
+// and the reverse step were 20 to 30 KB of code each and the instruction fetch
+// stalled the kernel (1.4 of 4.2 cycles per issue): 13.2 against 8.6 ms per 512^2
+// gradient on one B200, the dependent binary64 chain of a warp (39% of the issue
+// slots, 41% of the binary64 pipe at 8 warps per SM) bounding what is left.
+constexpr int kScratch = 60;
+constexpr int kAdjBlock = 64;
+#if defined(__CUDA_ARCH__)
+#define BHA_SCRATCH(name)                        \
+    extern __shared__ double bha_scratch_smem[]; \
+    double* const name = bha_scratch_smem + threadIdx.x;
+constexpr int kScratchStride = kAdjBlock;
+#else
+inline double* host_scratch() {
+    static thread_local double buf[kScratch];
+    return buf;
+}
+#define BHA_SCRATCH(name) double* const name = host_scratch();
+constexpr int kScratchStride = 1;
+#endif
 
 // Integrator state of one ray.
 struct Integ {
@@ -278,34 +367,33 @@ struct Integ {
     double k1[6];       // FSAL stage at y
     double h;
     double errp_mem;    // beta ln err_prev, err_prev the last accepted error norm (>= 1e-4)
-    double c0;          // cos(th) at y
+    double sn0, c0;     // sin(th), cos(th) at y
+    double h_acc;       // the last accepted step's size
     int have_k1;
     int tries;
     int steps;
 };
 
-// One accepted step of an attempt loop.
+// One accepted step: its ends' r, th and cosines; its stages are left in the
+// scratch (component i of k_(j+1) at 6 j + i) until the next attempt.
 struct StepRec {
-    double y[6];        // state at the start of the step
-    double yn[6];
-    double kr[7], kth[7];   // r and th components of k1..k7 (dense output)
+    double r0, th0, r1, th1;
     double h;
     double c0, c7;      // cos(th) at y and at yn
 };
 
 // Attempt steps from `s` until one is accepted (render.cpp:127-137 with
 // geodesic.h:123-204), then advance `s`.  Returns false when no acceptable
-// step was found (more than 40 rejections or |h| < 1e-14).
-__host__ __device__ BHA_NOINLINE bool advance(const FrameParams& F, const RayC& c, Integ& s, StepRec* rec) {
-    constexpr double A[6][5] = {{0, 0, 0, 0, 0},
-                                {A21, 0, 0, 0, 0},
-                                {A31, A32, 0, 0, 0},
-                                {A41, A42, A43, 0, 0},
-                                {A51, A52, A53, A54, 0},
-                                {A61, A62, A63, A64, A65}};
+// step was found (more than 40 rejections or |h| < 1e-14).  The sin/cos of the
+// stages and of the step's end come from the step's base angle by angle
+// addition, like the render's; a stored state holds them, so that a step
+// started from it repeats the one that passed it.
+__host__ __device__ __forceinline__ bool advance_step(const FrameParams& F, const RayC& c, Integ& s,
+                                                      StepRec* rec) {
+    BHA_SCRATCH(scr)
+    auto K = [&](int j, int i) -> double& { return scr[(6 * j + i) * kScratchStride]; };
     if (!s.have_k1) {
-        double sn0;
-        rhs6_th(c, s.y[1], s.y[2], s.y[4], s.y[5], s.k1, &sn0, &s.c0);
+        rhs6(c, s.y[1], s.sn0, s.c0, s.y[4], s.y[5], s.k1);
         s.have_k1 = 1;
     }
     for (;;) {
@@ -314,28 +402,47 @@ __host__ __device__ BHA_NOINLINE bool advance(const FrameParams& F, const RayC& 
             if (s.h > hmax) s.h = hmax;
         }
         const double h = s.h;
-        double k[7][6], t[6], yn[6], c7, sn, cs;
-        for (int i = 0; i < 6; ++i) k[0][i] = s.k1[i];
+        double yn[6], e[6], c7 = 0.0, sn7 = 0.0;
         #pragma unroll
-        for (int j = 1; j < 6; ++j) {
-            #pragma unroll
-            for (int i = 0; i < 6; ++i) {
-                double acc = 0.0;
+        for (int i = 0; i < 6; ++i) K(0, i) = s.k1[i];
+        #pragma unroll 1
+        for (int j = 1; j < 7; ++j) {
+            double acc[6] = {0, 0, 0, 0, 0, 0};
+            if (j == 6) {
                 #pragma unroll
-                for (int l = 0; l < j; ++l) acc += A[j][l] * k[l][i];
-                t[i] = s.y[i] + h * acc;
+                for (int i = 0; i < 6; ++i) e[i] = 0.0;
             }
-            rhs6_th(c, t[1], t[2], t[4], t[5], k[j], &sn, &cs);
+            // one case per stage, so that the loads and sums overlap
+            auto sums = [&](auto stage) {
+                constexpr int n = decltype(stage)::value;
+                #pragma unroll
+                for (int l = 0; l < n; ++l) {
+                    #pragma unroll
+                    for (int i = 0; i < 6; ++i) {
+                        if (n < 6 && (i == 0 || i == 3)) continue;   // t and phi enter no stage
+                        const double kk = K(l, i);
+                        acc[i] += tableau(n, l) * kk;
+                        if (n == 6) e[i] += tableau(7, l) * kk;
+                    }
+                }
+            };
+            by_stage(j, sums);
+            #pragma unroll
+            for (int i = 0; i < 6; ++i) yn[i] = s.y[i] + h * acc[i];
+            double d[6], sn, cs;
+            stage_sincos(yn[2], s.y[2], s.sn0, s.c0, &sn, &cs);
+            rhs6(c, yn[1], sn, cs, yn[4], yn[5], d);
+            #pragma unroll
+            for (int i = 0; i < 6; ++i) K(j, i) = d[i];
+            sn7 = sn;
+            c7 = cs;
         }
-        for (int i = 0; i < 6; ++i)
-            yn[i] = s.y[i] + h * (B1 * k[0][i] + B3 * k[2][i] + B4 * k[3][i] + B5 * k[4][i] + B6 * k[5][i]);
-        rhs6_th(c, yn[1], yn[2], yn[4], yn[5], k[6], &sn, &c7);
         double err2 = 0.0;
+        #pragma unroll
         for (int i = 0; i < 6; ++i) {
-            const double e = h * (E1 * k[0][i] + E3 * k[2][i] + E4 * k[3][i] + E5 * k[4][i] + E6 * k[5][i] +
-                                  E7 * k[6][i]);
+            const double ei = h * (e[i] + E7 * K(6, i));
             const double scl = F.atol + F.rtol * dmaxr(fabs(s.y[i]), fabs(yn[i]));
-            const double q = e * rcp_nr(scl);
+            const double q = ei * rcp_nr(scl);
             err2 += q * q;
         }
         // err: the square of the RMS norm; the PI factor 0.9 err^-alpha
@@ -354,27 +461,37 @@ __host__ __device__ BHA_NOINLINE bool advance(const FrameParams& F, const RayC& 
         s.tries = 0;
         ++s.steps;
         if (rec) {
-            for (int i = 0; i < 6; ++i) {
-                rec->y[i] = s.y[i];
-                rec->yn[i] = yn[i];
-            }
-            for (int j = 0; j < 7; ++j) {
-                rec->kr[j] = k[j][1];
-                rec->kth[j] = k[j][2];
-            }
+            rec->r0 = s.y[1];
+            rec->th0 = s.y[2];
+            rec->r1 = yn[1];
+            rec->th1 = yn[2];
             rec->h = h;
             rec->c0 = s.c0;
             rec->c7 = c7;
         }
+        #pragma unroll
         for (int i = 0; i < 6; ++i) {
             s.y[i] = yn[i];
-            s.k1[i] = k[6][i];
+            s.k1[i] = K(6, i);
         }
         s.c0 = c7;
+        s.sn0 = sn7;
         s.errp_mem = kBeta * dmaxr(0.5 * lq, kLnErrFloor);
+        s.h_acc = h;
         s.h = h * fac;
         return true;
     }
+}
+// The same for the replays, out of line.
+__host__ __device__ BHA_NOINLINE bool advance(const FrameParams& F, const RayC& c, Integ& s) {
+    return advance_step(F, c, s, nullptr);
+}
+// The dense output of component i (1: r, 2: th) of the step that advance_step
+// has just recorded.
+__host__ __device__ __forceinline__ DenseC step_dense(const StepRec& q, int i) {
+    BHA_SCRATCH(scr)
+    auto K = [&](int j) { return scr[(6 * j + i) * kScratchStride]; };
+    return dense_coef(q.h, i == 1 ? q.r0 : q.th0, i == 1 ? q.r1 : q.th1, K(0), K(2), K(3), K(4), K(5), K(6));
 }
 
 // Equatorial target angle pi/2 + m pi between th0 and th1 (render.cpp:180-189).
@@ -383,108 +500,131 @@ __host__ __device__ __forceinline__ double crossing_target(double th0, double th
     return 0.5 * kPi + m * kPi;
 }
 
-// Reverse of one component's dense output at s with weight v (adds into the
-// adjoints of y, yn and the stages k1, k3..k7 held as kb[0], kb[2..6]).
-__host__ __device__ __forceinline__ void dense_vjp(double h, double s, double v, int i, double* yb, double* ynb,
-                                                   double kb[7][6]) {
-    const double s1 = 1.0 - s;
-    const double r1b = v;
-    double r2b = s * v;
-    double r3b = s * s1 * v;
-    const double r4b = s * s * s1 * v;
-    const double r5b = s * s * s1 * s1 * v;
-    kb[0][i] += h * D1 * r5b;
-    kb[2][i] += h * D3 * r5b;
-    kb[3][i] += h * D4 * r5b;
-    kb[4][i] += h * D5 * r5b;
-    kb[5][i] += h * D6 * r5b;
-    kb[6][i] += h * D7 * r5b;
-    r2b += r4b;
-    kb[6][i] += -h * r4b;
-    r3b += -r4b;
-    kb[0][i] += h * r3b;
-    r2b += -r3b;
-    ynb[i] += r2b;
-    yb[i] += -r2b;
-    yb[i] += r1b;
-}
-
 // Carries the adjoint yb of the state after one accepted step (from ys with
-// step h) back to the state before it, accumulating the E, L_z and spin
-// adjoints.  rstar_b != 0 marks the step that ends on the disc: the hit
-// radius r* = P_r(s*) at the crossing theta(s*) = target of the dense
-// polynomials then receives the weight rstar_b (and yb, the adjoint of the
-// step's end state, is zero).
-__host__ __device__ BHA_NOINLINE void step_vjp(const RayC& c, const double ys[6], double h, double yb[6],
-                                               double* Eb, double* Lzb, double* ab, double rstar_b) {
-    constexpr double A[6][5] = {{0, 0, 0, 0, 0},
-                                {A21, 0, 0, 0, 0},
-                                {A31, A32, 0, 0, 0},
-                                {A41, A42, A43, 0, 0},
-                                {A51, A52, A53, A54, 0},
-                                {A61, A62, A63, A64, A65}};
-    // Stage inputs (r, th, p_r, p_th) and the sine and cosine of their th,
-    // kept for the stages' vector-Jacobian products.
-    double k[7][6], Y[6][4], Ysn[6], Ycs[6], t[6], yn[6];
-    Y[0][0] = ys[1]; Y[0][1] = ys[2]; Y[0][2] = ys[4]; Y[0][3] = ys[5];
-    rhs6_th(c, ys[1], ys[2], ys[4], ys[5], k[0], &Ysn[0], &Ycs[0]);
-    #pragma unroll
-    for (int j = 1; j < 6; ++j) {
-        #pragma unroll
-        for (int i = 0; i < 6; ++i) {
-            double acc = 0.0;
+// step h; sn0, cs0: sin and cos of its angle) back to the state before it,
+// accumulating the E, L_z and spin adjoints.  The six stages are computed again and their vector-Jacobian
+// products taken in reverse.  rstar_b != 0 marks the step that ends on the
+// disc: the hit radius r* = P_r(s*) at the crossing theta(s*) = target of the
+// dense polynomials then receives the weight rstar_b (and yb, the adjoint of
+// the step's end state, is zero).  yb[0] is zero throughout and yb[3] stays what
+// it is: nothing depends on t, and no right-hand side on phi.
+// Scratch: the stages' derivatives, then their adjoints, component i of stage j
+// at 4 j + i; from 24 on the stages' (r, th, p_r, p_th, sin, cos), 6 each.
+__host__ __device__ __forceinline__ void step_vjp(const RayC& c, const double y0[4], double sn0, double cs0, double h,
+                                                  double yb[6], double* Eb, double* Lzb, double* ab, double rstar_b) {
+    constexpr int kC[4] = {1, 2, 4, 5};      // r, th, p_r, p_th in the state
+    BHA_SCRATCH(scr)
+    auto K = [&](int j, int i) -> double& { return scr[(4 * j + i) * kScratchStride]; };
+    auto Y = [&](int j, int i) -> double& { return scr[(24 + 6 * j + i) * kScratchStride]; };
+    const bool event = rstar_b != 0.0;
+    double yn[4];
+    #pragma unroll 1
+    for (int j = 0; j < 6; ++j) {
+        double acc[4] = {0, 0, 0, 0}, t[4], sn = sn0, cs = cs0;
+        auto sums = [&](auto stage) {
+            constexpr int n = decltype(stage)::value;
             #pragma unroll
-            for (int l = 0; l < j; ++l) acc += A[j][l] * k[l][i];
-            t[i] = ys[i] + h * acc;
-        }
-        Y[j][0] = t[1]; Y[j][1] = t[2]; Y[j][2] = t[4]; Y[j][3] = t[5];
-        rhs6_th(c, t[1], t[2], t[4], t[5], k[j], &Ysn[j], &Ycs[j]);
+            for (int l = 0; l < n; ++l) {
+                #pragma unroll
+                for (int i = 0; i < 4; ++i) acc[i] += tableau(n, l) * K(l, i);
+            }
+        };
+        if (j > 0) by_stage(j, sums);
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) t[i] = y0[i] + h * acc[i];
+        if (j > 0) stage_sincos(t[1], y0[1], sn0, cs0, &sn, &cs);
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) Y(j, i) = t[i];
+        Y(j, 4) = sn;
+        Y(j, 5) = cs;
+        if (j == 5 && !event) break;         // k_6 enters the step's end alone
+        double d[4];
+        rhs4(c, t[0], sn, cs, t[2], t[3], d);
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) K(j, i) = d[i];
     }
-    for (int i = 0; i < 6; ++i)
-        yn[i] = ys[i] + h * (B1 * k[0][i] + B3 * k[2][i] + B4 * k[3][i] + B5 * k[4][i] + B6 * k[5][i]);
 
-    double kb[7][6], ynb[6], ybar[6];
-    for (int j = 0; j < 7; ++j)
-        for (int i = 0; i < 6; ++i) kb[j][i] = 0.0;
-    for (int i = 0; i < 6; ++i) {
-        ynb[i] = yb[i];
+    // The weights of the step's end (the adjoint of yn) and of the state at the
+    // start of the step, and the event's own weights of the stages: all of them
+    // D_j r5 of one component each, D_1 and D_7 with more.
+    double ynb[4], ybar[4], r5r = 0.0, r5th = 0.0, k1r = 0.0, k1th = 0.0;
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        ynb[i] = yb[kC[i]];
         ybar[i] = 0.0;
     }
-    if (rstar_b != 0.0) {
-        double sn7, cs7;
-        rhs6_th(c, yn[1], yn[2], yn[4], yn[5], k[6], &sn7, &cs7);
-        const DenseC cth = dense_coef(h, ys[2], yn[2], k[0][2], k[2][2], k[3][2], k[4][2], k[5][2], k[6][2]);
-        const DenseC crr = dense_coef(h, ys[1], yn[1], k[0][1], k[2][1], k[3][1], k[4][1], k[5][1], k[6][1]);
+    if (event) {
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            double acc = 0.0;
+            for (int l = 0; l < 6; ++l) acc += weight5(l) * K(l, i);
+            yn[i] = y0[i] + h * acc;
+        }
+        double sn7, cs7, k7[4];
+        sc(yn[1], &sn7, &cs7);
+        rhs4(c, yn[0], sn7, cs7, yn[2], yn[3], k7);
+        const DenseC cth = dense_coef(h, y0[1], yn[1], K(0, 1), K(2, 1), K(3, 1), K(4, 1), K(5, 1), k7[1]);
+        const DenseC crr = dense_coef(h, y0[0], yn[0], K(0, 0), K(2, 0), K(3, 0), K(4, 0), K(5, 0), k7[0]);
         const double target = crossing_target(cth.r1, cth.r1 + cth.r2);
-        const double s = dense_crossing(cth, target);
+        const double s = dense_crossing(cth, target), s1 = 1.0 - s;
         const double dth = dense_deriv(cth, s), dr = dense_deriv(crr, s);
-        dense_vjp(h, s, rstar_b, 1, ybar, ynb, kb);
-        if (dth != 0.0) dense_vjp(h, s, -rstar_b * dr / dth, 2, ybar, ynb, kb);
+        // the reverse of a component's dense output at s with weight v (its
+        // coefficients as dense_coef forms them)
+        const double v[2] = {rstar_b, (dth != 0.0) ? -rstar_b * dr / dth : 0.0};
+        double r5[2], k1w[2], k7b[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        #pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const double r4b = s * s * s1 * v[q], r3b = s * s1 * v[q] - r4b;
+            r5[q] = h * s * s * s1 * s1 * v[q];
+            k1w[q] = h * r3b;
+            k7b[1 + q] = D7 * r5[q] - h * r4b;
+            const double r2b = s * v[q] + r4b - r3b;
+            ynb[q] += r2b;
+            ybar[q] += v[q] - r2b;
+        }
+        r5r = r5[0]; r5th = r5[1];
+        k1r = k1w[0]; k1th = k1w[1];
         double g4[4] = {0.0, 0.0, 0.0, 0.0};
-        rhs6_vjp(c, yn[1], sn7, cs7, yn[4], yn[5], kb[6], g4, Eb, Lzb, ab);
-        ynb[1] += g4[0]; ynb[2] += g4[1]; ynb[4] += g4[2]; ynb[5] += g4[3];
-    }
-    for (int i = 0; i < 6; ++i) {
-        ybar[i] += ynb[i];
-        kb[0][i] += h * B1 * ynb[i];
-        kb[2][i] += h * B3 * ynb[i];
-        kb[3][i] += h * B4 * ynb[i];
-        kb[4][i] += h * B5 * ynb[i];
-        kb[5][i] += h * B6 * ynb[i];
+        rhs_vjp<false>(c, yn[0], sn7, cs7, yn[2], yn[3], k7b, g4, Eb, Lzb, ab);
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) ynb[i] += g4[i];
     }
     #pragma unroll
-    for (int j = 5; j >= 0; --j) {
-        double g4[4] = {0.0, 0.0, 0.0, 0.0};
-        rhs6_vjp(c, Y[j][0], Ysn[j], Ycs[j], Y[j][2], Y[j][3], kb[j], g4, Eb, Lzb, ab);
-        const double Yb[6] = {0.0, g4[0], g4[1], 0.0, g4[2], g4[3]};
+    for (int i = 0; i < 4; ++i) ybar[i] += ynb[i];
+    #pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        constexpr double Dw[6] = {D1, 0.0, D3, D4, D5, D6};
+        const double hb = h * weight5(j);
         #pragma unroll
-        for (int i = 0; i < 6; ++i) {
-            ybar[i] += Yb[i];
-            #pragma unroll
-            for (int l = 0; l < j; ++l) kb[l][i] += h * A[j][l] * Yb[i];
+        for (int i = 0; i < 4; ++i) {
+            double v = hb * ynb[i];
+            if (i == 0) v += Dw[j] * r5r + (j == 0 ? k1r : 0.0);
+            if (i == 1) v += Dw[j] * r5th + (j == 0 ? k1th : 0.0);
+            K(j, i) = v;
         }
     }
-    for (int i = 0; i < 6; ++i) yb[i] = ybar[i];
+    const double hphi = h * yb[3];
+    #pragma unroll 1
+    for (int j = 5; j >= 0; --j) {
+        double g4[4] = {0.0, 0.0, 0.0, 0.0};
+        const double db[6] = {0.0, K(j, 0), K(j, 1), weight5(j) * hphi, K(j, 2), K(j, 3)};
+        rhs_vjp<false>(c, Y(j, 0), Y(j, 4), Y(j, 5), Y(j, 2), Y(j, 3), db, g4, Eb, Lzb, ab);
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) ybar[i] += g4[i];
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) g4[i] *= h;
+        auto spread = [&](auto stage) {
+            constexpr int n = decltype(stage)::value;
+            #pragma unroll
+            for (int l = 0; l < n; ++l) {
+                #pragma unroll
+                for (int i = 0; i < 4; ++i) K(l, i) += tableau(n, l) * g4[i];
+            }
+        };
+        if (j > 0) by_stage(j, spread);
+    }
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) yb[kC[i]] = ybar[i];
 }
 
 // ---- shading in forward mode ---------------------------------------------------
@@ -602,6 +742,34 @@ __host__ __device__ inline bool escape_direction(const double y[6], double E_, d
     v[0] = v[0] / vn;
     v[1] = v[1] / vn;
     v[2] = v[2] / vn;
+    return true;
+}
+
+// The escape direction alone.
+__host__ __device__ inline bool escape_direction_value(const double y[6], double E, double Lz, double a,
+                                                       double v[3]) {
+    const double r = y[1], a2 = a * a;
+    double sn_raw, cs, sp, cp;
+    sc(y[2], &sn_raw, &cs);
+    sc(y[3], &sp, &cp);
+    const double sn = (fabs(sn_raw) < 1e-9) ? ((sn_raw < 0.0) ? -1e-9 : 1e-9) : sn_raw;
+    const double sn2 = sn * sn;
+    const double Sig = r * r + a2 * cs * cs;
+    const double Del = r * r - 2.0 * r + a2;
+    const double SD = Sig * Del;
+    const double dr = (Del / Sig) * y[4];
+    const double dth = y[5] / Sig;
+    const double dph = -2.0 * a * r / SD * (-E) + (Del - a2 * sn2) / (SD * sn2) * Lz;
+    const double R = std::sqrt(r * r + a2);
+    const double dR = (R > 0.0) ? r / R * dr : dr;
+    v[0] = dR * sn_raw * cp + R * cs * dth * cp - R * sn_raw * sp * dph;
+    v[1] = dR * sn_raw * sp + R * cs * dth * sp + R * sn_raw * cp * dph;
+    v[2] = dr * cs - r * sn_raw * dth;
+    const double vn = std::sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+    if (!(vn > 0.0)) return false;
+    v[0] /= vn;
+    v[1] /= vn;
+    v[2] /= vn;
     return true;
 }
 
@@ -789,34 +957,48 @@ __host__ __device__ inline void ray_start(const FrameParams& F, const AdjointFra
     ray_start_at(F, X, su, sv, y, E, Lz, dy, dE, dLz);
 }
 
-// Accepted steps of the replay buffer: the reverse pass recomputes a segment
-// in pieces of at most this many steps.
+// Accepted steps of the replay buffer: where states were thinned the reverse
+// pass recomputes a segment in pieces of at most this many steps.
 constexpr int kReplay = 16;
 
-// Checkpoint store of one ray: `slots` states of 8 doubles (y, h, beta ln err_prev)
-// after every `interval` accepted steps; full slots drop every second state
-// and double the interval.
+// Stored states of one ray: y, sin and cos of its angle, the proposed h and
+// beta ln err_prev after every `interval` accepted steps, and the size of the
+// step taken from there.  With
+// the interval at one, as every ray starts, the reverse sweep reads each
+// step's state and size back and integrates nothing again; full slots drop
+// every second state and double the interval, and a segment's steps are then
+// replayed from its first state.  Word w of slot j lies at
+// ck[(j kCkWords + w) stride]: on the device the lanes of a warp interleave
+// (stride 32), so that their accesses coalesce.
+constexpr int kCkWords = 11;
 struct Checkpoints {
     double* ck;
     int slots;
     int interval;
     int n;
-    __host__ __device__ void push(const Integ& st) {
-        double* p = ck + 8 * n;
-        for (int i = 0; i < 6; ++i) p[i] = st.y[i];
-        p[6] = st.h;
-        p[7] = st.errp_mem;
+    int stride;
+    __host__ __device__ __forceinline__ double* at(int slot, int word) const {
+        return ck + ((long long)slot * kCkWords + word) * stride;
+    }
+    __host__ __device__ __forceinline__ void push(const Integ& st) {
+        for (int i = 0; i < 6; ++i) *at(n, i) = st.y[i];
+        *at(n, 6) = st.h;
+        *at(n, 7) = st.errp_mem;
+        *at(n, 9) = st.sn0;
+        *at(n, 10) = st.c0;
         ++n;
     }
-    __host__ __device__ void after_step(const Integ& st) {
+    __host__ __device__ __forceinline__ void after_step(const Integ& st) {
+        if (interval == 1) *at(n - 1, 8) = st.h_acc;
         if (st.steps % interval != 0) return;
-        if (n == slots) {
-            for (int j = 0; j < slots / 2; ++j)
-                for (int i = 0; i < 8; ++i) ck[8 * j + i] = ck[8 * (2 * j) + i];
-            n = slots / 2;
-            interval *= 2;
-        }
+        if (n == slots) thin();
         if (st.steps % interval == 0) push(st);
+    }
+    __host__ __device__ BHA_NOINLINE void thin() {
+        for (int j = 0; j < slots / 2; ++j)
+            for (int i = 0; i < kCkWords; ++i) *at(j, i) = *at(2 * j, i);
+        n = slots / 2;
+        interval *= 2;
     }
 };
 
@@ -835,22 +1017,35 @@ struct Crossings {
 // crossing's step with its radius in *r_hit and without looking at whether
 // it hits the disc.  The crossing radius of a disc hit goes to *r_hit.
 // Checkpoints (cp) and the first two equatorial crossings (xr) are recorded
-// when given.
-__host__ __device__ inline int forward_run(const FrameParams& F, const RayC& c, Integ& s, Checkpoints* cp,
-                                           Crossings* xr, int stop_crossing, double* r_hit) {
+// when given.  end_falling: a ray moving inwards inside the innermost photon
+// orbit ends there as captured; no turning point is left to it and nothing
+// lies on its way (the disc ends at the ISCO), and the creep to the horizon it
+// is spared is most of a captured ray's steps.
+__host__ __device__ BHA_NOINLINE int forward_run(const FrameParams& F, const RayC& ray, Integ& state, Checkpoints* cp_io,
+                                                    Crossings* xr, int stop_crossing, double* r_hit,
+                                                    bool end_falling = false) {
     if (F.max_steps <= 0) return BH_HIT_EXHAUSTED;
+    // the ray in registers; handed back at its end
+    const RayC c = ray;
+    Integ s = state;
+    Checkpoints cps{nullptr, 0, 1, 0, 1};
+    if (cp_io) cps = *cp_io;
+    Checkpoints* const cp = cp_io ? &cps : nullptr;
+    auto end = [&](int what) {
+        state = s;
+        if (cp_io) *cp_io = cps;
+        return what;
+    };
     StepRec rec;
     int crossings = 0;
     for (;;) {
-        if (!advance(F, c, s, &rec)) return BH_HIT_HORIZON;   // no acceptable step (render.cpp:133-136)
-        const double rn = rec.yn[1];
-        if (rn <= F.r_stop) return BH_HIT_HORIZON;
+        if (!advance_step(F, c, s, &rec)) return end(BH_HIT_HORIZON);   // no acceptable step (render.cpp:133-136)
+        const double rn = rec.r1;
+        if (rn <= F.r_stop) return end(BH_HIT_HORIZON);
         if (F.disc_enabled && rec.c0 * rec.c7 < 0.0) {
-            const DenseC cth = dense_coef(rec.h, rec.y[2], rec.yn[2], rec.kth[0], rec.kth[2], rec.kth[3],
-                                          rec.kth[4], rec.kth[5], rec.kth[6]);
+            const DenseC cth = step_dense(rec, 2);
             const double s_end = dense_crossing(cth, crossing_target(cth.r1, cth.r1 + cth.r2));
-            const DenseC crr = dense_coef(rec.h, rec.y[1], rec.yn[1], rec.kr[0], rec.kr[2], rec.kr[3],
-                                          rec.kr[4], rec.kr[5], rec.kr[6]);
+            const DenseC crr = step_dense(rec, 1);
             const double rc = dense_eval(crr, s_end);
             if (xr) {
                 if (xr->n < 2) {
@@ -861,58 +1056,82 @@ __host__ __device__ inline int forward_run(const FrameParams& F, const RayC& c, 
             }
             if (++crossings == stop_crossing) {
                 *r_hit = rc;
-                return -1;
+                return end(-1);
             }
             if (rc >= F.r_in && rc <= F.r_out) {
                 *r_hit = rc;
-                return BH_HIT_DISC;
+                return end(BH_HIT_DISC);
             }
         }
-        if (rn > F.r_escape) return BH_HIT_SKY;
-        if (s.steps >= F.max_steps) return BH_HIT_EXHAUSTED;
+        if (rn > F.r_escape) return end(BH_HIT_SKY);
+        if (s.steps >= F.max_steps) return end(BH_HIT_EXHAUSTED);
+        if (end_falling && rn < F.r_promote && s.k1[1] < 0.0) return end(BH_HIT_HORIZON);
         if (cp) cp->after_step(s);
     }
 }
 
 // The reverse pass: carries the adjoint yb of the state after accepted step N
-// (and, when rstar_b != 0, the weight of the disc-crossing radius of step N)
-// back to the initial photon, segment by segment from the checkpoints, with
-// the E, L_z and spin adjoints accumulated.  Returns the steps replayed.
-__host__ __device__ inline long long reverse_sweep(const FrameParams& F, const RayC& c, const Checkpoints& cp,
-                                                   int N, double rstar_b, double yb[6], double* Eb, double* Lzb,
-                                                   double* ab) {
+// of size h_last (and, when rstar_b != 0, the weight of the disc-crossing
+// radius of step N) back to the initial photon, with the E, L_z and spin
+// adjoints accumulated.  Returns the steps replayed (none where every state
+// was kept).
+__host__ __device__ BHA_NOINLINE long long reverse_sweep(const FrameParams& F, const RayC& ray, const Checkpoints& cps,
+                                                         int N, double h_last, double rstar_b, double yb[6],
+                                                         double* Eb, double* Lzb, double* ab) {
+    constexpr int kC[4] = {1, 2, 4, 5};
+    const RayC c = ray;
+    const Checkpoints cp = cps;
     long long replay = 0;
-    const int interval = cp.interval;
-    double ys_buf[kReplay][6], hs_buf[kReplay];
-    for (int seg = (N - 1) / interval; seg >= 0; --seg) {
-        const int first = seg * interval + 1;               // first step of the segment
-        const int last = (first + interval - 1 < N) ? first + interval - 1 : N;
-        const int len = last - first + 1;
-        const int npiece = (len + kReplay - 1) / kReplay;
-        for (int piece = npiece - 1; piece >= 0; --piece) {
-            Integ r;
-            const double* p = cp.ck + 8 * seg;
-            for (int i = 0; i < 6; ++i) r.y[i] = p[i];
-            r.h = p[6];
-            r.errp_mem = p[7];
-            r.have_k1 = 0;
-            r.tries = 0;
-            r.steps = 0;
-            for (int j = 0; j < piece * kReplay; ++j) advance(F, c, r, nullptr);
-            const int m = (len - piece * kReplay < kReplay) ? len - piece * kReplay : kReplay;
-            for (int j = 0; j < m; ++j) {
-                StepRec q;
-                advance(F, c, r, &q);
-                for (int i = 0; i < 6; ++i) ys_buf[j][i] = q.y[i];
-                hs_buf[j] = q.h;
+    double buf[kReplay][7];                  // a replayed piece: r, th, p_r, p_th, the step's size, sin, cos
+    int first = 0, m = 0;                    // its steps: first + 1 .. first + m
+    double yv[6], Ev = *Eb, Lv = *Lzb, av = *ab;
+    for (int i = 0; i < 6; ++i) yv[i] = yb[i];
+    for (int j = N - 1; j >= 0; --j) {       // step j + 1, from state j
+        double y0[4], h, sn, cs;
+        if (cp.interval == 1) {
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) y0[i] = *cp.at(j, kC[i]);
+            h = (j == N - 1) ? h_last : *cp.at(j, 8);
+            sn = *cp.at(j, 9);
+            cs = *cp.at(j, 10);
+        } else {
+            if (j < first || m == 0) {
+                // replay the piece that ends with step j + 1 from the last
+                // stored state before it
+                const int seg = j / cp.interval, off = j - seg * cp.interval;
+                const int skip = (off / kReplay) * kReplay;
+                first = seg * cp.interval + skip;
+                m = j - first + 1;
+                Integ r;
+                for (int i = 0; i < 6; ++i) r.y[i] = *cp.at(seg, i);
+                r.h = *cp.at(seg, 6);
+                r.errp_mem = *cp.at(seg, 7);
+                r.sn0 = *cp.at(seg, 9);
+                r.c0 = *cp.at(seg, 10);
+                r.have_k1 = 0;
+                r.tries = 0;
+                r.steps = 0;
+                for (int q = 0; q < skip; ++q) advance(F, c, r);
+                for (int q = 0; q < m; ++q) {
+                    for (int i = 0; i < 4; ++i) buf[q][i] = r.y[kC[i]];
+                    buf[q][5] = r.sn0;
+                    buf[q][6] = r.c0;
+                    advance(F, c, r);
+                    buf[q][4] = r.h_acc;
+                }
+                replay += skip + m;
             }
-            replay += piece * kReplay + m;
-            for (int j = m - 1; j >= 0; --j) {
-                const bool final_step = first + piece * kReplay + j == N;
-                step_vjp(c, ys_buf[j], hs_buf[j], yb, Eb, Lzb, ab, final_step ? rstar_b : 0.0);
-            }
+            for (int i = 0; i < 4; ++i) y0[i] = buf[j - first][i];
+            h = buf[j - first][4];
+            sn = buf[j - first][5];
+            cs = buf[j - first][6];
         }
+        step_vjp(c, y0, sn, cs, h, yv, &Ev, &Lv, &av, (j == N - 1) ? rstar_b : 0.0);
     }
+    for (int i = 0; i < 6; ++i) yb[i] = yv[i];
+    *Eb = Ev;
+    *Lzb = Lv;
+    *ab = av;
     return replay;
 }
 
@@ -930,19 +1149,21 @@ __host__ __device__ inline RayC ray_consts(const FrameParams& F, double E, doubl
 
 __host__ __device__ inline void integ_start(const FrameParams& F, const double y0[6], Integ& s) {
     for (int i = 0; i < 6; ++i) s.y[i] = y0[i];
+    sc(y0[2], &s.sn0, &s.c0);
     s.h = F.h0;
     s.errp_mem = kBeta * kLnErrFloor;
+    s.h_acc = 0.0;
     s.have_k1 = 0;
     s.tries = 0;
     s.steps = 0;
 }
 
 // The forward pass, the seed and the reverse pass of one ray.  `ck` holds
-// `slots` checkpoints of 8 doubles.  With w == 0 (or forward_only) only the
+// `slots` states of kCkWords doubles.  With w == 0 (or forward_only) only the
 // luminance is computed.  xr (may be null) receives the ray's first two
 // equatorial crossings.
 __host__ __device__ inline void adjoint_ray(const FrameParams& F, const AdjointFrame& X, const SkyData& sky,
-                                            long long local_id, double w, double* ck, int slots,
+                                            long long local_id, double w, double* ck, int slots, int stride,
                                             bool forward_only, RayResult* out, Crossings* xr = nullptr) {
     double y0[6], E, Lz, dy0[2][6], dE[2], dLz[2];
     ray_start(F, X, local_id, y0, &E, &Lz, dy0, dE, dLz);
@@ -953,7 +1174,7 @@ __host__ __device__ inline void adjoint_ray(const FrameParams& F, const AdjointF
 
     Integ s;
     integ_start(F, y0, s);
-    Checkpoints cp{ck, slots, X.checkpoint_interval, 0};
+    Checkpoints cp{ck, slots, X.checkpoint_interval, 0, stride};
     cp.push(s);
     double r_hit = 0.0;
     const int what = forward_run(F, c, s, &cp, xr, 0, &r_hit);
@@ -993,7 +1214,7 @@ __host__ __device__ inline void adjoint_ray(const FrameParams& F, const AdjointF
         return;
 
     // ---- reverse and the initial photon ------------------------------------------------
-    out->replay = reverse_sweep(F, c, cp, s.steps, what == BH_HIT_DISC ? rstar_b : 0.0, yb, &Eb, &Lzb, &ab);
+    out->replay = reverse_sweep(F, c, cp, s.steps, s.h_acc, what == BH_HIT_DISC ? rstar_b : 0.0, yb, &Eb, &Lzb, &ab);
     for (int q = 0; q < 2; ++q) {
         double gq = Eb * dE[q] + Lzb * dLz[q];
         for (int i = 0; i < 6; ++i) gq += yb[i] * dy0[q][i];
@@ -1093,7 +1314,7 @@ enum { kEdgeOuter = 1, kEdgeInner = 2 };
 // continuation and replay).
 __host__ __device__ BHA_NOINLINE long long edge_sample(const FrameParams& F, const AdjointFrame& X, const SkyData& sky,
                                                  int px, int py, int k, int crossing, int edges, double w,
-                                                 double* ck, int slots, double out[3], int* cells,
+                                                 double* ck, int slots, int stride, double out[3], int* cells,
                                                  double* diag = nullptr) {
     out[0] = out[1] = out[2] = 0.0;
     *cells = 0;
@@ -1104,17 +1325,18 @@ __host__ __device__ BHA_NOINLINE long long edge_sample(const FrameParams& F, con
     const RayC c = ray_consts(F, E, Lz);
     Integ s;
     integ_start(F, y0, s);
-    Checkpoints cp{ck, slots, X.checkpoint_interval, 0};
+    Checkpoints cp{ck, slots, X.checkpoint_interval, 0, stride};
     cp.push(s);
     double rc = 0.0;
     if (forward_run(F, c, s, &cp, nullptr, crossing, &rc) != -1) return s.steps;
     const int step = s.steps;
+    const double h_step = s.h_acc;
 
     // What the ray meets when this crossing misses the disc: its
     // continuation traced on from there.
     Integ t = s;
     double r_hit = 0.0;
-    const int what = forward_run(F, c, t, nullptr, nullptr, 0, &r_hit);
+    const int what = forward_run(F, c, t, nullptr, nullptr, 0, &r_hit, true);
     long long work = t.steps;
     double Y_beyond = 0.0;
     if (what == BH_HIT_DISC) {
@@ -1136,7 +1358,7 @@ __host__ __device__ BHA_NOINLINE long long edge_sample(const FrameParams& F, con
     // d r_c / d(initial state, E, L_z, spin) by a reverse sweep seeded with r_c
     double yb[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     double Eb = 0.0, Lzb = 0.0, ab = 0.0;
-    work += reverse_sweep(F, c, cp, step, 1.0, yb, &Eb, &Lzb, &ab);
+    work += reverse_sweep(F, c, cp, step, h_step, 1.0, yb, &Eb, &Lzb, &ab);
 
     double dpr[2], dpth[2], dEp[2], dLzp[2];
     ray_start_pixel_tangents(F, su, sv, dpr, dpth, dEp, dLzp);

@@ -51,11 +51,13 @@ struct AdjointLaunch {
     const float* target;             // target luminance, row-major W x H (device)
     double* ray_grad;                // 4 per ray, pixel-major then sample (device)
     double* ray_Y;                   // luminance per ray in the same order, or nullptr
-    double* ckpt;                    // grid * block * checkpoint_slots * 8 doubles
+    double* ckpt;                    // grid * block * checkpoint_slots * kAdjSlotWords doubles
+    const HitRecord* hits;           // the render's hit records, work order (device)
+    int* rays;                       // the rays that have a gradient (work order ids; n_rays entries)
     // The edge pass: per crossing slot (2 per ray, slot = 2 * ray + crossing,
     // rays in work order) the radius of the ray's first two equatorial
     // crossings as the render found them (0: none; zeroed before the
-    // render), the candidate list ((slot << 2) | kEdge* bits) and 3 edge
+    // render; the second one's sign is set when a third followed), the candidate list ((slot << 2) | kEdge* bits) and 3 edge
     // contributions per slot.
     double* xing_r;
     unsigned long long* cand;
@@ -64,7 +66,7 @@ struct AdjointLaunch {
     // crossing (an image of order three or higher), in ray_grad order
     unsigned char* high_order;
     // next job, accepted, replayed, disc rays, sky rays, max interval, edge
-    // candidates, edge-pass steps, edge cells, high-order rays
+    // candidates, edge-pass steps, edge cells, high-order rays, rays with a gradient
     unsigned long long* counters;
     // loss; the four per-ray gradient sums (spin and inclination over the
     // rays of image order one and two); the three edge sums; the spin and
@@ -74,7 +76,8 @@ struct AdjointLaunch {
     int grid, block;
 };
 
-constexpr int kAdjCounters = 10;
+constexpr int kAdjCounters = 11;
+constexpr int kAdjSlotWords = 11;         // doubles per stored state
 constexpr int kAdjSums = 10;
 
 // Enqueues the edge pass's candidate selection over the sample grid, the
@@ -82,7 +85,9 @@ constexpr int kAdjSums = 10;
 // of the per-ray gradients, the edge contributions and the loss; `counters`
 // and `edge_out` must be zeroed before.
 cudaError_t launch_adjoint(const AdjointLaunch& L, cudaStream_t stream);
-// Resident blocks of the adjoint kernel per SM at `block_size` threads.
+// Threads per block of the adjoint kernel, and its resident blocks per SM at
+// `block_size` threads.
+int adjoint_block_size();
 int adjoint_blocks_per_sm(int block_size);
 
 }  // namespace bhg

@@ -52,8 +52,8 @@ int make_adjoint_frame(const bh_render_config& c, const FrameParams& F, AdjointF
         err = "the adjoint needs |spin| < 1";
         return BH_ERR_INVALID_ARG;
     }
-    X.checkpoint_interval = 16;
-    X.checkpoint_slots = 64;
+    X.checkpoint_interval = 1;
+    X.checkpoint_slots = 512;
 
     // Camera: slot 0 = spin, slot 1 = polar angle.
     using D2 = Dual<2>;

@@ -78,7 +78,7 @@ struct bh_ctx {
     DevBuf sel_flag, sel_list;         // near-critical classification of a mixed launch's rays
     // Adjoint: target image, per-ray gradients and luminances, checkpoint
     // slots, counters, sums and the edge pass's buffers.
-    DevBuf adj_target, adj_grad, adj_Y, adj_ckpt, adj_counters, adj_sums, adj_xr, adj_cand, adj_edge, adj_high;
+    DevBuf adj_target, adj_grad, adj_Y, adj_ckpt, adj_counters, adj_sums, adj_xr, adj_cand, adj_edge, adj_high, adj_rays;
     DevBuf band_done;
     // Display transform: blur scratch, glare weights, meter state, 8-bit output.
     DevBuf disp_tmp, disp_near, disp_far, disp_k, disp_state, disp_rgb;
@@ -664,7 +664,7 @@ void bh_gpu_destroy(bh_ctx* ctx) {
     for (DevBuf* b : {&ctx->hits, &ctx->pixels, &ctx->rays, &ctx->lum, &ctx->frames, &ctx->ray_end, &ctx->deferred,
                       &ctx->pix_end, &ctx->partials, &ctx->fstats, &ctx->jet, &ctx->adj_target, &ctx->adj_grad, &ctx->adj_Y,
                       &ctx->adj_ckpt, &ctx->adj_counters, &ctx->adj_sums, &ctx->adj_xr, &ctx->adj_cand, &ctx->adj_edge,
-                      &ctx->adj_high, &ctx->eval_in, &ctx->eval_out, &ctx->disp_tmp, &ctx->disp_near,
+                      &ctx->adj_high, &ctx->adj_rays, &ctx->eval_in, &ctx->eval_out, &ctx->disp_tmp, &ctx->disp_near,
                       &ctx->disp_far, &ctx->disp_k, &ctx->disp_state, &ctx->disp_rgb, &ctx->sel_flag,
                       &ctx->sel_list, &ctx->band_done})
         if (b->p) cudaFree(b->p);
@@ -871,17 +871,18 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
         std::string err;
         if ((rc = make_adjoint_frame(c, frames[0], X, err)) != BH_OK) return fail(ctx, rc, err);
     }
-    const int block = 128;
+    const int block = adjoint_block_size();
     int bps = adjoint_blocks_per_sm(block);
     if (bps < 1) bps = 1;
-    const int grid = ctx->sm_count * bps;
     const size_t npx = static_cast<size_t>(c.width) * c.height;
     const long long n_rays = frames[0].n_rays;
+    // no more blocks than jobs (a ray, and an edge term for each of its two crossings)
+    const int grid = static_cast<int>(std::min<long long>(ctx->sm_count * bps, (3 * n_rays + block - 1) / block));
     if ((rc = ensure(ctx, ctx->pixels, npx * sizeof(bh_xyz))) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->adj_target, npx * sizeof(float))) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->adj_grad, static_cast<size_t>(n_rays) * 4 * sizeof(double))) != BH_OK) return rc;
     if (ray_Y && (rc = ensure(ctx, ctx->adj_Y, static_cast<size_t>(n_rays) * sizeof(double))) != BH_OK) return rc;
-    const size_t ck_bytes = static_cast<size_t>(grid) * block * X.checkpoint_slots * 8 * sizeof(double);
+    const size_t ck_bytes = static_cast<size_t>(grid) * block * X.checkpoint_slots * kAdjSlotWords * sizeof(double);
     if ((rc = ensure(ctx, ctx->adj_ckpt, ck_bytes)) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->adj_counters, kAdjCounters * sizeof(unsigned long long))) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->adj_sums, kAdjSums * sizeof(double))) != BH_OK) return rc;
@@ -890,6 +891,7 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
     if ((rc = ensure(ctx, ctx->adj_cand, n_slots * sizeof(unsigned long long))) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->adj_edge, n_slots * 3 * sizeof(double))) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->adj_high, static_cast<size_t>(n_rays))) != BH_OK) return rc;
+    if ((rc = ensure(ctx, ctx->adj_rays, static_cast<size_t>(n_rays) * sizeof(int))) != BH_OK) return rc;
 
     CK(cudaMemcpyAsync(ctx->adj_target.p, target, npx * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     ctx->h2d += static_cast<long long>(npx * sizeof(float));
@@ -916,6 +918,8 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
     L.ray_grad = static_cast<double*>(ctx->adj_grad.p);
     L.ray_Y = ray_Y ? static_cast<double*>(ctx->adj_Y.p) : nullptr;
     L.ckpt = static_cast<double*>(ctx->adj_ckpt.p);
+    L.hits = static_cast<const HitRecord*>(ctx->hits.p);
+    L.rays = static_cast<int*>(ctx->adj_rays.p);
     L.xing_r = static_cast<double*>(ctx->adj_xr.p);
     L.cand = static_cast<unsigned long long*>(ctx->adj_cand.p);
     L.edge_out = static_cast<double*>(ctx->adj_edge.p);

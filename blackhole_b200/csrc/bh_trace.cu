@@ -1075,8 +1075,10 @@ __device__ bool attempt(const TraceArgs& A, Lane<P>& L) {
         if (SURF && A.xing) {
             // the crossings the discrete adjoint's edge pass starts from
             double* x = A.xing + 2 * L.gid;
+            // (a third one sets the sign of the second's radius)
             if (x[0] == 0.0) x[0] = rc;
             else if (x[1] == 0.0) x[1] = rc;
+            else x[1] = -fabs(x[1]);
         }
         if (rc >= F.r_in && rc <= F.r_out) {
             what = BH_HIT_DISC;

@@ -110,9 +110,9 @@ int bhx_ray(const bh_render_config* cfg, long long local_id, double w, int forwa
     const int rc = prepare(cfg, F, X, sd);
     if (rc != BH_OK) return rc;
     if (slots > 0) X.checkpoint_slots = slots;
-    std::vector<double> ck(static_cast<size_t>(X.checkpoint_slots) * 8);
+    std::vector<double> ck(static_cast<size_t>(X.checkpoint_slots) * adj::kCkWords);
     adj::RayResult r;
-    adj::adjoint_ray(F, X, sd, local_id, w, ck.data(), X.checkpoint_slots, forward_only != 0, &r);
+    adj::adjoint_ray(F, X, sd, local_id, w, ck.data(), X.checkpoint_slots, 1, forward_only != 0, &r);
     out[0] = r.Y;
     for (int q = 0; q < 4; ++q) out[1 + q] = r.grad[q];
     out[5] = r.what;
@@ -152,14 +152,14 @@ int bhx_crossings(const bh_render_config* cfg, long long local_id, double r[2], 
     SkyData sd;
     const int rc = prepare(cfg, F, X, sd);
     if (rc != BH_OK) return rc;
-    std::vector<double> ck(static_cast<size_t>(X.checkpoint_slots) * 8);
+    std::vector<double> ck(static_cast<size_t>(X.checkpoint_slots) * adj::kCkWords);
     adj::RayResult res;
     adj::Crossings xr;
     xr.n = 0;
     xr.count = 0;
     xr.r[0] = xr.r[1] = 0.0;
     xr.step[0] = xr.step[1] = 0;
-    adj::adjoint_ray(F, X, sd, local_id, 0.0, ck.data(), X.checkpoint_slots, true, &res, &xr);
+    adj::adjoint_ray(F, X, sd, local_id, 0.0, ck.data(), X.checkpoint_slots, 1, true, &res, &xr);
     for (int k = 0; k < 2; ++k) {
         r[k] = xr.r[k];
         steps[k] = xr.step[k];
@@ -184,11 +184,11 @@ int bhx_edge(const bh_render_config* cfg, int px, int py, int k, int crossing, i
     SkyData sd;
     const int rc = prepare(cfg, F, X, sd);
     if (rc != BH_OK) return rc;
-    std::vector<double> ck(static_cast<size_t>(X.checkpoint_slots) * 8);
+    std::vector<double> ck(static_cast<size_t>(X.checkpoint_slots) * adj::kCkWords);
     for (int i = 0; i < 12; ++i) diag[i] = 0.0;
     int cells = 0;
     diag[11] = static_cast<double>(
-        adj::edge_sample(F, X, sd, px, py, k, crossing, edges, w, ck.data(), X.checkpoint_slots, out, &cells,
+        adj::edge_sample(F, X, sd, px, py, k, crossing, edges, w, ck.data(), X.checkpoint_slots, 1, out, &cells,
                          diag));
     diag[10] = cells;
     return BH_OK;

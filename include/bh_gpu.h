@@ -428,8 +428,9 @@ typedef struct bh_grad4 {
    spin, the camera inclination, the Eddington ratio and the disc's outer
    radius.  The frame is rendered in binary64 (whatever cfg->precision says);
    the gradient is the discrete adjoint of that render: each ray's accepted
-   DP5 step sequence is replayed backwards from checkpoints (every 16 accepted
-   steps, 64 per ray in flight; the interval doubles for longer rays), with
+   DP5 step sequence is taken backwards from its stored states (one per
+   accepted step, 512 per ray in flight; for longer rays every second, fourth
+   .. state is kept and the steps between are replayed), with
    the step sizes and each ray's termination class held fixed.  To that the
    edge term is added: the motion of the disc's outer edge (r_out) and inner
    edge (the ISCO) across the image, which a point-sampled frame shows only
