@@ -48,6 +48,7 @@ struct bh_ctx {
     // best on the 1024^2 edge-on frame: the tight register caps, blocks of
     // 128 for FP64 and 256 for mixed).
     bh_launch_params launch[2] = {{128, 1, 32, 0, 1}, {256, 1, 32, 0, 1}};
+    bool launch_set[2] = {false, false};   // by bh_gpu_set_launch or the autotuner
     unsigned long long budget = 0;
     std::atomic<int> abort_requested{0};
     int32_t* h_one = nullptr;          // pinned 1, source of the abort copy
@@ -103,13 +104,6 @@ struct bh_ctx {
 namespace {
 
 constexpr int kReduceBlocks = 512;
-// Blocks of the near-critical binary64 kernel beside a mixed-precision launch.
-constexpr int kSideBlocks = 32;
-// Registers of one SM, and the registers a warp of threads using `per_thread`
-// is allocated (in units of 256).
-constexpr long long kSmRegs = 65536;
-long long warp_regs(int per_thread) { return (static_cast<long long>(per_thread) * 32 + 255) / 256 * 256; }
-
 int fail(bh_ctx* ctx, int code, const std::string& msg) {
     if (ctx) ctx->err = msg;
     return code;
@@ -311,8 +305,20 @@ int plan_launch(bh_ctx* ctx, std::vector<FrameParams>& frames, bh_xyz* d_pixels,
     std::memcpy(s + fbytes + 2 * n * sizeof(long long), &q, sizeof q);
 
     const int prec = frames[0].precision_tag;
-    const bh_launch_params& lp = ctx->launch[prec == BH_PRECISION_MIXED ? 1 : 0];
-    const bh_launch_params& lp64 = ctx->launch[0];
+    bh_launch_params lp = ctx->launch[prec == BH_PRECISION_MIXED ? 1 : 0];
+    if (prec == BH_PRECISION_FP64 && !ctx->launch_set[0]) {
+        // A few waves of rays are bounded by the longest serial chains, which
+        // the wide register cap (no spills) shortens; larger launches by
+        // throughput, which the tight one's twelve warps per SM serve better.
+        // One B200, ms per frame, tight and wide: 256^2 kerr 1.70 and 1.33,
+        // edge-on 2.65 and 2.14; 384^2 2.35 and 2.10, 3.33 and 2.94; 512^2 3.09 and
+        // 3.16, 4.09 and 3.69; 1024^2 10.3 and 10.9, 12.2 and 13.0.  With the jet:
+        // 256 x 144 3.45 and 3.21, 384 x 216 4.55 and 4.47, 512 x 288 5.64 and 5.83.
+        const bh_launch_params wide{64, 1, 32, 0, 2};
+        const long long lanes = static_cast<long long>(ctx->sm_count) * 64 *
+                                std::max(1, trace_blocks_per_sm(BH_PRECISION_FP64, 64, true));
+        if (rays <= (any_jet ? 3 : 4) * lanes) lp = wide;
+    }
     int bps = lp.blocks_per_sm > 0 ? lp.blocks_per_sm : trace_blocks_per_sm(prec, lp.block_size, lp.reg_variant == 2);
     if (bps < 1) bps = 1;
     TraceLaunch& tl = p.tl;
@@ -343,27 +349,16 @@ int plan_launch(bh_ctx* ctx, std::vector<FrameParams>& frames, bh_xyz* d_pixels,
     tl.jet = any_jet ? static_cast<double*>(ctx->jet.p) : nullptr;
     tl.surfaces = any_surface ? 1 : 0;
     if (p.mixed && any_near_critical) {
-        // Near-critical rays in binary64 on kSideBlocks blocks beside the
-        // binary32 kernel.  The binary32 grid gives up the slots those blocks
-        // take, so that both are resident at once whichever is placed first;
-        // as many binary32 blocks start in those slots after them.
+        // Near-critical rays in binary64 beside the binary32 kernel, on as
+        // many blocks as fit: those without a ray end at once.
         tl.near_critical = 1;
-        tl.grid_side = std::min(kSideBlocks, ctx->sm_count);
+        tl.grid_side = ctx->sm_count * std::max(1, trace_blocks_per_sm(BH_PRECISION_FP64, 64, true));
         tl.frames_side = static_cast<const FrameParams*>(ctx->frames.p) + n;
         tl.side_stream = ctx->side_stream;
         tl.fork_event = ctx->fork_event;
         tl.join_event = ctx->join_event;
         tl.sel_flag = static_cast<unsigned char*>(ctx->sel_flag.p);
         tl.sel_list = static_cast<int*>(ctx->sel_list.p);
-        tl.grid_list = ctx->sm_count * std::max(1, trace_blocks_per_sm(BH_PRECISION_FP64, 128, 0));
-        if (lp.blocks_per_sm <= 0) {
-            const long long side_regs = 4 * warp_regs(trace_registers(BH_PRECISION_FP64, 0));
-            const long long block_regs = (lp.block_size / 32) * warp_regs(trace_registers(prec, tl.reg_variant));
-            const int beside = block_regs > 0 ? static_cast<int>((kSmRegs - side_regs) / block_regs) : bps;
-            const int lost = std::max(0, bps - std::max(0, beside));
-            tl.grid_late = std::min(tl.grid - 1, tl.grid_side * lost);
-            tl.grid -= tl.grid_late;
-        }
     }
 
     ShadeLaunch& sl = p.sl;
@@ -1209,6 +1204,7 @@ int bh_gpu_set_launch(bh_ctx* ctx, int precision, const bh_launch_params* p) {
     if (n.block_size * trace_registers(precision, n.reg_variant == 2) > 65536)
         return fail(ctx, BH_ERR_INVALID_ARG, "block_size too large for the kernel's register count");
     ctx->launch[slot] = n;
+    ctx->launch_set[slot] = true;
     return BH_OK;
 }
 
@@ -1233,6 +1229,8 @@ static int autotune_impl(bh_ctx* ctx, const bh_render_config* cfgs, int n, bh_la
         return fail(ctx, BH_ERR_INVALID_ARG, "unknown precision");
     const int slot = prec == BH_PRECISION_MIXED ? 1 : 0;
     const bh_launch_params keep = ctx->launch[slot];
+    const bool keep_set = ctx->launch_set[slot];
+    ctx->launch_set[slot] = true;
     std::vector<std::vector<bh_xyz>> px(n);
     std::vector<bh_xyz*> outs(n);
     for (int i = 0; i < n; ++i) {
@@ -1256,6 +1254,7 @@ static int autotune_impl(bh_ctx* ctx, const bh_render_config* cfgs, int n, bh_la
                                       : bh_gpu_render_batch(ctx, cfgs, n, outs.data(), st.data());
                         if (rc != BH_OK) {
                             ctx->launch[slot] = keep;
+                            ctx->launch_set[slot] = keep_set;
                             return rc;
                         }
                         ms = std::min(ms, st[0].kernel_ms);

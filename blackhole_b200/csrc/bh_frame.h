@@ -147,7 +147,6 @@ struct QueueState {
     unsigned long long resume_next;  // next unclaimed deferred ray
     unsigned long long select_next;  // next near-critical ray the binary64 kernel takes (list or scan)
     unsigned long long selected;     // near-critical rays the classification pass listed
-    unsigned long long select_next2; // next listed ray of the binary64 pass after the binary32 kernels
     int32_t abort;                   // set by the host (1) or by the budget check (2)
     int32_t status;
 };

@@ -183,7 +183,7 @@ extern "C" int bh_gpu_trace_noalloc(int device, const bh_render_config* cfg, bh_
     // Near-critical rays in binary64 as the context API traces them, here
     // before the binary32 kernel on the caller's stream (no stream of our own).
     tl.near_critical = F.fp64_near_critical;
-    tl.grid_side = sms;
+    tl.grid_side = 2 * sms;
     tl.frames_side = frame_side;
     tl.side_stream = nullptr;
     return launch_trace(tl, s) == cudaSuccess ? BH_OK : BH_ERR_CUDA;

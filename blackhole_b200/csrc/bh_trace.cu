@@ -558,9 +558,6 @@ struct TraceArgs {
     int select;              // 0: every ray; 1: near-critical rays only; 2: all others
     const unsigned char* sel_flag;   // per ray: kRay* class from the classification pass, or null
     const int* sel_list;     // the near-critical rays' global ids, or null (then select 1 scans)
-    long long list_cap;      // select 1 with a list: the rays [0, list_cap) beside the binary32
-                             // kernel (phase 0), the rest [list_cap, ..) after it (phase 1)
-    int phase;
     unsigned int* band_done; // finished rays per row band, or null
     long long rays_per_band;
 };
@@ -689,7 +686,7 @@ __device__ bool start_ray(const TraceArgs& A, Lane<P>& L, long long id) {
         L.gid = dr->gid;
         L.frame = dr->frame;
     } else {
-        L.gid = (A.select == 1 && A.sel_list) ? A.sel_list[id + (A.phase ? A.list_cap : 0)] : (int)id;
+        L.gid = (A.select == 1 && A.sel_list) ? A.sel_list[id] : (int)id;
         // the binary32 kernel leaves the listed rays to the binary64 one
         if (A.select == 2 && A.sel_flag && A.sel_flag[L.gid] == kRayBinary64) return false;
         L.frame = find_frame(A.frame_ray_end, A.nframes, L.gid);
@@ -1299,13 +1296,7 @@ __global__ void __maxnreg__(MAXREG) trace_kernel(TraceArgs A) {
     unsigned long long* counter = RESUME ? &A.queue->resume_next
                                            : (A.select == 1 ? &A.queue->select_next : &A.queue->next);
     if (!RESUME && A.select == 1 && A.sel_list) {
-        const long long listed = (long long)*(volatile unsigned long long*)&A.queue->selected;
-        if (A.phase == 0) {
-            total = listed < A.list_cap ? listed : A.list_cap;
-        } else {
-            total = listed > A.list_cap ? listed - A.list_cap : 0;
-            counter = &A.queue->select_next2;
-        }
+        total = (long long)*(volatile unsigned long long*)&A.queue->selected;
     }
     Lane<P> L;
     bool active = false, done = false;
@@ -1385,6 +1376,7 @@ constexpr int kRegMixed = 128;
 constexpr int kRegMixedWide = 168;
 constexpr int kRegFp64 = 168;
 constexpr int kRegFp64Wide = 232;
+constexpr int kSideBlock = 64;   // threads per block of the near-critical kernel beside a mixed launch
 
 // The right-hand side the trace kernels integrate, evaluated at given
 // states (known-answer tests of the device arithmetic): in = 8 doubles per
@@ -1424,14 +1416,11 @@ __global__ void eval_rhs_kernel(const FrameParams* __restrict__ Fp, const double
 }
 
 template <class P, int MAXREG, bool JET, int SURF, bool RESUME = false>
-cudaError_t launch_t(const TraceLaunch& L, int grid, int block, cudaStream_t s, int select = 0,
-                     int phase = 0) {
+cudaError_t launch_t(const TraceLaunch& L, int grid, int block, cudaStream_t s, int select = 0) {
     TraceArgs A;
     A.frames = (select == 1) ? L.frames_side : L.frames;
     A.sel_flag = select ? L.sel_flag : nullptr;
     A.sel_list = (select == 1) ? L.sel_list : nullptr;
-    A.list_cap = (long long)L.grid_side * 128;
-    A.phase = phase;
     A.frame_ray_end = L.frame_ray_end;
     A.nframes = L.nframes;
     A.total_rays = L.total_rays;
@@ -1442,11 +1431,11 @@ cudaError_t launch_t(const TraceLaunch& L, int grid, int block, cudaStream_t s, 
     A.refill = L.refill < 1 ? 1 : (L.refill > 32 ? 32 : L.refill);
     A.select = select;
     if (select == 1) {
-        // few rays found among many looked at: refill a lane as soon as it
-        // is idle, one id at a time, so a lane tracing a ray does not hold
-        // up the search of the other 31
+        // Without a list few rays are found among many looked at: refill a
+        // lane as soon as it is idle, one id at a time, so a lane tracing a ray
+        // does not hold up the search of the other 31.
         A.rays_per_thread = 1;
-        A.refill = 1;
+        A.refill = L.sel_list ? 32 : 1;
     }
     A.budget = L.budget;
     A.jet = L.jet;
@@ -1456,6 +1445,9 @@ cudaError_t launch_t(const TraceLaunch& L, int grid, int block, cudaStream_t s, 
     trace_kernel<P, MAXREG, JET, SURF, RESUME><<<grid, block, 0, s>>>(A);
     return cudaGetLastError();
 }
+
+// Does nothing (it orders two launches, see launch_trace_t).
+__global__ void gate_kernel() {}
 
 // Raises each band counter to its band's ray count (after the trace kernels).
 __global__ void band_release_kernel(unsigned int* band_done, int nbands, long long total, long long per_band) {
@@ -1521,12 +1513,11 @@ cudaError_t launch_trace_t(const TraceLaunch& L, cudaStream_t stream) {
         cudaError_t e;
         const bool side = L.near_critical && L.side_stream && L.fork_event && L.join_event;
         if (L.near_critical) {
-            // The near-critical rays in binary64 (the kernel of the binary64
-            // path's default cap, blocks of 128: the same arithmetic as a
-            // binary64 frame) beside the binary32 launch (the two
-            // share no data but the queue's separate counters and never wait
-            // on each other), or before it on the same stream.  With a flag
-            // array, a classification pass lists them first.
+            // The near-critical rays in binary64 (the binary64 path's
+            // arithmetic) beside the binary32 launch (the two share no data
+            // but the queue's separate counters and never wait on each
+            // other), or before it on the same stream.  With a flag array, a
+            // classification pass lists them first.
             if (L.sel_flag) {
                 const long long want = (L.total_rays + 255) / 256;
                 const int cgrid = (int)(want < 4LL * L.grid ? want : 4LL * L.grid);
@@ -1536,36 +1527,41 @@ cudaError_t launch_trace_t(const TraceLaunch& L, cudaStream_t stream) {
                 if ((e = cudaGetLastError()) != cudaSuccess) return e;
             }
         }
-        // Beside: the binary32 kernel on the side stream from the fork on, with
-        // the block slots the binary64 kernel's blocks leave; on `stream` the
-        // binary64 kernel, then binary32 blocks for those slots, which take
-        // from the same queue whatever is left when the binary64 blocks are
-        // done (neither kernel waits for the other).  The pass over rays the
-        // binary32 kernels hand over runs after both, on `stream`.
+        // Beside: the binary32 kernel on the side stream from the fork on.  The
+        // binary64 kernel's grid could fill the GPU, a lane per listed ray in
+        // flight; its blocks that find no ray left end at once, and the
+        // binary32 kernel's blocks take the slots they leave.  So the long
+        // serial chains start first and end in the shadow of the binary32
+        // work, however many rays are listed.  (On 32 blocks, with the rest
+        // of a long list after the binary32 kernel: 2048^2 photon ring 8.1
+        // against 7.7 ms, 16 frames of 256^2 to 1024^2 20.1 against 18.9, M87
+        // jets 7.9 against 7.3.)  The wide register cap: fewer lanes, but a
+        // lone ray's attempt takes a quarter less (161 x 90 preview 1.24
+        // against 1.07 ms; the large frames the same).
         const int sel = L.near_critical ? 2 : 0;
-        auto launch32 = [&](int grid, cudaStream_t s) {
-            return L.reg_variant ? launch_t<Mixed, kRegMixedWide, JET, SURF>(L, grid, L.block_size, s, sel)
-                                 : launch_t<Mixed, kRegMixed, JET, SURF>(L, grid, L.block_size, s, sel);
-        };
+        cudaStream_t s32 = side ? L.side_stream : stream;
         if (side) {
             if ((e = cudaEventRecord(L.fork_event, stream)) != cudaSuccess) return e;
             if ((e = cudaStreamWaitEvent(L.side_stream, L.fork_event, 0)) != cudaSuccess) return e;
         }
         if (L.near_critical &&
-            (e = launch_t<Fp64, kRegFp64, JET, SURF>(L, L.grid_side, 128, stream, 1)) != cudaSuccess)
+            (e = launch_t<Fp64, kRegFp64Wide, JET, SURF>(L, L.grid_side, kSideBlock, stream, 1)) != cudaSuccess)
             return e;
-        if ((e = launch32(L.grid, side ? L.side_stream : stream)) != cudaSuccess) return e;
         if (side) {
-            if (L.grid_late > 0 && (e = launch32(L.grid_late, stream)) != cudaSuccess) return e;
+            // An empty kernel before the binary32 one: both kernels are ready
+            // at the fork, and the binary64 blocks are to be placed first (the
+            // other way round they wait for the persistent binary32 blocks to
+            // end: 3.3 against 2.7 ms per 1024^2 frame).
+            gate_kernel<<<1, 32, 0, s32>>>();
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        }
+        e = L.reg_variant ? launch_t<Mixed, kRegMixedWide, JET, SURF>(L, L.grid, L.block_size, s32, sel)
+                          : launch_t<Mixed, kRegMixed, JET, SURF>(L, L.grid, L.block_size, s32, sel);
+        if (e != cudaSuccess) return e;
+        if (side) {
             if ((e = cudaEventRecord(L.join_event, L.side_stream)) != cudaSuccess) return e;
             if ((e = cudaStreamWaitEvent(stream, L.join_event, 0)) != cudaSuccess) return e;
         }
-        // Listed near-critical rays beyond one per lane of the binary64 kernel
-        // beside (a frame dense in them, like one centred on the photon ring):
-        // on the whole GPU once the binary32 kernels are done.
-        if (L.near_critical && L.sel_list &&
-            (e = launch_t<Fp64, kRegFp64, JET, SURF>(L, L.grid_list, 128, stream, 1, 1)) != cudaSuccess)
-            return e;
         if (L.resume_event) cudaEventRecord(L.resume_event, stream);
         // The deferred rays, in binary64 under the wide register cap: every
         // block reads the deferred count.

@@ -319,8 +319,10 @@ int  bh_gpu_render_batch(bh_ctx* ctx, const bh_render_config* cfgs, int n,
                          bh_xyz* const* outs, bh_render_stats* stats);
 
 /* Launch shape of the trace kernel of `precision` (BH_PRECISION_*, or -1 for
-   both) used by the next calls; zero fields keep the current value.  The
-   binary64 pass that finishes mixed-precision rays uses the FP64 shape. */
+   both) used by the next calls; zero fields keep the current value.  While no
+   shape has been set (or tuned), binary64 launches of few rays run blocks of
+   64 under the wide register cap; the shape does not change results.  The
+   binary64 passes of a mixed launch have shapes of their own. */
 int  bh_gpu_set_launch(bh_ctx* ctx, int precision, const bh_launch_params* p);
 int  bh_gpu_get_launch(const bh_ctx* ctx, int precision, bh_launch_params* p);
 

@@ -97,3 +97,23 @@ def test_rays_past_the_poles(renderer, orc, theta_deg, spin, precision):
     assert np.quantile(np.abs(got["g"][disc] / chk["g"][disc] - 1.0), 0.95) <= g_tol
     d = np.linalg.norm(got["dir"][sky] - chk["dir"][sky], axis=1)
     assert np.quantile(d, 0.95) <= d_tol
+
+
+@pytest.mark.parametrize("width,height,jet", [(9, 4, False), (388, 390, False), (389, 390, False), (447, 254, True),
+                                              (449, 254, True)])
+def test_launch_shape_does_not_change_binary64_frames(width, height, jet):
+    """On both sides of the ray counts where the library picks another register
+    cap (four and three waves of lanes on 148 SMs), and at a frame of one partial
+    warp: the same bits as under the tight cap."""
+    from blackhole_b200 import Renderer, workloads
+
+    cfg = workloads.quasar_jets(width, height) if jet else workloads.kerr_fp64_256()
+    cfg.width, cfg.height, cfg.star_count = width, height, 20000
+    with Renderer(0) as r:
+        auto = r.trace_rays(cfg)
+        r.set_launch(block_size=128, rays_per_thread=1, refill=32, reg_variant=1, precision=abi.PRECISION_FP64)
+        tight = r.trace_rays(cfg)
+    for k in ("what", "steps", "attempts", "y", "g", "dir"):
+        assert np.array_equal(auto[k], tight[k]), k
+    # the jet's sum is rounded by each kernel as it was compiled
+    assert np.allclose(auto["jet"], tight["jet"], rtol=1e-11, atol=1e-14 * max(1e-300, tight["jet"].max()))
