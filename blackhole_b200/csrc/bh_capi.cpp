@@ -12,6 +12,7 @@
 #include <atomic>
 #include <chrono>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <cstdlib>
@@ -82,7 +83,11 @@ struct bh_ctx {
     DevBuf adj_target, adj_grad, adj_Y, adj_ckpt, adj_counters, adj_sums, adj_xr, adj_cand, adj_edge, adj_high, adj_rays;
     DevBuf band_done;
     // Display transform: blur scratch, glare weights, meter state, 8-bit output.
-    DevBuf disp_tmp, disp_near, disp_far, disp_k, disp_state, disp_rgb;
+    DevBuf disp_tmp, disp_near, disp_far, disp_k, disp_state, disp_rgb, disp_frames;
+    // A film's images are copied out on copy_stream, each group of frames
+    // after its event.
+    cudaStream_t copy_stream = nullptr;
+    cudaEvent_t disp_done[4] = {};
     // bh_gpu_eval: inputs and outputs.
     DevBuf eval_in, eval_out;
     QueueState* d_queue = nullptr;
@@ -104,6 +109,10 @@ struct bh_ctx {
 namespace {
 
 constexpr int kReduceBlocks = 512;
+// A display group's pixels at most (a quarter of a film, or this), and the
+// groups whose copies can be outstanding.
+constexpr size_t kDisplayGroupPixels = 16u << 20;
+constexpr size_t kDisplayEvents = 4;
 int fail(bh_ctx* ctx, int code, const std::string& msg) {
     if (ctx) ctx->err = msg;
     return code;
@@ -635,6 +644,9 @@ int bh_gpu_create(int device, bh_ctx** out) {
     if ((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess) return bail(e);
     if ((e = cudaStreamCreateWithFlags(&ctx->abort_stream, cudaStreamNonBlocking)) != cudaSuccess) return bail(e);
     if ((e = cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking)) != cudaSuccess) return bail(e);
+    if ((e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking)) != cudaSuccess) return bail(e);
+    for (auto& ev : ctx->disp_done)
+        if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return bail(e);
     if ((e = cudaEventCreateWithFlags(&ctx->fork_event, cudaEventDisableTiming)) != cudaSuccess) return bail(e);
     if ((e = cudaEventCreateWithFlags(&ctx->join_event, cudaEventDisableTiming)) != cudaSuccess) return bail(e);
     if ((e = cudaMalloc(&ctx->d_queue, sizeof(QueueState))) != cudaSuccess) return bail(e);
@@ -660,7 +672,7 @@ void bh_gpu_destroy(bh_ctx* ctx) {
                       &ctx->pix_end, &ctx->partials, &ctx->fstats, &ctx->jet, &ctx->adj_target, &ctx->adj_grad, &ctx->adj_Y,
                       &ctx->adj_ckpt, &ctx->adj_counters, &ctx->adj_sums, &ctx->adj_xr, &ctx->adj_cand, &ctx->adj_edge,
                       &ctx->adj_high, &ctx->adj_rays, &ctx->eval_in, &ctx->eval_out, &ctx->disp_tmp, &ctx->disp_near,
-                      &ctx->disp_far, &ctx->disp_k, &ctx->disp_state, &ctx->disp_rgb, &ctx->sel_flag,
+                      &ctx->disp_far, &ctx->disp_k, &ctx->disp_state, &ctx->disp_rgb, &ctx->disp_frames, &ctx->sel_flag,
                       &ctx->sel_list, &ctx->band_done})
         if (b->p) cudaFree(b->p);
     cudaFree(ctx->d_table);
@@ -682,6 +694,9 @@ void bh_gpu_destroy(bh_ctx* ctx) {
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->abort_stream) cudaStreamDestroy(ctx->abort_stream);
     if (ctx->side_stream) cudaStreamDestroy(ctx->side_stream);
+    if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
+    for (auto& ev : ctx->disp_done)
+        if (ev) cudaEventDestroy(ev);
     if (ctx->fork_event) cudaEventDestroy(ctx->fork_event);
     if (ctx->join_event) cudaEventDestroy(ctx->join_event);
     delete ctx;
@@ -965,23 +980,35 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
     return BH_OK;
 }
 
-// The display transform of the W x H frame at d_pixels (device), on
-// ctx->stream; copies the 8-bit image and the exposure back and synchronises.
-static int display_impl(bh_ctx* ctx, const bh_display* d, bh_xyz* d_pixels, int width, int height,
-                        uint8_t* out_rgb, double* exposure_used) {
+// One frame of display_impl: its pixels on the device and where its bytes go.
+struct DisplayJob {
+    bh_xyz* pixels;
+    int width, height;
+    uint8_t* out;          // host, or null
+};
+
+// Enqueues the copies of group g's images, after its event.
+static int copy_group(bh_ctx* ctx, const DisplayJob* jobs, const DisplayFrame* frames,
+                      const std::vector<int>& group_end, size_t g) {
+    CK(cudaStreamWaitEvent(ctx->copy_stream, ctx->disp_done[g % kDisplayEvents], 0));
+    for (int i = g ? group_end[g - 1] : 0; i < group_end[g]; ++i)
+        if (jobs[i].out)
+            CK(cudaMemcpyAsync(jobs[i].out, frames[i].rgb, static_cast<size_t>(jobs[i].width) * jobs[i].height * 3,
+                               cudaMemcpyDeviceToHost, ctx->copy_stream));
+    return BH_OK;
+}
+
+// The display transform of n frames (device), on ctx->stream; copies the 8-bit
+// images and the exposures back and synchronises.
+static int display_impl(bh_ctx* ctx, const bh_display* d, const DisplayJob* jobs, int n, double* exposures) {
     if (!(d->glare >= 0.0 && d->glare <= 1.0)) return fail(ctx, BH_ERR_INVALID_ARG, "glare must be in [0, 1]");
     if (d->tonemap < BH_TONEMAP_LINEAR || d->tonemap > BH_TONEMAP_HDR)
         return fail(ctx, BH_ERR_INVALID_ARG, "unknown tonemap");
-    const size_t npx = static_cast<size_t>(width) * height;
     int rc;
     DisplayLaunch L;
     std::memset(&L, 0, sizeof L);
-    L.pixels = d_pixels;
-    L.width = width;
-    L.height = height;
-    L.glare = d->glare;
-    L.glare_radius = d->glare_radius;
-    if (d->glare > 0.0 && d->glare_radius > 0.0) {
+    const bool glare = d->glare > 0.0 && d->glare_radius > 0.0;
+    if (glare) {
         // img::add_glare's kernels (image.cpp:61-68), normalised on the host.
         std::vector<double> w;
         int r[2];
@@ -997,38 +1024,121 @@ static int display_impl(bh_ctx* ctx, const bh_display* d, bh_xyz* d_pixels, int 
             for (double& v : k) v /= sum;
             w.insert(w.end(), k.begin(), k.end());
         }
-        if ((rc = ensure(ctx, ctx->disp_k, w.size() * sizeof(double))) != BH_OK) return rc;
-        for (DevBuf* b : {&ctx->disp_tmp, &ctx->disp_near, &ctx->disp_far})
-            if ((rc = ensure(ctx, *b, npx * sizeof(bh_xyz))) != BH_OK) return rc;
-        CK(cudaMemcpyAsync(ctx->disp_k.p, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice,
-                           ctx->stream));
-        ctx->h2d += static_cast<long long>(w.size() * sizeof(double));
-        L.k_near = static_cast<const double*>(ctx->disp_k.p);
-        L.k_far = L.k_near + (2 * r[0] + 1);
-        L.r_near = r[0];
-        L.r_far = r[1];
-        L.tmp = static_cast<bh_xyz*>(ctx->disp_tmp.p);
-        L.nearp = static_cast<bh_xyz*>(ctx->disp_near.p);
-        L.farp = static_cast<bh_xyz*>(ctx->disp_far.p);
+        L.w.r_near = r[0];
+        L.w.r_far = r[1];
+        L.w.core = 1.0 - d->glare;
+        L.w.a = 0.7 * d->glare;
+        L.w.b = 0.3 * d->glare;
+        L.glare = (r[0] <= kGlareMaxRadius && r[1] <= kGlareMaxRadius) ? 1 : 2;
+        if (L.glare == 1) {
+            std::copy(w.begin(), w.begin() + 2 * r[0] + 1, L.w.near_w);
+            std::copy(w.begin() + 2 * r[0] + 1, w.end(), L.w.far_w);
+        } else {
+            if ((rc = ensure(ctx, ctx->disp_k, w.size() * sizeof(double))) != BH_OK) return rc;
+            CK(cudaMemcpyAsync(ctx->disp_k.p, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice,
+                               ctx->stream));
+            ctx->h2d += static_cast<long long>(w.size() * sizeof(double));
+            L.k_near = static_cast<const double*>(ctx->disp_k.p);
+            L.k_far = L.k_near + (2 * r[0] + 1);
+        }
     }
-    if ((rc = ensure(ctx, ctx->disp_state, sizeof(ExposureState) + 2 * sizeof(double))) != BH_OK) return rc;
-    if (out_rgb && (rc = ensure(ctx, ctx->disp_rgb, npx * 3)) != BH_OK) return rc;
+    // Frames in groups: the glare scratch stays bounded, and a film's images
+    // are copied out while the next group is developed.
+    std::vector<DisplayFrame> frames(n);
+    std::vector<int> group_end;
+    size_t rgb_bytes = 0, scratch = 0, group_px = 0, total_px = 0;
+    for (int i = 0; i < n; ++i) total_px += static_cast<size_t>(jobs[i].width) * jobs[i].height;
+    const size_t group_most = std::max<size_t>(std::min(total_px / 4 + 1, kDisplayGroupPixels), 1);
+    bool develop = false;
+    for (int i = 0; i < n; ++i) {
+        const size_t npx = static_cast<size_t>(jobs[i].width) * jobs[i].height;
+        const int group_begin = group_end.empty() ? 0 : group_end.back();
+        if (group_px > 0 && (group_px + npx > group_most || i - group_begin >= 32768)) {
+            group_end.push_back(i);
+            group_px = 0;
+        }
+        DisplayFrame& f = frames[i];
+        f = DisplayFrame{jobs[i].pixels, nullptr, static_cast<long long>(group_px), jobs[i].width, jobs[i].height, i, 0};
+        group_px += npx;
+        scratch = std::max(scratch, group_px);
+        rgb_bytes += npx * 3;
+        develop = develop || jobs[i].out;
+    }
+    group_end.push_back(n);
+    if (develop && (rc = ensure(ctx, ctx->disp_rgb, rgb_bytes)) != BH_OK) return rc;
+    if (develop) {
+        uint8_t* p = static_cast<uint8_t*>(ctx->disp_rgb.p);
+        for (int i = 0; i < n; ++i) {
+            frames[i].rgb = p;
+            p += static_cast<size_t>(jobs[i].width) * jobs[i].height * 3;
+        }
+    }
+    if (glare) {
+        for (DevBuf* b : {&ctx->disp_near, &ctx->disp_far})
+            if ((rc = ensure(ctx, *b, scratch * sizeof(bh_xyz))) != BH_OK) return rc;
+        if (L.glare == 2 && (rc = ensure(ctx, ctx->disp_tmp, scratch * sizeof(bh_xyz))) != BH_OK) return rc;
+        L.tmp_near = static_cast<bh_xyz*>(ctx->disp_near.p);
+        L.tmp_far = static_cast<bh_xyz*>(ctx->disp_far.p);
+        L.tmp = static_cast<bh_xyz*>(ctx->disp_tmp.p);
+    }
+    const bool meter = !(d->exposure > 0.0);
+    if ((rc = ensure(ctx, ctx->disp_frames, n * sizeof(DisplayFrame))) != BH_OK) return rc;
+    CK(cudaMemcpyAsync(ctx->disp_frames.p, frames.data(), n * sizeof(DisplayFrame), cudaMemcpyHostToDevice,
+                       ctx->stream));
+    ctx->h2d += static_cast<long long>(n * sizeof(DisplayFrame));
+    if (meter) {
+        if ((rc = ensure(ctx, ctx->disp_state, n * sizeof(ExposureState))) != BH_OK) return rc;
+        CK(cudaMemsetAsync(ctx->disp_state.p, 0, n * sizeof(ExposureState), ctx->stream));
+    }
     L.exposure = d->exposure;
     L.key = d->key;
-    L.state = static_cast<ExposureState*>(ctx->disp_state.p);
-    L.exposure_out = reinterpret_cast<double*>(static_cast<unsigned char*>(ctx->disp_state.p) + sizeof(ExposureState));
-    L.reduce_blocks = ctx->sm_count * 4;
+    L.states = static_cast<ExposureState*>(ctx->disp_state.p);
+    L.sm_count = ctx->sm_count;
+    L.develop = develop ? 1 : 0;
     L.tonemap = d->tonemap;
     L.log_k = std::pow(10.0, std::min(std::max(d->log_decades, 1.0), 20.0));
     L.denom = std::log10(1.0 + L.log_k);
-    L.rgb = out_rgb ? static_cast<uint8_t*>(ctx->disp_rgb.p) : nullptr;
-    CK(launch_display(L, ctx->stream));
-    double e = 0.0;
-    CK(cudaMemcpyAsync(&e, L.exposure_out, sizeof e, cudaMemcpyDeviceToHost, ctx->stream));
-    if (out_rgb) CK(cudaMemcpyAsync(out_rgb, ctx->disp_rgb.p, npx * 3, cudaMemcpyDeviceToHost, ctx->stream));
+    for (size_t g = 0, i = 0; g < group_end.size(); ++g) {
+        L.frames = static_cast<const DisplayFrame*>(ctx->disp_frames.p) + i;
+        L.h_frames = frames.data() + i;
+        L.n = group_end[g] - static_cast<int>(i);
+        L.max_width = L.max_height = 0;
+        L.max_pixels = 0;
+        for (size_t j = i; j < i + L.n; ++j) {
+            L.max_width = std::max(L.max_width, frames[j].width);
+            L.max_height = std::max(L.max_height, frames[j].height);
+            L.max_pixels = std::max(L.max_pixels, static_cast<long long>(frames[j].width) * frames[j].height);
+        }
+        CK(launch_display(L, ctx->stream));
+        if (group_end.size() > 1) CK(cudaEventRecord(ctx->disp_done[g % kDisplayEvents], ctx->stream));
+        // copies of an earlier group, on their own stream, once the event of
+        // this one is about to be reused
+        i = group_end[g];
+        if (group_end.size() > 1 && g + 1 >= kDisplayEvents) {
+            if ((rc = copy_group(ctx, jobs, frames.data(), group_end, g + 1 - kDisplayEvents)) != BH_OK) return rc;
+        }
+    }
+    if (group_end.size() > 1) {
+        const size_t from = group_end.size() >= kDisplayEvents ? group_end.size() - kDisplayEvents + 1 : 0;
+        for (size_t g = from; g < group_end.size(); ++g)
+            if ((rc = copy_group(ctx, jobs, frames.data(), group_end, g)) != BH_OK) return rc;
+    } else {
+        for (int i = 0; i < n; ++i)
+            if (jobs[i].out)
+                CK(cudaMemcpyAsync(jobs[i].out, frames[i].rgb, static_cast<size_t>(jobs[i].width) * jobs[i].height * 3,
+                                   cudaMemcpyDeviceToHost, ctx->stream));
+    }
+    if (develop) ctx->d2h += static_cast<long long>(rgb_bytes);
+    if (meter) {
+        CK(cudaMemcpy2DAsync(exposures, sizeof(double),
+                             static_cast<const unsigned char*>(ctx->disp_state.p) + offsetof(ExposureState, exposure),
+                             sizeof(ExposureState), sizeof(double), n, cudaMemcpyDeviceToHost, ctx->stream));
+        ctx->d2h += static_cast<long long>(n * sizeof(double));
+    } else {
+        std::fill(exposures, exposures + n, d->exposure);
+    }
+    if (group_end.size() > 1) CK(cudaStreamSynchronize(ctx->copy_stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    ctx->d2h += static_cast<long long>(sizeof e + (out_rgb ? npx * 3 : 0));
-    if (exposure_used) *exposure_used = e;
     return BH_OK;
 }
 
@@ -1065,7 +1175,11 @@ int bh_gpu_develop(bh_ctx* ctx, const bh_xyz* pixels, int width, int height, con
     if ((rc = ensure(ctx, ctx->pixels, npx * sizeof(bh_xyz))) != BH_OK) return rc;
     CK(cudaMemcpyAsync(ctx->pixels.p, pixels, npx * sizeof(bh_xyz), cudaMemcpyHostToDevice, ctx->stream));
     ctx->h2d += static_cast<long long>(npx * sizeof(bh_xyz));
-    return display_impl(ctx, d, static_cast<bh_xyz*>(ctx->pixels.p), width, height, out_rgb, exposure_used);
+    const DisplayJob job{static_cast<bh_xyz*>(ctx->pixels.p), width, height, out_rgb};
+    double e = 0.0;
+    if ((rc = display_impl(ctx, d, &job, 1, &e)) != BH_OK) return rc;
+    if (exposure_used) *exposure_used = e;
+    return BH_OK;
 }
 
 int bh_gpu_render_rgb(bh_ctx* ctx, const bh_render_config* cfg, const bh_display* d, uint8_t* out_rgb,
@@ -1081,9 +1195,10 @@ int bh_gpu_render_rgb(bh_ctx* ctx, const bh_render_config* cfg, const bh_display
     if ((rc = ensure(ctx, ctx->pixels, npx * sizeof(bh_xyz))) != BH_OK) return rc;
     if ((rc = enqueue(ctx, frames, static_cast<bh_xyz*>(ctx->pixels.p), nullptr, ctx->stream, true)) != BH_OK)
         return rc;
-    if ((rc = display_impl(ctx, d, static_cast<bh_xyz*>(ctx->pixels.p), cfg->width, cfg->height, out_rgb,
-                           exposure_used)) != BH_OK)
-        return rc;
+    const DisplayJob job{static_cast<bh_xyz*>(ctx->pixels.p), cfg->width, cfg->height, out_rgb};
+    double e = 0.0;
+    if ((rc = display_impl(ctx, d, &job, 1, &e)) != BH_OK) return rc;
+    if (exposure_used) *exposure_used = e;
     const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return finish(ctx, 1, stats, nullptr, true, secs);
 }
@@ -1102,15 +1217,15 @@ int bh_gpu_render_batch_rgb(bh_ctx* ctx, const bh_render_config* cfgs, int n, co
     if ((rc = ensure(ctx, ctx->pixels, npx * sizeof(bh_xyz))) != BH_OK) return rc;
     if ((rc = enqueue(ctx, frames, static_cast<bh_xyz*>(ctx->pixels.p), nullptr, ctx->stream, true)) != BH_OK)
         return rc;
+    std::vector<DisplayJob> jobs(n);
+    std::vector<double> used(n);
     size_t off = 0;
     for (int i = 0; i < n; ++i) {
-        double e = 0.0;
-        rc = display_impl(ctx, d, static_cast<bh_xyz*>(ctx->pixels.p) + off, cfgs[i].width, cfgs[i].height,
-                          outs_rgb[i], &e);
-        if (rc != BH_OK) return rc;
-        if (exposure_used) exposure_used[i] = e;
+        jobs[i] = DisplayJob{static_cast<bh_xyz*>(ctx->pixels.p) + off, cfgs[i].width, cfgs[i].height, outs_rgb[i]};
         off += static_cast<size_t>(cfgs[i].width) * cfgs[i].height;
     }
+    if ((rc = display_impl(ctx, d, jobs.data(), n, used.data())) != BH_OK) return rc;
+    if (exposure_used) std::copy(used.begin(), used.end(), exposure_used);
     const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return finish(ctx, n, stats, nullptr, true, secs);
 }

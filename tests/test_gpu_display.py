@@ -83,3 +83,32 @@ def test_bad_display_settings_are_refused(renderer):
         renderer.develop(img, tonemap=7)
     with pytest.raises(BHError):
         renderer.develop(img, glare=1.5)
+
+
+@pytest.mark.parametrize("shape,radius", [((1, 1), 3.0), ((2, 3), 6.6), ((65, 85), 6.6), ((64, 86), 6.7), ((63, 200), 0.2),
+                                          ((130, 32), 2.4)])
+def test_glare_at_the_edges_of_its_tiles(renderer, shape, radius):
+    """Frames smaller than the taps, ragged against the 256-element rows and the
+    64-row columns, and radii on both sides of the tiled kernels' largest (60
+    taps either way): the reference's sums in the reference's order, so the
+    same exposure and bytes as the restatement."""
+    o = oracle.oracle()
+    rng = np.random.default_rng(shape[0] * 1000 + shape[1])
+    img = np.exp(rng.normal(0.0, 3.0, size=shape + (3,)))
+    rgb, e = renderer.develop(img, glare=0.4, glare_radius=radius, tonemap=abi.TONEMAP_REINHARD)
+    g = o.add_glare(img, 0.4, radius)
+    assert e == o.auto_exposure(g)
+    _same_bytes(rgb, o.develop(g, e, abi.TONEMAP_REINHARD, 16.0))
+
+
+def test_film_of_uneven_frames_is_its_frames(renderer):
+    """Frames of several sizes in groups (more groups than outstanding copies),
+    glared and metered: frame by frame the single-frame call's bytes."""
+    base = kerr_a09_i60(width=8, height=8)
+    base.star_count = 1000
+    sizes = [(8, 8), (33, 5), (64, 48), (1, 7), (70, 41), (40, 64), (9, 90), (64, 64), (17, 3), (50, 50)]
+    cfgs = [base.replace(width=w, height=h) for w, h in sizes]
+    film, used = renderer.render_batch_rgb(cfgs, glare=0.3, glare_radius=2.0)
+    for c, rgb, e in zip(cfgs, film, used):
+        single, e1 = renderer.render_rgb(c, glare=0.3, glare_radius=2.0)
+        assert e == e1 and np.array_equal(rgb, single)
