@@ -76,7 +76,7 @@ struct bh_ctx {
     int32_t* d_bin_start = nullptr;
     HostSky sky_meta;
 
-    DevBuf hits, pixels, rays, lum, frames, ray_end, pix_end, partials, fstats, deferred, jet;
+    DevBuf hits, pixels, rays, frames, ray_end, partials, fstats, deferred, jet;
     DevBuf sel_flag, sel_list;         // near-critical classification of a mixed launch's rays
     // Adjoint: target image, per-ray gradients and luminances, checkpoint
     // slots, counters, sums and the edge pass's buffers.
@@ -108,7 +108,7 @@ struct bh_ctx {
 
 namespace {
 
-constexpr int kReduceBlocks = 512;
+constexpr int kShadeBlocks = 8192, kShadeBlocksLeast = 64;
 // A display group's pixels at most (a quarter of a film, or this), and the
 // groups whose copies can be outstanding.
 constexpr size_t kDisplayGroupPixels = 16u << 20;
@@ -235,7 +235,7 @@ void stats_add(bh_render_stats* s, const FrameStats& f) {
 struct Plan {
     int n = 0;
     int nf = 0;          // frames staged: n, or 2n with the binary64 treatment of mixed frames
-    long long rays = 0, pix = 0;
+    long long rays = 0;
     bool mixed = false;
     TraceLaunch tl;
     ShadeLaunch sl;
@@ -258,16 +258,17 @@ int plan_launch(bh_ctx* ctx, std::vector<FrameParams>& frames, bh_xyz* d_pixels,
         pix += static_cast<long long>(frames[i].width) * frames[i].height;
     }
     p.rays = rays;
-    p.pix = pix;
     int rc;
     if ((rc = ensure(ctx, ctx->hits, static_cast<size_t>(rays) * sizeof(HitRecord))) != BH_OK) return rc;
-    if ((rc = ensure(ctx, ctx->lum, static_cast<size_t>(pix) * sizeof(double))) != BH_OK) return rc;
     p.mixed = frames[0].precision_tag == BH_PRECISION_MIXED;
     p.nf = p.mixed ? 2 * n : n;
     if ((rc = ensure(ctx, ctx->frames, p.nf * sizeof(FrameParams))) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->ray_end, n * sizeof(long long))) != BH_OK) return rc;
-    if ((rc = ensure(ctx, ctx->pix_end, n * sizeof(long long))) != BH_OK) return rc;
-    if ((rc = ensure(ctx, ctx->partials, static_cast<size_t>(n) * kReduceBlocks * sizeof(FrameStats))) != BH_OK)
+    // shading blocks per frame: 8192 in all at most, 64 per frame at least
+    long long frame_px = 0;
+    for (int i = 0; i < n; ++i) frame_px = std::max(frame_px, static_cast<long long>(frames[i].width) * frames[i].height);
+    const int shade_grid = shade_blocks(frame_px, std::max(kShadeBlocks / n, kShadeBlocksLeast));
+    if ((rc = ensure(ctx, ctx->partials, static_cast<size_t>(n) * shade_grid * sizeof(double))) != BH_OK)
         return rc;
     if ((rc = ensure(ctx, ctx->fstats, n * sizeof(FrameStats))) != BH_OK) return rc;
     bool any_jet = false, any_surface = false, any_near_critical = false;
@@ -284,10 +285,10 @@ int plan_launch(bh_ctx* ctx, std::vector<FrameParams>& frames, bh_xyz* d_pixels,
         return rc;
 
     // Pinned staging: [frames][binary64 treatment of mixed frames][ray ends]
-    // [pixel ends][queue state].  The previous launch's copies out of it must
+    // [queue state].  The previous launch's copies out of it must
     // have completed.
     const size_t fbytes = static_cast<size_t>(p.nf) * sizeof(FrameParams);
-    p.stage_bytes = fbytes + 2 * n * sizeof(long long) + sizeof(QueueState);
+    p.stage_bytes = fbytes + n * sizeof(long long) + sizeof(QueueState);
     CK(cudaEventSynchronize(ctx->stage_free));
     if (p.stage_bytes > ctx->stage_cap) {
         if (ctx->stage) CK(cudaFreeHost(ctx->stage));
@@ -303,15 +304,12 @@ int plan_launch(bh_ctx* ctx, std::vector<FrameParams>& frames, bh_xyz* d_pixels,
         std::memcpy(s + i * sizeof(FrameParams), &g, sizeof g);
     }
     long long* ends = reinterpret_cast<long long*>(s + fbytes);
-    for (int i = 0; i < n; ++i) {
-        ends[i] = frames[i].ray_begin + frames[i].n_rays;
-        ends[n + i] = frames[i].pixel_begin + static_cast<long long>(frames[i].width) * frames[i].height;
-    }
+    for (int i = 0; i < n; ++i) ends[i] = frames[i].ray_begin + frames[i].n_rays;
     QueueState q;
     std::memset(&q, 0, sizeof q);
     q.budget = ctx->budget;
     q.abort = ctx->abort_requested.load() ? 1 : 0;
-    std::memcpy(s + fbytes + 2 * n * sizeof(long long), &q, sizeof q);
+    std::memcpy(s + fbytes + n * sizeof(long long), &q, sizeof q);
 
     const int prec = frames[0].precision_tag;
     bh_launch_params lp = ctx->launch[prec == BH_PRECISION_MIXED ? 1 : 0];
@@ -373,27 +371,25 @@ int plan_launch(bh_ctx* ctx, std::vector<FrameParams>& frames, bh_xyz* d_pixels,
     ShadeLaunch& sl = p.sl;
     std::memset(&sl, 0, sizeof sl);
     sl.frames = tl.frames;
-    sl.frame_pixel_end = static_cast<const long long*>(ctx->pix_end.p);
     sl.nframes = n;
-    sl.total_pixels = pix;
+    sl.blocks = shade_grid;
+    sl.pixel_lo = 0;
+    sl.pixel_hi = frame_px;
     sl.hits = tl.hits;
     sl.sky = sky_data(ctx);
     sl.pixels = d_pixels;
     sl.rays = d_rays;
-    sl.pixel_lum = static_cast<double*>(ctx->lum.p);
-    sl.ray_class = nullptr;
     sl.jet = tl.jet;
+    sl.stats = static_cast<FrameStats*>(ctx->fstats.p);
+    sl.flux = static_cast<double*>(ctx->partials.p);
+    sl.flux_per_frame = shade_grid;
 
     ReduceLaunch& rl = p.rl;
     std::memset(&rl, 0, sizeof rl);
-    rl.frames = tl.frames;
     rl.nframes = n;
-    rl.hits = tl.hits;
-    rl.pixel_lum = sl.pixel_lum;
-    rl.jet = tl.jet;
-    rl.partials = static_cast<FrameStats*>(ctx->partials.p);
-    rl.out = static_cast<FrameStats*>(ctx->fstats.p);
-    rl.blocks_per_frame = kReduceBlocks;
+    rl.flux_per_frame = shade_grid;
+    rl.flux = sl.flux;
+    rl.stats = sl.stats;
     return BH_OK;
 }
 
@@ -407,11 +403,10 @@ int record_launch(bh_ctx* ctx, const Plan& p, cudaStream_t stream, bool timed, b
     const size_t fbytes = static_cast<size_t>(p.nf) * sizeof(FrameParams);
     CK(cudaMemcpyAsync(ctx->frames.p, s, fbytes, cudaMemcpyHostToDevice, stream));
     CK(cudaMemcpyAsync(ctx->ray_end.p, s + fbytes, n * sizeof(long long), cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(ctx->pix_end.p, s + fbytes + n * sizeof(long long), n * sizeof(long long),
-                       cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(ctx->d_queue, s + fbytes + 2 * n * sizeof(long long), sizeof(QueueState),
+    CK(cudaMemcpyAsync(ctx->d_queue, s + fbytes + n * sizeof(long long), sizeof(QueueState),
                        cudaMemcpyHostToDevice, stream));
     if (!captured) CK(cudaEventRecord(ctx->stage_free, stream));
+    CK(cudaMemsetAsync(ctx->fstats.p, 0, n * sizeof(FrameStats), stream));
     if (timed) CK(cudaEventRecord(ctx->ev[0], stream));
     if (p.rays > 0) CK(launch_trace(p.tl, stream));
     if (timed) CK(cudaEventRecord(ctx->ev[1], stream));
@@ -474,6 +469,11 @@ int record_banded(bh_ctx* ctx, Plan& p, const bh_render_config* cfg, bh_xyz* out
     const long long px_band = static_cast<long long>(kBandRows) * W;
     int rc;
     if ((rc = ensure(ctx, ctx->band_done, static_cast<size_t>(nb) * sizeof(unsigned int))) != BH_OK) return rc;
+    // each band's shading blocks leave flux partials of their own
+    const int band_grid = shade_blocks(px_band, std::max(kShadeBlocks / nb, kShadeBlocksLeast));
+    if ((rc = ensure(ctx, ctx->partials, static_cast<size_t>(nb) * band_grid * sizeof(double))) != BH_OK) return rc;
+    p.rl.flux = static_cast<double*>(ctx->partials.p);
+    p.rl.flux_per_frame = nb * band_grid;
     unsigned int* done = static_cast<unsigned int*>(ctx->band_done.p);
     p.tl.band_done = done;
     p.tl.rays_per_band = px_band * S * S;
@@ -483,12 +483,11 @@ int record_banded(bh_ctx* ctx, Plan& p, const bh_render_config* cfg, bh_xyz* out
     const size_t fbytes = static_cast<size_t>(p.nf) * sizeof(FrameParams);
     CK(cudaMemcpyAsync(ctx->frames.p, st, fbytes, cudaMemcpyHostToDevice, stream));
     CK(cudaMemcpyAsync(ctx->ray_end.p, st + fbytes, sizeof(long long), cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(ctx->pix_end.p, st + fbytes + sizeof(long long), sizeof(long long), cudaMemcpyHostToDevice,
-                       stream));
-    CK(cudaMemcpyAsync(ctx->d_queue, st + fbytes + 2 * sizeof(long long), sizeof(QueueState), cudaMemcpyHostToDevice,
+    CK(cudaMemcpyAsync(ctx->d_queue, st + fbytes + sizeof(long long), sizeof(QueueState), cudaMemcpyHostToDevice,
                        stream));
     CK(cudaEventRecord(ctx->stage_free, stream));
     CK(cudaMemsetAsync(done, 0, static_cast<size_t>(nb) * sizeof(unsigned int), stream));
+    CK(cudaMemsetAsync(ctx->fstats.p, 0, sizeof(FrameStats), stream));
     CK(cudaEventRecord(ctx->ev[0], stream));
     // The band streams start once the counters are cleared.
     const int ns = std::min(nb, kBandStreams);
@@ -506,7 +505,9 @@ int record_banded(bh_ctx* ctx, Plan& p, const bh_render_config* cfg, bh_xyz* out
             return fail(ctx, BH_ERR_CUDA, "stream wait on a row band failed");
         ShadeLaunch sl = p.sl;
         sl.pixel_lo = lo;
-        sl.total_pixels = hi;
+        sl.pixel_hi = hi;
+        sl.blocks = band_grid;
+        sl.flux = static_cast<double*>(ctx->partials.p) + static_cast<size_t>(b) * band_grid;
         CK(launch_shade(sl, bs));
         CK(cudaMemcpyAsync(out_pixels + lo, static_cast<bh_xyz*>(ctx->pixels.p) + lo,
                            static_cast<size_t>(hi - lo) * sizeof(bh_xyz), cudaMemcpyDeviceToHost, bs));
@@ -668,8 +669,8 @@ void bh_gpu_destroy(bh_ctx* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    for (DevBuf* b : {&ctx->hits, &ctx->pixels, &ctx->rays, &ctx->lum, &ctx->frames, &ctx->ray_end, &ctx->deferred,
-                      &ctx->pix_end, &ctx->partials, &ctx->fstats, &ctx->jet, &ctx->adj_target, &ctx->adj_grad, &ctx->adj_Y,
+    for (DevBuf* b : {&ctx->hits, &ctx->pixels, &ctx->rays, &ctx->frames, &ctx->ray_end, &ctx->deferred,
+                      &ctx->partials, &ctx->fstats, &ctx->jet, &ctx->adj_target, &ctx->adj_grad, &ctx->adj_Y,
                       &ctx->adj_ckpt, &ctx->adj_counters, &ctx->adj_sums, &ctx->adj_xr, &ctx->adj_cand, &ctx->adj_edge,
                       &ctx->adj_high, &ctx->adj_rays, &ctx->eval_in, &ctx->eval_out, &ctx->disp_tmp, &ctx->disp_near,
                       &ctx->disp_far, &ctx->disp_k, &ctx->disp_state, &ctx->disp_rgb, &ctx->disp_frames, &ctx->sel_flag,

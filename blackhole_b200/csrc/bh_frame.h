@@ -53,6 +53,13 @@ struct FrameParams {
     long long n_rays;                // width * height * S^2
     long long pixel_begin;           // first pixel of this frame in the batch pixel buffer
 
+    // binary32 copies for the quick near-critical test of every ray
+    struct QuickCamera {
+        float tanf, inv_aspect, cr, sr, cp, sp, cy, sy;
+        float tet00, tet03, tet22, tet33, ml_tt, ml_tp, ml_thth, ml_pp;
+        float cs2, inv_sn2, a, a2, r_plus, cam_r, inv_s, inv_w, inv_h;
+    } quick;
+
     // ---- Novikov-Thorne disc (disc.h) -----------------------------------
     int32_t disc_enabled;
     int32_t disc_sigma;

@@ -70,32 +70,35 @@ int trace_blocks_per_sm(int precision, int block_size, int variant);
 // the plain, surface and jet kernels).
 int trace_registers(int precision, int variant);
 
+// Shades the frame-local pixels [pixel_lo, pixel_hi) (work order) of each
+// frame on `blocks` blocks, and adds those pixels' counts and maxima to the
+// frame's stats (zeroed before); each block's flux goes to a partial of its own
+// (flux_per_frame of them per frame, this launch's first one at `flux`).
 struct ShadeLaunch {
     const FrameParams* frames;
-    const long long* frame_pixel_end;   // cumulative pixel counts
     int nframes;
-    long long total_pixels;
+    int blocks;
+    long long pixel_lo, pixel_hi;
     const HitRecord* hits;
     SkyData sky;
-    bh_xyz* pixels;                  // device, total_pixels entries (frame-major, row-major)
+    bh_xyz* pixels;                  // device (frame-major, row-major)
     bh_ray_result* rays;             // optional device per-sample results (single frame)
-    double* pixel_lum;               // device, total_pixels luminance for the flux sum
-    unsigned char* ray_class;        // device, per-ray class after shading
     const double* jet;               // jet emission per ray (TraceLaunch::jet), or null
-    long long pixel_lo;              // shade global pixels [pixel_lo, total_pixels) only
+    FrameStats* stats;
+    double* flux;
+    int flux_per_frame;
 };
 
+// Blocks for `pixels` of one frame, `most` at most.
+int shade_blocks(long long pixels, int most);
 cudaError_t launch_shade(const ShadeLaunch& L, cudaStream_t stream);
 
+// Sums each frame's flux partials into its stats.
 struct ReduceLaunch {
-    const FrameParams* frames;
     int nframes;
-    const HitRecord* hits;
-    const double* pixel_lum;
-    const double* jet;               // jet emission per ray, or null
-    FrameStats* partials;            // nframes * blocks_per_frame
-    FrameStats* out;                 // nframes
-    int blocks_per_frame;
+    int flux_per_frame;
+    const double* flux;              // nframes * flux_per_frame
+    FrameStats* stats;
 };
 
 cudaError_t launch_reduce(const ReduceLaunch& L, cudaStream_t stream);

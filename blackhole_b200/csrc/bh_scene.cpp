@@ -457,6 +457,14 @@ int make_frame(const bh_render_config& c, FrameParams& F, std::string& err) {
     F.seed = c.seed;
     F.width = c.width;
     F.height = c.height;
+    {
+        FrameParams::QuickCamera& q = F.quick;
+        auto f = [](double v) { return static_cast<float>(v); };
+        q = {f(F.tanf), f(1.0 / F.aspect), f(F.cr), f(F.sr), f(F.cp), f(F.sp), f(F.cy), f(F.sy),
+             f(F.tet00), f(F.tet03), f(F.tet22), f(F.tet33), f(F.ml_tt), f(F.ml_tp), f(F.ml_thth), f(F.ml_pp),
+             f(F.cam_cs2), f(1.0 / F.cam_sn2), f(F.a), f(F.a2), f(F.r_plus), f(F.cam_r),
+             f(F.inv_S), f(1.0 / c.width), f(1.0 / c.height)};
+    }
     F.n_rays = static_cast<long long>(c.width) * c.height * S * S;
 
     // Novikov-Thorne disc (disc.h:73-82, W constants of disc.h:46-60).

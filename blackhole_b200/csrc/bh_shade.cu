@@ -3,12 +3,13 @@
 //   shade_kernel      per-pixel shading of the terminated rays (render.cpp:265-393,
 //                     disc.h:94-126, spectrum.cpp:123-134, scene.h:111-223) and the
 //                     sample average of render.cpp:456-462.
-//   reduce kernels    deterministic per-frame stats (render.cpp:481-494): fixed-shape
-//                     block reductions, then a fixed-order sum of the block partials.
+//                     It sums the per-frame stats (render.cpp:481-494) on the way.
+//   flux_kernel       a fixed-order sum of a frame's flux.
 //
 // Everything here is binary64: it runs once per ray, after the integration.
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstdint>
 
 #include "../../include/bh_gpu.h"
@@ -124,25 +125,38 @@ __device__ void sky_radiance(const SkyData& sky, const FrameParams& F, const dou
         if (span_p < 1) span_p = 1;
         const int sp = (span_p * 2 + 1 >= kLon) ? kLon / 2 : span_p;
         const int pbase = (int)((phi + kPi) / (2.0 * kPi) * kLon);
-        for (int a = -F.span_t; a <= F.span_t; ++a) {
-            const int ti = it + a;
-            if (ti < 0 || ti >= kLat) continue;
-            for (int b = -sp; b <= sp; ++b) {
-                int pi = pbase + b;
-                pi = ((pi % kLon) + kLon) % kLon;
-                const int bin = ti * kLon + pi;
-                const int k0 = __ldg(&sky.bin_start[bin]), k1 = __ldg(&sky.bin_start[bin + 1]);
-                for (int k = k0; k < k1; ++k) {
-                    const double4 s = sky.star_pos[k];
-                    const double dot = dclamp(d[0] * s.x + d[1] * s.y + d[2] * s.z, -1.0, 1.0);
-                    if (dot < F.cut_dot) continue;   // outside the cutoff, without the acos
-                    const double ang = (dot > 0.9999995) ? sqrt(dmaxr(0.0, 2.0 * (1.0 - dot))) : acos(dot);
-                    if (ang > cutoff) continue;
-                    const double w = norm * exp(-ang * ang * inv2s2) * s.w;
-                    const double4 c = sky.star_col[k];
-                    o[0] += w * c.x * c.z;
-                    o[1] += w;
-                    o[2] += w * c.y * c.z;
+        // The stars k0 <= k < k1, in catalogue order.
+        auto stars = [&](int k0, int k1) {
+            for (int k = k0; k < k1; ++k) {
+                const double4 s = sky.star_pos[k];
+                const double dot = dclamp(d[0] * s.x + d[1] * s.y + d[2] * s.z, -1.0, 1.0);
+                if (dot < F.cut_dot) continue;   // outside the cutoff, without the acos
+                const double ang = (dot > 0.9999995) ? sqrt(dmaxr(0.0, 2.0 * (1.0 - dot))) : acos(dot);
+                if (ang > cutoff) continue;
+                const double w = norm * exp(-ang * ang * inv2s2) * s.w;
+                const double4 c = sky.star_col[k];
+                o[0] += w * c.x * c.z;
+                o[1] += w;
+                o[2] += w * c.y * c.z;
+            }
+        };
+        const int lo = pbase - sp, hi = pbase + sp;
+        if (lo >= 0 && hi < kLon) {
+            // the window's bins of a row are neighbours, and so are their stars:
+            // one run per row
+            for (int a = -F.span_t; a <= F.span_t; ++a) {
+                const int ti = it + a;
+                if (ti < 0 || ti >= kLat) continue;
+                stars(__ldg(&sky.bin_start[ti * kLon + lo]), __ldg(&sky.bin_start[ti * kLon + hi + 1]));
+            }
+        } else {
+            for (int a = -F.span_t; a <= F.span_t; ++a) {
+                const int ti = it + a;
+                if (ti < 0 || ti >= kLat) continue;
+                for (int b = lo; b <= hi; ++b) {
+                    const int pi = ((b % kLon) + kLon) % kLon;
+                    const int bin = ti * kLon + pi;
+                    stars(__ldg(&sky.bin_start[bin]), __ldg(&sky.bin_start[bin + 1]));
                 }
             }
         }
@@ -284,184 +298,179 @@ __device__ void shade_one(const SkyData& sky, const FrameParams& F, const HitRec
     }
 }
 
-struct ShadeArgs {
-    const FrameParams* frames;
-    const long long* frame_pixel_end;
-    int nframes;
-    long long total_pixels;
-    const HitRecord* hits;
-    SkyData sky;
-    bh_xyz* pixels;
-    bh_ray_result* rays;
-    double* pixel_lum;
-    const double* jet;
-    long long pixel_lo;
-};
-
-__global__ void shade_kernel(ShadeArgs A) {
-    const long long gp = A.pixel_lo + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gp >= A.total_pixels) return;
-    const int f = find_frame(A.frame_pixel_end, A.nframes, gp);
-    const FrameParams& F = A.frames[f];
-    const long long p = gp - F.pixel_begin;        // frame-local pixel, band order
-    int px, py;
-    pixel_xy(F.width, F.height, p, &px, &py);
-    const int SS = F.S * F.S;
-    double acc[3] = {0.0, 0.0, 0.0};
-    for (int k = 0; k < SS; ++k) {
-        const long long rid = F.ray_begin + p * SS + k;
-        const HitRecord hr = A.hits[rid];
-        double c[3], g, dir[3];
-        shade_one(A.sky, F, hr, c, &g, dir);
-        // Whatever the ray ended on, the jet light it collected on the way is
-        // added in the jet's one colour (render.cpp:377-392).
-        const double jet = (F.jet_enabled && A.jet) ? A.jet[rid] : 0.0;
-        if (jet > 0.0) {
-            c[0] += F.jet_col[0] * jet;
-            c[1] += F.jet_col[1] * jet;
-            c[2] += F.jet_col[2] * jet;
-        }
-        acc[0] += c[0]; acc[1] += c[1]; acc[2] += c[2];
-        if (A.rays) {
-            bh_ray_result& o = A.rays[((long long)py * F.width + px) * SS + k];
-            o.what = hr.what;
-            o.steps = hr.steps;
-            #pragma unroll
-            for (int i = 0; i < 8; ++i) o.y[i] = hr.y[i];
-            o.g = g;
-            o.dir[0] = dir[0]; o.dir[1] = dir[1]; o.dir[2] = dir[2];
-            o.xyz.x = c[0]; o.xyz.y = c[1]; o.xyz.z = c[2];
-            o.attempts = hr.attempts;
-            o.reserved = 0;
-            o.max_norm = hr.max_norm;
-            o.max_q = hr.max_q;
-            o.jet = jet;
-        }
-    }
-    const double w = F.inv_SS;
-    bh_xyz& out = A.pixels[F.pixel_begin + (long long)py * F.width + px];
-    out.x = acc[0] * w;
-    out.y = acc[1] * w;
-    out.z = acc[2] * w;
-    A.pixel_lum[gp] = acc[1] * w;
-}
-
-// ---- deterministic stats reduction ------------------------------------------
-
-struct ReduceArgs {
-    const FrameParams* frames;
-    int nframes;
-    const HitRecord* hits;
-    const double* pixel_lum;
-    const double* jet;
-    FrameStats* partials;
-    FrameStats* out;
-    int bpf;
+// A thread's share of a frame's stats (render.cpp:481-494).
+struct StatsAcc {
+    unsigned long long steps = 0, attempts = 0;
+    unsigned rays = 0, cls[6] = {0, 0, 0, 0, 0, 0}, jet = 0;
+    double mn = 0.0, mq = 0.0, flux = 0.0;
 };
 
 __device__ __forceinline__ unsigned long long dbits(double x) { return (unsigned long long)__double_as_longlong(x); }
 
-constexpr int kRedThreads = 256;
+__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    return v;
+}
+__device__ __forceinline__ double warp_sum(double v) {
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    return v;
+}
+__device__ __forceinline__ unsigned long long warp_max(unsigned long long v) {
+    #pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        const unsigned long long u = __shfl_xor_sync(kFull, v, o);
+        if (u > v) v = u;
+    }
+    return v;
+}
 
-__global__ void __launch_bounds__(kRedThreads) reduce_partial_kernel(ReduceArgs A) {
-    const int f = blockIdx.y;
-    const FrameParams& F = A.frames[f];
-    __shared__ unsigned long long s_cnt[kRedThreads][10];
-    __shared__ double s_max[kRedThreads][2];
-    __shared__ double s_flux[kRedThreads];
-    unsigned long long c[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const double* jet = (F.jet_enabled && A.jet) ? A.jet + F.ray_begin : nullptr;
-    double mn = 0.0, mq = 0.0, flux = 0.0;
-    const long long stride = (long long)A.bpf * kRedThreads;
-    for (long long i = (long long)blockIdx.x * kRedThreads + threadIdx.x; i < F.n_rays; i += stride) {
-        const HitRecord& h = A.hits[F.ray_begin + i];
-        c[0] += 1;
-        c[1] += (unsigned long long)h.steps;
-        c[2] += (unsigned long long)h.attempts;
-        if (h.what >= 0 && h.what <= 5) c[3 + h.what] += 1;
-        mn = dmaxr(mn, h.max_norm);
-        mq = dmaxr(mq, h.max_q);
-        if (jet && jet[i] > 0.0) c[9] += 1;
-    }
-    const long long npx = (long long)F.width * F.height;
-    for (long long i = (long long)blockIdx.x * kRedThreads + threadIdx.x; i < npx; i += stride)
-        flux += A.pixel_lum[F.pixel_begin + i];
-    for (int k = 0; k < 10; ++k) s_cnt[threadIdx.x][k] = c[k];
-    s_max[threadIdx.x][0] = mn;
-    s_max[threadIdx.x][1] = mq;
-    s_flux[threadIdx.x] = flux;
+constexpr int kShadeThreads = 128;
+constexpr int kShadeWarps = kShadeThreads / 32;
+
+static_assert(offsetof(FrameStats, steps) == 8 && offsetof(FrameStats, attempts) == 16 &&
+                  offsetof(FrameStats, captured) == 24 && offsetof(FrameStats, disc_hits) == 32 &&
+                  offsetof(FrameStats, sun_hits) == 40 && offsetof(FrameStats, star_hits) == 48 &&
+                  offsetof(FrameStats, escaped) == 56 && offsetof(FrameStats, exhausted) == 64 &&
+                  offsetof(FrameStats, jet_rays) == 72 && BH_HIT_HORIZON == 0 && BH_HIT_DISC == 1 && BH_HIT_SUN == 2 &&
+                  BH_HIT_STAR == 3 && BH_HIT_SKY == 4 && BH_HIT_EXHAUSTED == 5,
+              "block_stats adds the counters in this order");
+
+// The block's sum of its threads' stats: counts and maxima, whose sums do not
+// depend on the order, are added to the frame's stats; the flux goes to the
+// block's partial.
+__device__ void block_stats(const StatsAcc& t, FrameStats* out, double* flux) {
+    __shared__ unsigned long long s_sum[10], s_max[2];
+    __shared__ double s_flux[kShadeWarps];
+    if (threadIdx.x < 10) s_sum[threadIdx.x] = 0ull;
+    if (threadIdx.x < 2) s_max[threadIdx.x] = 0ull;
     __syncthreads();
-    for (int off = kRedThreads / 2; off > 0; off >>= 1) {
-        if (threadIdx.x < off) {
-            for (int k = 0; k < 10; ++k) s_cnt[threadIdx.x][k] += s_cnt[threadIdx.x + off][k];
-            s_max[threadIdx.x][0] = dmaxr(s_max[threadIdx.x][0], s_max[threadIdx.x + off][0]);
-            s_max[threadIdx.x][1] = dmaxr(s_max[threadIdx.x][1], s_max[threadIdx.x + off][1]);
-            s_flux[threadIdx.x] += s_flux[threadIdx.x + off];
-        }
-        __syncthreads();
+    unsigned long long v[10] = {__reduce_add_sync(kFull, t.rays), warp_sum(t.steps), warp_sum(t.attempts)};
+    #pragma unroll
+    for (int q = 0; q < 6; ++q) v[3 + q] = __reduce_add_sync(kFull, t.cls[q]);
+    v[9] = __reduce_add_sync(kFull, t.jet);
+    // non-negative doubles order like their bits
+    const unsigned long long mn = warp_max(dbits(t.mn)), mq = warp_max(dbits(t.mq));
+    const double f = warp_sum(t.flux);
+    if ((threadIdx.x & 31) == 0) {
+        s_flux[threadIdx.x >> 5] = f;
+        #pragma unroll
+        for (int q = 0; q < 10; ++q)
+            if (v[q]) atomicAdd(&s_sum[q], v[q]);
+        atomicMax(&s_max[0], mn);
+        atomicMax(&s_max[1], mq);
     }
-    if (threadIdx.x == 0) {
-        FrameStats& o = A.partials[(long long)f * A.bpf + blockIdx.x];
-        o.rays = s_cnt[0][0];
-        o.steps = s_cnt[0][1];
-        o.attempts = s_cnt[0][2];
-        o.captured = s_cnt[0][3 + BH_HIT_HORIZON];
-        o.disc_hits = s_cnt[0][3 + BH_HIT_DISC];
-        o.sun_hits = s_cnt[0][3 + BH_HIT_SUN];
-        o.star_hits = s_cnt[0][3 + BH_HIT_STAR];
-        o.escaped = s_cnt[0][3 + BH_HIT_SKY];
-        o.exhausted = s_cnt[0][3 + BH_HIT_EXHAUSTED];
-        o.jet_rays = s_cnt[0][9];
-        o.max_norm_bits = dbits(s_max[0][0]);
-        o.max_q_bits = dbits(s_max[0][1]);
-        o.total_flux = s_flux[0];
+    __syncthreads();
+    if (threadIdx.x < 10) {
+        // rays, steps, attempts, the six classes in BH_HIT_* order, jet rays:
+        // the order of FrameStats' counters
+        if (s_sum[threadIdx.x]) atomicAdd(&out->rays + threadIdx.x, s_sum[threadIdx.x]);
+    } else if (threadIdx.x == 32) {
+        atomicMax(&out->max_norm_bits, s_max[0]);
+    } else if (threadIdx.x == 64) {
+        atomicMax(&out->max_q_bits, s_max[1]);
+    } else if (threadIdx.x == 96) {
+        double s = s_flux[0];
+        for (int i = 1; i < kShadeWarps; ++i) s += s_flux[i];
+        *flux = s;
     }
 }
 
-// One block per frame: thread t sums the partials t, t + kRedThreads, ... in
-// that order, then a fixed tree combines the threads: the same bits on every
-// run.
-__global__ void __launch_bounds__(kRedThreads) reduce_final_kernel(ReduceArgs A) {
-    const int f = blockIdx.x;
-    __shared__ unsigned long long s_cnt[kRedThreads][10];
-    __shared__ double s_max[kRedThreads][2];
-    __shared__ double s_flux[kRedThreads];
-    unsigned long long c[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    double mn = 0.0, mq = 0.0, flux = 0.0;
-    for (int b = threadIdx.x; b < A.bpf; b += kRedThreads) {
-        const FrameStats& p = A.partials[(long long)f * A.bpf + b];
-        c[0] += p.rays; c[1] += p.steps; c[2] += p.attempts;
-        c[3] += p.captured; c[4] += p.disc_hits; c[5] += p.sun_hits;
-        c[6] += p.star_hits; c[7] += p.escaped; c[8] += p.exhausted; c[9] += p.jet_rays;
-        mn = dmaxr(mn, __longlong_as_double((long long)p.max_norm_bits));
-        mq = dmaxr(mq, __longlong_as_double((long long)p.max_q_bits));
-        flux += p.total_flux;
-    }
-    for (int k = 0; k < 10; ++k) s_cnt[threadIdx.x][k] = c[k];
-    s_max[threadIdx.x][0] = mn;
-    s_max[threadIdx.x][1] = mq;
-    s_flux[threadIdx.x] = flux;
-    __syncthreads();
-    for (int off = kRedThreads / 2; off > 0; off >>= 1) {
-        if (threadIdx.x < off) {
-            for (int k = 0; k < 10; ++k) s_cnt[threadIdx.x][k] += s_cnt[threadIdx.x + off][k];
-            s_max[threadIdx.x][0] = dmaxr(s_max[threadIdx.x][0], s_max[threadIdx.x + off][0]);
-            s_max[threadIdx.x][1] = dmaxr(s_max[threadIdx.x][1], s_max[threadIdx.x + off][1]);
-            s_flux[threadIdx.x] += s_flux[threadIdx.x + off];
+struct ShadeArgs {
+    const FrameParams* frames;
+    long long pixel_lo, pixel_hi;
+    const HitRecord* hits;
+    SkyData sky;
+    bh_xyz* pixels;
+    bh_ray_result* rays;
+    const double* jet;
+    FrameStats* stats;
+    double* flux;
+    int flux_per_frame;
+};
+
+// The frame's pixels (grid.y: frames) shaded, 128 at a time per block, and
+// its stats summed on the way: the hit records (96 bytes a ray) are read once.
+// With the stats in a pass of their own over the records a 1024^2 mixed frame
+// took 162 us for both, now 128, a 2048^2 one 445 and 290.  What is left is the
+// shading's binary64 chains (20 warps per SM; 16 and 24 the same within 5%).
+__global__ void __launch_bounds__(kShadeThreads, 5) shade_kernel(ShadeArgs A) {
+    const FrameParams& F = A.frames[blockIdx.y];
+    const long long npx = (long long)F.width * F.height;
+    const long long hi = (A.pixel_hi < npx) ? A.pixel_hi : npx;
+    const int SS = F.S * F.S;
+    StatsAcc st;
+    for (long long p = A.pixel_lo + (long long)blockIdx.x * kShadeThreads + threadIdx.x; p < hi;
+         p += (long long)gridDim.x * kShadeThreads) {      // frame-local pixel, band order
+        int px, py;
+        pixel_xy(F.width, F.height, p, &px, &py);
+        double acc[3] = {0.0, 0.0, 0.0};
+        for (int k = 0; k < SS; ++k) {
+            const long long rid = F.ray_begin + p * SS + k;
+            const HitRecord hr = A.hits[rid];
+            double c[3], g, dir[3];
+            shade_one(A.sky, F, hr, c, &g, dir);
+            // Whatever the ray ended on, the jet light it collected on the way is
+            // added in the jet's one colour (render.cpp:377-392).
+            const double jet = (F.jet_enabled && A.jet) ? A.jet[rid] : 0.0;
+            if (jet > 0.0) {
+                c[0] += F.jet_col[0] * jet;
+                c[1] += F.jet_col[1] * jet;
+                c[2] += F.jet_col[2] * jet;
+                st.jet += 1;
+            }
+            acc[0] += c[0]; acc[1] += c[1]; acc[2] += c[2];
+            st.rays += 1;
+            st.steps += (unsigned long long)hr.steps;
+            st.attempts += (unsigned long long)hr.attempts;
+            #pragma unroll
+            for (int q = 0; q < 6; ++q) st.cls[q] += (hr.what == q) ? 1u : 0u;
+            st.mn = dmaxr(st.mn, hr.max_norm);
+            st.mq = dmaxr(st.mq, hr.max_q);
+            if (A.rays) {
+                bh_ray_result& o = A.rays[((long long)py * F.width + px) * SS + k];
+                o.what = hr.what;
+                o.steps = hr.steps;
+                #pragma unroll
+                for (int i = 0; i < 8; ++i) o.y[i] = hr.y[i];
+                o.g = g;
+                o.dir[0] = dir[0]; o.dir[1] = dir[1]; o.dir[2] = dir[2];
+                o.xyz.x = c[0]; o.xyz.y = c[1]; o.xyz.z = c[2];
+                o.attempts = hr.attempts;
+                o.reserved = 0;
+                o.max_norm = hr.max_norm;
+                o.max_q = hr.max_q;
+                o.jet = jet;
+            }
         }
-        __syncthreads();
+        const double w = F.inv_SS;
+        bh_xyz& out = A.pixels[F.pixel_begin + (long long)py * F.width + px];
+        out.x = acc[0] * w;
+        out.y = acc[1] * w;
+        out.z = acc[2] * w;
+        st.flux += acc[1] * w;
     }
-    if (threadIdx.x == 0) {
-        FrameStats t = {};
-        t.rays = s_cnt[0][0]; t.steps = s_cnt[0][1]; t.attempts = s_cnt[0][2];
-        t.captured = s_cnt[0][3]; t.disc_hits = s_cnt[0][4]; t.sun_hits = s_cnt[0][5];
-        t.star_hits = s_cnt[0][6]; t.escaped = s_cnt[0][7]; t.exhausted = s_cnt[0][8];
-        t.jet_rays = s_cnt[0][9];
-        t.max_norm_bits = dbits(s_max[0][0]);
-        t.max_q_bits = dbits(s_max[0][1]);
-        t.total_flux = s_flux[0];
-        A.out[f] = t;
-    }
+    block_stats(st, &A.stats[blockIdx.y], &A.flux[(long long)blockIdx.y * A.flux_per_frame + blockIdx.x]);
+}
+
+constexpr int kRedThreads = 256;
+
+// The flux of a frame, one block each: thread t sums the partials t,
+// t + kRedThreads, ... in that order, then a fixed tree combines the threads:
+// the same bits on every run.
+__global__ void __launch_bounds__(kRedThreads) flux_kernel(const double* __restrict__ partials, int count,
+                                                           FrameStats* __restrict__ out) {
+    __shared__ double s_flux[kRedThreads / 32];
+    const double* mine = partials + (long long)blockIdx.x * count;
+    double f = 0.0;
+    for (int b = threadIdx.x; b < count; b += kRedThreads) f += mine[b];
+    f = warp_sum(f);
+    if ((threadIdx.x & 31) == 0) s_flux[threadIdx.x >> 5] = f;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int i = 1; i < kRedThreads / 32; ++i) f += s_flux[i];
+    out[blockIdx.x].total_flux = f;
 }
 
 
@@ -485,41 +494,31 @@ cudaError_t launch_eval_shade(int what, const FrameParams* d_frame, const double
     return cudaGetLastError();
 }
 
+int shade_blocks(long long pixels, int most) {
+    const long long want = (pixels + kShadeThreads - 1) / kShadeThreads;
+    return (int)(want < 1 ? 1 : (want < most ? want : most));
+}
+
 cudaError_t launch_shade(const ShadeLaunch& L, cudaStream_t stream) {
-    if (L.total_pixels <= 0) return cudaSuccess;
+    if (L.pixel_hi <= L.pixel_lo || L.nframes <= 0) return cudaSuccess;
     ShadeArgs A;
     A.frames = L.frames;
-    A.frame_pixel_end = L.frame_pixel_end;
-    A.nframes = L.nframes;
-    A.total_pixels = L.total_pixels;
+    A.pixel_lo = L.pixel_lo;
+    A.pixel_hi = L.pixel_hi;
     A.hits = L.hits;
     A.sky = L.sky;
     A.pixels = L.pixels;
     A.rays = L.rays;
-    A.pixel_lum = L.pixel_lum;
     A.jet = L.jet;
-    A.pixel_lo = L.pixel_lo;
-    const int bs = 128;
-    const long long grid = (L.total_pixels - L.pixel_lo + bs - 1) / bs;
-    if (grid <= 0) return cudaSuccess;
-    shade_kernel<<<(unsigned)grid, bs, 0, stream>>>(A);
+    A.stats = L.stats;
+    A.flux = L.flux;
+    A.flux_per_frame = L.flux_per_frame;
+    shade_kernel<<<dim3((unsigned)L.blocks, (unsigned)L.nframes), kShadeThreads, 0, stream>>>(A);
     return cudaGetLastError();
 }
 
 cudaError_t launch_reduce(const ReduceLaunch& L, cudaStream_t stream) {
-    ReduceArgs A;
-    A.frames = L.frames;
-    A.nframes = L.nframes;
-    A.hits = L.hits;
-    A.pixel_lum = L.pixel_lum;
-    A.jet = L.jet;
-    A.partials = L.partials;
-    A.out = L.out;
-    A.bpf = L.blocks_per_frame;
-    reduce_partial_kernel<<<dim3(L.blocks_per_frame, L.nframes), kRedThreads, 0, stream>>>(A);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    reduce_final_kernel<<<L.nframes, kRedThreads, 0, stream>>>(A);
+    flux_kernel<<<L.nframes, kRedThreads, 0, stream>>>(L.flux, L.flux_per_frame, L.stats);
     return cudaGetLastError();
 }
 
