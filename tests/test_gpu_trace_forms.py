@@ -117,3 +117,32 @@ def test_launch_shape_does_not_change_binary64_frames(width, height, jet):
         assert np.array_equal(auto[k], tight[k]), k
     # the jet's sum is rounded by each kernel as it was compiled
     assert np.allclose(auto["jet"], tight["jet"], rtol=1e-11, atol=1e-14 * max(1e-300, tight["jet"].max()))
+
+
+@pytest.mark.parametrize("centre,radius,fov", [
+    ((0.0, 22.0, 0.0), 4.0, 1.2),          # beside the hole
+    ((45.0, 5.0, 8.0), 0.3, 0.6),          # a small one close to the camera, between two steps
+    ((-400.0, 60.0, 30.0), 40.0, 0.9),     # far behind, where the steps are long
+    ((60.0, 0.0, 10.0), 12.0, 0.6),        # the camera just outside it
+])
+@pytest.mark.parametrize("precision", [abi.PRECISION_FP64, abi.PRECISION_MIXED])
+def test_no_step_misses_the_sun(renderer, orc, centre, radius, fov, precision):
+    """The binary32 test of a step against the Sun leaves out only steps that
+    the oracle does not probe either: the same rays end on it (the suite's two
+    flips allowed), at the same place."""
+    from blackhole_b200.config import SunBody
+
+    cfg = RenderConfig(
+        M_kg=4.3e6 * M_SUN, spin=0.6, cam=Camera(r=60.0, theta=math.radians(80.0), phi=0.0, fov=fov, yaw=0.15),
+        width=41, height=31, sqrt_spp=1, disc_r_out=20.0, sun_enabled=True, sun=SunBody(centre=centre, radius=radius),
+        rtol=1e-9, atol=1e-11, r_escape=600.0, star_count=0, quiet=True,
+    )
+    chk, _ = orc.trace_rays(cfg)
+    cfg.precision = precision
+    got = renderer.trace_rays(cfg)
+    sun = chk["what"] == abi.HIT_SUN
+    assert sun.sum() > 5
+    assert ((got["what"] == abi.HIT_SUN) != sun).sum() <= 2
+    both = sun & (got["what"] == abi.HIT_SUN)
+    tol = 1e-6 if precision == abi.PRECISION_FP64 else 1e-3
+    assert np.quantile(np.abs(got["y"][both, 1] / chk["y"][both, 1] - 1.0), 0.95) <= tol
