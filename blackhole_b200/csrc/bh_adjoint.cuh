@@ -500,6 +500,11 @@ __host__ __device__ __forceinline__ double crossing_target(double th0, double th
     return 0.5 * kPi + m * kPi;
 }
 
+// What the render records of a ray's accepted step (kTrajWords doubles): r, th,
+// p_r, p_th at its start, its size, and sin and cos of the angle.  Word w of
+// step j of ray i lies at traj[(j kTrajWords + w) n_rays + i], so that the lanes
+// of a warp write and read side by side.
+
 // Carries the adjoint yb of the state after one accepted step (from ys with
 // step h; sn0, cs0: sin and cos of its angle) back to the state before it,
 // accumulating the E, L_z and spin adjoints.  The six stages are computed again and their vector-Jacobian
@@ -1158,6 +1163,48 @@ __host__ __device__ inline void integ_start(const FrameParams& F, const double y
     s.steps = 0;
 }
 
+// The luminance of a ray that ended in `what` (disc: at radius r_hit; sky: in
+// state y = (t, r, th, phi, p_r, p_th)) and, times the loss weight w, its
+// derivatives: where the reverse pass starts.
+struct Seed {
+    double Y, d_edd;
+    double yb[6];        // with respect to the state at the end of the last step (sky)
+    double rstar_b;      // with respect to the hit radius (disc)
+    double Eb, Lzb, ab;
+    __host__ __device__ bool any() const {
+        return rstar_b != 0.0 || Eb != 0.0 || Lzb != 0.0 || ab != 0.0 || yb[1] != 0.0 || yb[2] != 0.0 ||
+               yb[3] != 0.0 || yb[4] != 0.0 || yb[5] != 0.0;
+    }
+};
+__host__ __device__ BHA_NOINLINE void seed_ray(const FrameParams& F, const AdjointFrame& X, const SkyData& sky,
+                                               int what, double r_hit, const double y[6], double E, double Lz,
+                                               double w, Seed& o) {
+    o = Seed{};
+    if (what == BH_HIT_DISC) {
+        const D5 Y = disc_luminance(F, X, sky.table, r_hit, E, Lz);
+        o.Y = Y.v;
+        o.rstar_b = w * Y.d[kS5R];
+        o.Eb = w * Y.d[kS5E];
+        o.Lzb = w * Y.d[kS5L];
+        o.ab = w * Y.d[kS5A];
+        o.d_edd = w * Y.d[kS5M];
+    } else if (what == BH_HIT_SKY) {
+        D8 v[3];
+        if (escape_direction(y, E, Lz, F.a, v)) {
+            const double d[3] = {v[0].v, v[1].v, v[2].v};
+            double gY[3];
+            o.Y = sky_luminance(sky, F, d, gY);
+            double gs[8];
+            for (int k = 0; k < 8; ++k)
+                gs[k] = w * (gY[0] * v[0].d[k] + gY[1] * v[1].d[k] + gY[2] * v[2].d[k]);
+            for (int k = 0; k < 5; ++k) o.yb[k + 1] = gs[k];
+            o.Eb = gs[5];
+            o.Lzb = gs[6];
+            o.ab = gs[7];
+        }
+    }
+}
+
 // The forward pass, the seed and the reverse pass of one ray.  `ck` holds
 // `slots` states of kCkWords doubles.  With w == 0 (or forward_only) only the
 // luminance is computed.  xr (may be null) receives the ray's first two
@@ -1182,39 +1229,18 @@ __host__ __device__ inline void adjoint_ray(const FrameParams& F, const AdjointF
     out->steps = s.steps;
     out->interval = cp.interval;
 
-    // ---- seed --------------------------------------------------------------------
-    double yb[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    double Eb = 0.0, Lzb = 0.0, ab = 0.0, rstar_b = 0.0;
-    if (what == BH_HIT_DISC) {
-        const D5 Y = disc_luminance(F, X, sky.table, r_hit, E, Lz);
-        out->Y = Y.v;
-        rstar_b = w * Y.d[kS5R];
-        Eb = w * Y.d[kS5E];
-        Lzb = w * Y.d[kS5L];
-        ab = w * Y.d[kS5A];
-        out->grad[2] = w * Y.d[kS5M];
-    } else if (what == BH_HIT_SKY) {
-        D8 v[3];
-        if (escape_direction(s.y, E, Lz, F.a, v)) {
-            const double d[3] = {v[0].v, v[1].v, v[2].v};
-            double gY[3];
-            out->Y = sky_luminance(sky, F, d, gY);
-            double gs[8];
-            for (int k = 0; k < 8; ++k)
-                gs[k] = w * (gY[0] * v[0].d[k] + gY[1] * v[1].d[k] + gY[2] * v[2].d[k]);
-            yb[1] = gs[0]; yb[2] = gs[1]; yb[3] = gs[2]; yb[4] = gs[3]; yb[5] = gs[4];
-            Eb = gs[5];
-            Lzb = gs[6];
-            ab = gs[7];
-        }
-    }
+    Seed sd;
+    seed_ray(F, X, sky, what, r_hit, s.y, E, Lz, w, sd);
+    out->Y = sd.Y;
+    out->grad[2] = sd.d_edd;
+    double Eb = sd.Eb, Lzb = sd.Lzb, ab = sd.ab;
+    double* const yb = sd.yb;
+    const double rstar_b = sd.rstar_b;
     if (forward_only || w == 0.0 || (what != BH_HIT_DISC && what != BH_HIT_SKY)) return;
-    if (rstar_b == 0.0 && Eb == 0.0 && Lzb == 0.0 && ab == 0.0 && yb[1] == 0.0 && yb[2] == 0.0 &&
-        yb[3] == 0.0 && yb[4] == 0.0 && yb[5] == 0.0)
-        return;
+    if (!sd.any()) return;
 
     // ---- reverse and the initial photon ------------------------------------------------
-    out->replay = reverse_sweep(F, c, cp, s.steps, s.h_acc, what == BH_HIT_DISC ? rstar_b : 0.0, yb, &Eb, &Lzb, &ab);
+    out->replay = reverse_sweep(F, c, cp, s.steps, s.h_acc, rstar_b, yb, &Eb, &Lzb, &ab);
     for (int q = 0; q < 2; ++q) {
         double gq = Eb * dE[q] + Lzb * dLz[q];
         for (int i = 0; i < 6; ++i) gq += yb[i] * dy0[q][i];
@@ -1301,65 +1327,33 @@ __host__ __device__ inline double line_in_cell(double gx, double gy, double cx, 
 // Edges of the disc an equatorial crossing can be near.
 enum { kEdgeOuter = 1, kEdgeInner = 2 };
 
-// The edge term of equatorial crossing number `crossing` (1 or 2) of sample k
-// of pixel (px, py), for the disc edges in `edges` (kEdgeOuter: r_out;
-// kEdgeInner: r_in, the ISCO) and pixel weight w = dLoss/d(pixel).  With
-// phi = r_out - r_c (outer) or r_c - r_in (inner), positive on the disc side,
-//   d(pixel)/dq = (Y_disc - Y_beyond) (d phi/d q) L / |grad r_c|.
-// out[0..2] receive the contributions to dLoss/d(r_out), d(spin),
-// d(inclination); *cells the number of edges that cross the sample's cell.
-// diag (may be null) receives r_c, |grad r_c| (per pixel), d r_c/d(spin,
-// inclination), d r_c/d(su, sv), and per edge (outer, inner) L and
-// Y_disc - Y_beyond.  Returns the accepted steps integrated (forward,
-// continuation and replay).
-__host__ __device__ BHA_NOINLINE long long edge_sample(const FrameParams& F, const AdjointFrame& X, const SkyData& sky,
-                                                 int px, int py, int k, int crossing, int edges, double w,
-                                                 double* ck, int slots, int stride, double out[3], int* cells,
-                                                 double* diag = nullptr) {
-    out[0] = out[1] = out[2] = 0.0;
-    *cells = 0;
+// The luminance of a ray that ended in `what` (as seed_ray).
+__host__ __device__ BHA_NOINLINE double luminance(const FrameParams& F, const AdjointFrame& X, const SkyData& sky,
+                                                  int what, double r_hit, const double y[6], double E, double Lz) {
+    if (what == BH_HIT_DISC) return disc_luminance(F, X, sky.table, r_hit, E, Lz).v;
+    double d[3], gY[3];
+    if (what == BH_HIT_SKY && escape_direction_value(y, E, Lz, F.a, d)) return sky_luminance(sky, F, d, gY);
+    return 0.0;
+}
+
+// The luminance jumps across the edges in `edges`: the disc's side is its
+// luminance at r_out along this ray; the Novikov-Thorne flux vanishes at r_in.
+__host__ __device__ BHA_NOINLINE void edge_jumps(const FrameParams& F, const AdjointFrame& X, const SkyData& sky,
+                                                 int edges, double Y_beyond, double E, double Lz, double dY[2]) {
+    dY[0] = (edges & kEdgeOuter) ? disc_luminance(F, X, sky.table, F.r_out, E, Lz).v - Y_beyond : 0.0;
+    dY[1] = (edges & kEdgeInner) ? -Y_beyond : 0.0;
+}
+
+// The edge terms of a sample's crossing at radius rc with jumps dY, from
+// d r_c / d(initial state, E, L_z, spin) = (yb, Eb, Lzb, ab); see edge_sample.
+__host__ __device__ BHA_NOINLINE void edge_finish(const FrameParams& F, const AdjointFrame& X, int px, int py, int k,
+                                                  int edges, double w, double rc, const double dY[2],
+                                                  const double yb[6], double Eb, double Lzb, double ab,
+                                                  double out[3], int* cells, double* diag) {
     double su, sv, xp, yp;
     sample_position_at(F, px, py, k, &su, &sv, &xp, &yp);
     double y0[6], E, Lz, dy0[2][6], dE[2], dLz[2];
     ray_start_at(F, X, su, sv, y0, &E, &Lz, dy0, dE, dLz);
-    const RayC c = ray_consts(F, E, Lz);
-    Integ s;
-    integ_start(F, y0, s);
-    Checkpoints cp{ck, slots, X.checkpoint_interval, 0, stride};
-    cp.push(s);
-    double rc = 0.0;
-    if (forward_run(F, c, s, &cp, nullptr, crossing, &rc) != -1) return s.steps;
-    const int step = s.steps;
-    const double h_step = s.h_acc;
-
-    // What the ray meets when this crossing misses the disc: its
-    // continuation traced on from there.
-    Integ t = s;
-    double r_hit = 0.0;
-    const int what = forward_run(F, c, t, nullptr, nullptr, 0, &r_hit, true);
-    long long work = t.steps;
-    double Y_beyond = 0.0;
-    if (what == BH_HIT_DISC) {
-        Y_beyond = disc_luminance(F, X, sky.table, r_hit, E, Lz).v;
-    } else if (what == BH_HIT_SKY) {
-        D8 v[3];
-        if (escape_direction(t.y, E, Lz, F.a, v)) {
-            const double d[3] = {v[0].v, v[1].v, v[2].v};
-            double gY[3];
-            Y_beyond = sky_luminance(sky, F, d, gY);
-        }
-    }
-    // the disc's side of each edge: its luminance at r_out along this ray; the
-    // Novikov-Thorne flux vanishes at r_in
-    const double dY[2] = {(edges & kEdgeOuter) ? disc_luminance(F, X, sky.table, F.r_out, E, Lz).v - Y_beyond : 0.0,
-                          (edges & kEdgeInner) ? -Y_beyond : 0.0};
-    if (dY[0] == 0.0 && dY[1] == 0.0 && !diag) return work;
-
-    // d r_c / d(initial state, E, L_z, spin) by a reverse sweep seeded with r_c
-    double yb[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    double Eb = 0.0, Lzb = 0.0, ab = 0.0;
-    work += reverse_sweep(F, c, cp, step, h_step, 1.0, yb, &Eb, &Lzb, &ab);
-
     double dpr[2], dpth[2], dEp[2], dLzp[2];
     ray_start_pixel_tangents(F, su, sv, dpr, dpth, dEp, dLzp);
     double drc[2];
@@ -1407,6 +1401,56 @@ __host__ __device__ BHA_NOINLINE long long edge_sample(const FrameParams& F, con
         diag[8] = L[1];
         diag[9] = dY[1];
     }
+}
+
+// The edge term of equatorial crossing number `crossing` (1 or 2) of sample k
+// of pixel (px, py), for the disc edges in `edges` (kEdgeOuter: r_out;
+// kEdgeInner: r_in, the ISCO) and pixel weight w = dLoss/d(pixel).  With
+// phi = r_out - r_c (outer) or r_c - r_in (inner), positive on the disc side,
+//   d(pixel)/dq = (Y_disc - Y_beyond) (d phi/d q) L / |grad r_c|.
+// out[0..2] receive the contributions to dLoss/d(r_out), d(spin),
+// d(inclination); *cells the number of edges that cross the sample's cell.
+// diag (may be null) receives r_c, |grad r_c| (per pixel), d r_c/d(spin,
+// inclination), d r_c/d(su, sv), and per edge (outer, inner) L and
+// Y_disc - Y_beyond.  Returns the accepted steps integrated (forward,
+// continuation and replay).
+__host__ __device__ BHA_NOINLINE long long edge_sample(const FrameParams& F, const AdjointFrame& X, const SkyData& sky,
+                                                 int px, int py, int k, int crossing, int edges, double w,
+                                                 double* ck, int slots, int stride, double out[3], int* cells,
+                                                 double* diag = nullptr) {
+    out[0] = out[1] = out[2] = 0.0;
+    *cells = 0;
+    double su, sv, xp, yp;
+    sample_position_at(F, px, py, k, &su, &sv, &xp, &yp);
+    double y0[6], E, Lz, dy0[2][6], dE[2], dLz[2];
+    ray_start_at(F, X, su, sv, y0, &E, &Lz, dy0, dE, dLz);
+    const RayC c = ray_consts(F, E, Lz);
+    Integ s;
+    integ_start(F, y0, s);
+    Checkpoints cp{ck, slots, X.checkpoint_interval, 0, stride};
+    cp.push(s);
+    double rc = 0.0;
+    if (forward_run(F, c, s, &cp, nullptr, crossing, &rc) != -1) return s.steps;
+    const int step = s.steps;
+    const double h_step = s.h_acc;
+
+    // What the ray meets when this crossing misses the disc: its
+    // continuation traced on from there.
+    Integ t = s;
+    double r_hit = 0.0;
+    const int what = forward_run(F, c, t, nullptr, nullptr, 0, &r_hit, true);
+    long long work = t.steps;
+    const double Y_beyond = luminance(F, X, sky, what, r_hit, t.y, E, Lz);
+    double dY[2];
+    edge_jumps(F, X, sky, edges, Y_beyond, E, Lz, dY);
+    if (dY[0] == 0.0 && dY[1] == 0.0 && !diag) return work;
+
+    // d r_c / d(initial state, E, L_z, spin) by a reverse sweep seeded with r_c
+    double yb[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    double Eb = 0.0, Lzb = 0.0, ab = 0.0;
+    work += reverse_sweep(F, c, cp, step, h_step, 1.0, yb, &Eb, &Lzb, &ab);
+
+    edge_finish(F, X, px, py, k, edges, w, rc, dY, yb, Eb, Lzb, ab, out, cells, diag);
     return work;
 }
 

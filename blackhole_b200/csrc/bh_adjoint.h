@@ -53,7 +53,14 @@ struct AdjointLaunch {
     double* ray_Y;                   // luminance per ray in the same order, or nullptr
     double* ckpt;                    // grid * block * checkpoint_slots * kAdjSlotWords doubles
     const HitRecord* hits;           // the render's hit records, work order (device)
-    int* rays;                       // the rays that have a gradient (work order ids; n_rays entries)
+    // The rays that have a gradient (work order ids; n_rays entries): those whose
+    // steps the render recorded from the front, the others from the back.
+    int* rays;
+    const double* traj;              // the recorded steps (TraceLaunch::traj), or null
+    int traj_cap;
+    const int* abort;                // nonzero: the render was stopped and its records are not complete
+    const int* xing_step;            // TraceLaunch::xing_step, disc_end
+    const double* disc_end;
     // The edge pass: per crossing slot (2 per ray, slot = 2 * ray + crossing,
     // rays in work order) the radius of the ray's first two equatorial
     // crossings as the render found them (0: none; zeroed before the
@@ -66,7 +73,9 @@ struct AdjointLaunch {
     // crossing (an image of order three or higher), in ray_grad order
     unsigned char* high_order;
     // next job, accepted, replayed, disc rays, sky rays, max interval, edge
-    // candidates, edge-pass steps, edge cells, high-order rays, rays with a gradient
+    // candidates, edge-pass steps, edge cells, high-order rays, rays with a gradient and recorded steps, other rays with a
+    // gradient, next recorded ray and recorded steps, other rays with a
+    // gradient, next job of the recorded rays
     unsigned long long* counters;
     // loss; the four per-ray gradient sums (spin and inclination over the
     // rays of image order one and two); the three edge sums; the spin and
@@ -74,9 +83,12 @@ struct AdjointLaunch {
     double* sums;
     long long n_rays;
     int grid, block;
+    int grid_reverse;                // blocks of the kernel over the recorded rays
+    cudaStream_t side_stream;        // the edge terms and the rays without records run here, beside it
+    cudaEvent_t fork_event, join_event;
 };
 
-constexpr int kAdjCounters = 11;
+constexpr int kAdjCounters = 13;
 constexpr int kAdjSlotWords = 11;         // doubles per stored state
 constexpr int kAdjSums = 10;
 
@@ -88,6 +100,7 @@ cudaError_t launch_adjoint(const AdjointLaunch& L, cudaStream_t stream);
 // Threads per block of the adjoint kernel, and its resident blocks per SM at
 // `block_size` threads.
 int adjoint_block_size();
+int reverse_blocks_per_sm();
 int adjoint_blocks_per_sm(int block_size);
 
 }  // namespace bhg

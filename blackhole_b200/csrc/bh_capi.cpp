@@ -81,6 +81,7 @@ struct bh_ctx {
     // Adjoint: target image, per-ray gradients and luminances, checkpoint
     // slots, counters, sums and the edge pass's buffers.
     DevBuf adj_target, adj_grad, adj_Y, adj_ckpt, adj_counters, adj_sums, adj_xr, adj_cand, adj_edge, adj_high, adj_rays;
+    DevBuf adj_traj, adj_xstep, adj_end;   // the render's recorded steps
     DevBuf band_done;
     // Display transform: blur scratch, glare weights, meter state, 8-bit output.
     DevBuf disp_tmp, disp_near, disp_far, disp_k, disp_state, disp_rgb, disp_frames;
@@ -113,6 +114,12 @@ constexpr int kShadeBlocks = 8192, kShadeBlocksLeast = 64;
 // groups whose copies can be outstanding.
 constexpr size_t kDisplayGroupPixels = 16u << 20;
 constexpr size_t kDisplayEvents = 4;
+// Steps per ray the adjoint's render records: kTrajCap, or as many as the bytes
+// allow (512^2 rays: 512 steps, 7.5 GB); not at all under kTrajCapLeast, where
+// the ordinary ray (150 to 250 steps) would not fit, and not where the record
+// would take more than a quarter of the device memory that is free.
+constexpr int kTrajCap = 512, kTrajCapLeast = 224;
+constexpr size_t kTrajMostBytes = 8ull << 30;
 int fail(bh_ctx* ctx, int code, const std::string& msg) {
     if (ctx) ctx->err = msg;
     return code;
@@ -672,9 +679,9 @@ void bh_gpu_destroy(bh_ctx* ctx) {
     for (DevBuf* b : {&ctx->hits, &ctx->pixels, &ctx->rays, &ctx->frames, &ctx->ray_end, &ctx->deferred,
                       &ctx->partials, &ctx->fstats, &ctx->jet, &ctx->adj_target, &ctx->adj_grad, &ctx->adj_Y,
                       &ctx->adj_ckpt, &ctx->adj_counters, &ctx->adj_sums, &ctx->adj_xr, &ctx->adj_cand, &ctx->adj_edge,
-                      &ctx->adj_high, &ctx->adj_rays, &ctx->eval_in, &ctx->eval_out, &ctx->disp_tmp, &ctx->disp_near,
-                      &ctx->disp_far, &ctx->disp_k, &ctx->disp_state, &ctx->disp_rgb, &ctx->disp_frames, &ctx->sel_flag,
-                      &ctx->sel_list, &ctx->band_done})
+                      &ctx->adj_high, &ctx->adj_rays, &ctx->adj_traj, &ctx->adj_xstep, &ctx->adj_end, &ctx->eval_in,
+                      &ctx->eval_out, &ctx->disp_tmp, &ctx->disp_near, &ctx->disp_far, &ctx->disp_k, &ctx->disp_state,
+                      &ctx->disp_rgb, &ctx->disp_frames, &ctx->sel_flag, &ctx->sel_list, &ctx->band_done})
         if (b->p) cudaFree(b->p);
     cudaFree(ctx->d_table);
     cudaFree(ctx->d_star_pos);
@@ -904,6 +911,23 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
     if ((rc = ensure(ctx, ctx->adj_high, static_cast<size_t>(n_rays))) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->adj_rays, static_cast<size_t>(n_rays) * sizeof(int))) != BH_OK) return rc;
 
+    // The render records its rays' steps where they fit; a ray with more steps
+    // than the cap, and every ray of a larger frame, is integrated again.
+    const size_t step_bytes = static_cast<size_t>(n_rays) * kTrajWords * sizeof(double);
+    const int traj_cap = static_cast<int>(std::min<size_t>(kTrajCap, kTrajMostBytes / step_bytes));
+    bool record = traj_cap >= kTrajCapLeast;
+    if (record && step_bytes * traj_cap > ctx->adj_traj.cap) {
+        size_t free_bytes = 0, all_bytes = 0;
+        CK(cudaMemGetInfo(&free_bytes, &all_bytes));
+        record = step_bytes * traj_cap <= (free_bytes + ctx->adj_traj.cap) / 4;
+    }
+    if (record && (ensure(ctx, ctx->adj_traj, step_bytes * traj_cap) != BH_OK ||
+                   ensure(ctx, ctx->adj_xstep, n_slots * sizeof(int)) != BH_OK ||
+                   ensure(ctx, ctx->adj_end, static_cast<size_t>(n_rays) * kEndWords * sizeof(double)) != BH_OK)) {
+        cudaGetLastError();            // no room: without records
+        record = false;
+    }
+
     CK(cudaMemcpyAsync(ctx->adj_target.p, target, npx * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     ctx->h2d += static_cast<long long>(npx * sizeof(float));
     CK(cudaMemsetAsync(ctx->adj_xr.p, 0, n_slots * sizeof(double), ctx->stream));
@@ -914,6 +938,10 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
         if ((rc = plan_launch(ctx, frames, static_cast<bh_xyz*>(ctx->pixels.p), nullptr, false, p)) != BH_OK)
             return rc;
         p.tl.xing = static_cast<double*>(ctx->adj_xr.p);
+        p.tl.traj = record ? static_cast<double*>(ctx->adj_traj.p) : nullptr;
+        p.tl.traj_cap = traj_cap;
+        p.tl.xing_step = static_cast<int*>(ctx->adj_xstep.p);
+        p.tl.disc_end = static_cast<double*>(ctx->adj_end.p);
         ctx->h2d += static_cast<long long>(p.stage_bytes);
         if ((rc = record_launch(ctx, p, ctx->stream, false)) != BH_OK) return rc;
     }
@@ -931,6 +959,16 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
     L.ckpt = static_cast<double*>(ctx->adj_ckpt.p);
     L.hits = static_cast<const HitRecord*>(ctx->hits.p);
     L.rays = static_cast<int*>(ctx->adj_rays.p);
+    L.traj = record ? static_cast<const double*>(ctx->adj_traj.p) : nullptr;
+    L.traj_cap = traj_cap;
+    L.abort = &ctx->d_queue->abort;
+    L.xing_step = static_cast<const int*>(ctx->adj_xstep.p);
+    L.disc_end = static_cast<const double*>(ctx->adj_end.p);
+    L.grid_reverse = static_cast<int>(std::min<long long>(ctx->sm_count * std::max(1, reverse_blocks_per_sm()),
+                                                          (n_rays + block - 1) / block));
+    L.side_stream = ctx->side_stream;
+    L.fork_event = ctx->fork_event;
+    L.join_event = ctx->join_event;
     L.xing_r = static_cast<double*>(ctx->adj_xr.p);
     L.cand = static_cast<unsigned long long*>(ctx->adj_cand.p);
     L.edge_out = static_cast<double*>(ctx->adj_edge.p);

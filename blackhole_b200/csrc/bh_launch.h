@@ -32,6 +32,20 @@ struct TraceLaunch {
                                      // frame of the launch has a jet
     double* xing;                    // radii of each ray's first two equatorial crossings
                                      // (2 per ray, zeroed before; 0 = none), or null
+    // With xing: the accepted steps of each ray are recorded too, the first
+    // traj_cap of them, kTrajWords doubles each (r, th, p_r, p_th, the step's
+    // size, sin and cos of th, at its start; word w of step j of ray i at
+    // traj[(j kTrajWords + w) total_rays + i]), but for those of a ray that is
+    // falling in (it has no gradient, and the creep to the horizon is most of
+    // its steps).  Null: not.  xing_step: the step of each crossing (2 per ray),
+    // kNotRecorded while falling in; disc_end: where a ray that hit the disc
+    // would go on, kEndWords doubles each (the state at the end of its last
+    // step, the next step's size, the controller's memory, sin and cos of th;
+    // word w of ray i at disc_end[w total_rays + i]).
+    double* traj;
+    int traj_cap;
+    int* xing_step;
+    double* disc_end;
     int surfaces;                    // 1 when a frame of the launch has the Sun or a neutron star
     // Mixed precision: near-critical rays (escaping rays that circle close to
     // the photon shell) traced by a binary64 kernel of grid_side blocks of 64
@@ -59,6 +73,8 @@ struct TraceLaunch {
 // Bytes of one deferred-ray record.
 size_t deferred_record_bytes();
 constexpr size_t kDeferredRecordBytes = 96;   // checked against the record in bh_trace.cu
+
+constexpr int kTrajWords = 7, kEndWords = 10, kNotRecorded = 0x7fffffff;
 
 // Persistent trace kernel over all rays of all frames.
 cudaError_t launch_trace(const TraceLaunch& L, cudaStream_t stream);

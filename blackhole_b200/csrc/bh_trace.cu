@@ -586,6 +586,10 @@ struct TraceArgs {
     unsigned long long budget;
     double* jet;             // jet emission per ray (jet kernels only)
     double* xing;            // first two equatorial crossing radii per ray, or null
+    double* traj;            // recorded steps (TraceLaunch::traj), or null
+    int traj_cap;
+    int* xing_step;
+    double* disc_end;
     int select;              // 0: every ray; 1: near-critical rays only; 2: all others
     const unsigned char* sel_flag;   // per ray: kRay* class from the classification pass, or null
     const int* sel_list;     // the near-critical rays' global ids, or null (then select 1 scans)
@@ -1047,6 +1051,15 @@ __device__ bool attempt(const TraceArgs& A, Lane<P>& L) {
 
     // ---- accepted -----------------------------------------------------------
     L.tries = 0;
+    if constexpr (SURF == kSurfCrossings && !P::kMixed) {
+        // the step for the reverse sweep; a ray that is falling in has none
+        if (A.traj && L.steps < A.traj_cap && !(L.y[1] < F.r_promote && L.k1[1] < 0.0)) {
+            double* p = A.traj + (long long)L.steps * kTrajWords * A.total_rays + L.gid;
+            const double v[kTrajWords] = {L.y[1], L.y[2], L.y[4], L.y[5], L.h, L.sn0, L.c0};
+            #pragma unroll
+            for (int w = 0; w < kTrajWords; ++w) p[w * A.total_rays] = v[w];
+        }
+    }
     ++L.steps;
     const double rn = (double)yn[1];
     const double pt = -(double)L.E, pph = (double)L.Lz;
@@ -1107,9 +1120,12 @@ __device__ bool attempt(const TraceArgs& A, Lane<P>& L) {
             // the crossings the discrete adjoint's edge pass starts from
             double* x = A.xing + 2 * L.gid;
             // (a third one sets the sign of the second's radius)
-            if (x[0] == 0.0) x[0] = rc;
-            else if (x[1] == 0.0) x[1] = rc;
+            const int q = (x[0] == 0.0) ? 0 : (x[1] == 0.0) ? 1 : 2;
+            if (q < 2) x[q] = rc;
             else x[1] = -fabs(x[1]);
+            if (q < 2 && A.traj)
+                A.xing_step[2 * L.gid + q] =
+                    (L.y[1] < F.r_promote && L.k1[1] < 0.0) ? kNotRecorded : L.steps;
         }
         if (rc >= F.r_in && rc <= F.r_out) {
             what = BH_HIT_DISC;
@@ -1288,6 +1304,14 @@ __device__ bool attempt(const TraceArgs& A, Lane<P>& L) {
         state8(L, ptph, yh);
     }
     if (what >= 0) {
+        if constexpr (SURF == kSurfCrossings && !P::kMixed) {
+            if (A.traj && what == BH_HIT_DISC) {
+                const double v[kEndWords] = {L.y[0], L.y[1], L.y[2], L.y[3], L.y[4],
+                                             L.y[5], L.h,    L.errp_mem, L.sn0, L.c0};
+                #pragma unroll
+                for (int w = 0; w < kEndWords; ++w) A.disc_end[w * A.total_rays + L.gid] = v[w];
+            }
+        }
         if (P::kMixed && L.mirror) {          // back to the true angle
             yh[2] = kPi - yh[2];
             yh[6] = -yh[6];
@@ -1486,6 +1510,10 @@ cudaError_t launch_t(const TraceLaunch& L, int grid, int block, cudaStream_t s, 
     A.budget = L.budget;
     A.jet = L.jet;
     A.xing = L.xing;
+    A.traj = L.traj;
+    A.traj_cap = L.traj_cap;
+    A.xing_step = L.xing_step;
+    A.disc_end = L.disc_end;
     A.band_done = L.band_done;
     A.rays_per_band = L.rays_per_band > 0 ? L.rays_per_band : 1;
     trace_kernel<P, MAXREG, JET, SURF, RESUME><<<grid, block, 0, s>>>(A);

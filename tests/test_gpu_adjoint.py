@@ -280,3 +280,105 @@ def test_gradient_descent_recovers_the_scene(renderer):
     assert final < 1e-3 * first
     assert abs(a - 0.7) < 2e-3 and abs(math.degrees(inc) - 50.0) < 0.05
     assert abs(edd - 0.2) < 1e-3 and abs(r_out - 25.0) < 0.05
+
+
+def _check_lib():
+    from blackhole_b200.build import CHECK_LIB, build_check
+
+    if not os.path.exists(CHECK_LIB):
+        build_check()
+    lib = C.CDLL(CHECK_LIB)
+    D, P = C.POINTER(C.c_double), C.POINTER(abi.bh_render_config)
+    lib.bhx_ray.argtypes = [P, C.c_longlong, C.c_double, C.c_int, C.c_int, D]
+    lib.bhx_crossings.argtypes = [P, C.c_longlong, D, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]
+    lib.bhx_edge.argtypes = [P, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_double, D, D]
+    lib.bhx_edge_mask.argtypes = [P, C.c_double, C.c_double, C.POINTER(C.c_int)]
+    return lib
+
+
+def _scene(n, spin, deg):
+    c = workloads.adjoint_512()
+    c.width = c.height = n
+    c.spin, c.cam.theta = spin, math.radians(deg)
+    return c
+
+
+@pytest.mark.parametrize("n,spin,deg,every", [(40, 0.7, 50.0, 37), (160, 0.998, 85.0, 401), (828, 0.7, 50.0, 9973)])
+def test_recorded_and_integrated_rays_match_the_cpu_adjoint(renderer, n, spin, deg, every):
+    """The reverse sweep takes a ray's steps from the render's record; a ray
+    with more than 512 steps, and each ray of a frame of more than 684 784
+    (828^2 here), is integrated again.  Tolerance: 1e-6 of the ray's gradient as
+    above; 1e-4 for the rays of more than 300 steps, which circle the photon
+    shell and grow the two sides' rounding by up to 1e8 before they end."""
+    lib = _check_lib()
+    cfg = _scene(n, spin, deg)
+    Y = _lum(renderer, cfg).reshape(-1)
+    _, per_ray, _ = renderer.adjoint(cfg, np.zeros((n, n), dtype=np.float32), per_ray=True)
+    rays = renderer.trace_rays(cfg)
+    order = abi.work_order(n, n, 1)            # ray id -> trace_rays index
+    longest = np.argsort(rays["steps"][order] * (np.abs(per_ray[order, 0]) > 0))[-12:]
+    c = cfg.to_c()
+    compared = 0
+    for rid in sorted(set(range(0, n * n, every)) | set(int(i) for i in longest)):
+        idx = order[rid]
+        out = np.zeros(9)
+        assert lib.bhx_ray(C.byref(c), rid, 2.0 * Y[idx], 0, 0, out.ctypes.data_as(C.POINTER(C.c_double))) == abi.OK
+        if out[5] != rays["what"][idx]:
+            continue                           # ends at rounding distance from another event
+        tol = 1e-4 if out[6] > 300 else 1e-6
+        compared += 1
+        assert np.allclose(per_ray[idx], out[1:5], rtol=tol, atol=tol * np.abs(out[1:5]).max()), (rid, out)
+    assert compared >= 12
+
+
+@pytest.mark.parametrize("n,spin,deg", [(24, 0.7, 50.0), (33, 0.998, 85.0)])
+def test_edge_terms_match_the_cpu_adjoint(renderer, n, spin, deg):
+    """The edge sums over all candidate crossings (recorded steps, the ray
+    continued past a disc hit) against the CPU-compiled edge term of the same
+    candidates, to 1e-6 of the sum of their magnitudes (as for the rays)."""
+    lib = _check_lib()
+    cfg = _scene(n, spin, deg)
+    Y = _lum(renderer, cfg)
+    g = renderer.adjoint(cfg, np.zeros((n, n), dtype=np.float32))
+    order = abi.work_order(n, n, 1)
+    c = cfg.to_c()
+    D = C.POINTER(C.c_double)
+    r = np.zeros((n, n, 2))
+    for rid in range(n * n):
+        rr, st, cnt = np.zeros(2), (C.c_int * 2)(), C.c_int()
+        assert lib.bhx_crossings(C.byref(c), rid, rr.ctypes.data_as(D), st, C.byref(cnt), None) == abi.OK
+        r[order[rid] // n, order[rid] % n] = rr
+    total, size, cand = np.zeros(3), np.zeros(3), 0
+    for y in range(n):
+        for x in range(n):
+            for j in range(2):
+                rc = r[y, x, j]
+                if rc == 0.0:
+                    break
+                near = [r[b, a, j] for a, b in ((x + 1, y), (x - 1, y), (x, y + 1), (x, y - 1))
+                        if 0 <= a < n and 0 <= b < n and r[b, a, j] != 0.0]
+                m = C.c_int()
+                assert lib.bhx_edge_mask(C.byref(c), rc, max([abs(rc - q) for q in near], default=0.0),
+                                         C.byref(m)) == abi.OK
+                if not m.value:
+                    continue
+                cand += 1
+                out, diag = np.zeros(3), np.zeros(12)
+                assert lib.bhx_edge(C.byref(c), x, y, 0, j + 1, m.value, 2.0 * Y[y, x], out.ctypes.data_as(D),
+                                    diag.ctypes.data_as(D)) == abi.OK
+                total += out
+                size += np.abs(out)
+    assert g["edge_candidates"] == cand and cand > 10
+    got = np.array([g["d_r_out"], g["edge_spin"], g["edge_inclination"]])
+    assert (np.abs(got - total) <= 1e-6 * size).all(), (got, total, size)
+
+
+def test_stopped_adjoint_is_an_error_and_the_next_is_whole(renderer, c4):
+    cfg, target, g, per_ray, _ = c4
+    renderer.set_step_budget(1000)
+    try:
+        with pytest.raises(BHError):
+            renderer.adjoint(cfg, target)
+    finally:
+        renderer.set_step_budget(0)
+    assert renderer.adjoint(cfg, target)["d_spin"] == g["d_spin"]
