@@ -63,6 +63,7 @@ struct bh_ctx {
     CUresult (*wait_value32)(CUstream, CUdeviceptr, cuuint32_t, unsigned int) = nullptr;
     cudaStream_t band_stream[8] = {};
     cudaEvent_t band_join[8] = {};
+    cudaStream_t batch_stream[2] = {};      // a batch's frames are shaded and copied on these
 
     std::vector<double> h_table;
     double* d_table = nullptr;
@@ -454,6 +455,13 @@ void setup_band_pipeline(bh_ctx* ctx) {
             cudaGetLastError();
             return;
         }
+    int least = 0, most_urgent = 0;
+    if (cudaDeviceGetStreamPriorityRange(&least, &most_urgent) != cudaSuccess) most_urgent = 0;
+    for (cudaStream_t& bs : ctx->batch_stream)
+        if (cudaStreamCreateWithPriority(&bs, cudaStreamNonBlocking, most_urgent) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
     // The wait must work here: one on a word this stream has just zeroed
     // (the queue's first counter, zero anyway) returns at once.
     auto wait = reinterpret_cast<CUresult (*)(CUstream, CUdeviceptr, cuuint32_t, unsigned int)>(fn);
@@ -526,6 +534,118 @@ int record_banded(bh_ctx* ctx, Plan& p, const bh_render_config* cfg, bh_xyz* out
     CK(cudaEventRecord(ctx->ev[2], stream));
     CK(launch_reduce(p.rl, stream));
     ctx->d2h += npx * static_cast<long long>(sizeof(bh_xyz));
+    return BH_OK;
+}
+
+// ---- bh_gpu_render_batch's pipeline -----------------------------------------
+// A batch's frames finish in order too.  The persistent trace holds every
+// block slot until its queue is empty, so with it no frame is shaded, and none
+// copied, before the trace ends: the copies, 24 bytes a pixel, are a sixth of a
+// binary32 batch.  Here each warp of the binary32 kernel ends after one batch
+// of rays, and the shading, on streams of the highest priority, takes the
+// slots of the blocks that end.  The trace pays for that (a block's start per
+// 32 rays of a warp, a wider shading block that waits for two slots): 16
+// frames of 256^2 to 1024^2 14.9 ms with the shading inside -> 16.2, but the
+// call 18.1 -> 16.6; 4 of 1024^2 10.1 -> 8.8; 2 of 512^2 2.71 -> 2.35; 6 of 256^2 2.27 -> 2.20.
+// Blocks of 128 threads 16.9, two batches per warp 17.1; one to five streams
+// the same (on eight, some share a hardware queue with the trace's own and
+// wait for its end: 17.2).
+// A binary64 trace takes 4.5 times as long per pixel and the slots' cost with
+// it (6 of 512^2 13.5 -> 14.1 ms), and so does one with a jet or with several
+// samples a pixel; a launch shape set by the user stays as it was set.  Those,
+// and frames so small that the calls per frame would cost more than the
+// overlap gives, are one graph with the copies after it.
+constexpr long long kBatchBandRays = 1 << 14, kBatchBands = 1024;   // rays per counter at least; counters
+constexpr long long kBatchPiecePixels = 1 << 18;                    // 2^17 and 2^18 the same
+constexpr int kBatchShadeBlocks = 1024;                             // 64 to 2048 the same
+constexpr int kBatchBlock = 64;
+constexpr size_t kBatchFramePixels = 1 << 16;
+
+bool batch_goes_out_early(const bh_ctx* ctx, const Plan& p, size_t npx) {
+    return ctx->wait_value32 && p.mixed && !p.tl.jet && !ctx->launch_set[1] &&
+           p.rays < 2 * static_cast<long long>(npx) && npx >= kBatchFramePixels * std::max(p.n, 2);
+}
+
+// The launch of plan `p` (frames of a batch, d_pixels on the device) with each
+// frame shaded and copied to the host in pieces as they finish.
+int record_batch(bh_ctx* ctx, Plan& p, const std::vector<FrameParams>& frames, bh_xyz* const* outs,
+                 cudaStream_t stream) {
+    const int n = p.n;
+    constexpr int kStreams = sizeof ctx->batch_stream / sizeof ctx->batch_stream[0];
+    // a band of the counters: rays of the launch, whatever frame they are of
+    const long long band = std::max(kBatchBandRays, (p.rays + kBatchBands - 1) / kBatchBands);
+    const int nb = static_cast<int>((p.rays + band - 1) / band);
+    // rows of a piece: a multiple of the 4-row pixel order
+    auto piece_rows = [](const FrameParams& F) {
+        return std::max<long long>(4, (kBatchPiecePixels / F.width) & ~3ll);
+    };
+    int most = 1;
+    for (const FrameParams& F : frames)
+        most = std::max(most, static_cast<int>((F.height + piece_rows(F) - 1) / piece_rows(F)));
+    const int grid = shade_blocks(kBatchPiecePixels, kBatchShadeBlocks);
+    int rc;
+    if ((rc = ensure(ctx, ctx->band_done, static_cast<size_t>(nb) * sizeof(unsigned int))) != BH_OK) return rc;
+    const size_t flux = static_cast<size_t>(n) * most * grid;
+    if ((rc = ensure(ctx, ctx->partials, flux * sizeof(double))) != BH_OK) return rc;
+    p.rl.flux = static_cast<double*>(ctx->partials.p);
+    p.rl.flux_per_frame = most * grid;
+    unsigned int* done = static_cast<unsigned int*>(ctx->band_done.p);
+    p.tl.band_done = done;
+    p.tl.rays_per_band = band;
+    p.tl.nbands = nb;
+    p.tl.draws = 1;
+    p.tl.refill = 32;            // a warp's one draw hands a ray to each lane
+    p.tl.block_size = kBatchBlock;
+    const long long per_block = static_cast<long long>(kBatchBlock) * p.tl.rays_per_thread;
+    p.tl.grid = static_cast<int>(std::max<long long>(1, (p.rays + per_block - 1) / per_block));
+    const unsigned char* st = ctx->stage;
+    const size_t fbytes = static_cast<size_t>(p.nf) * sizeof(FrameParams);
+    CK(cudaMemcpyAsync(ctx->frames.p, st, fbytes, cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(ctx->ray_end.p, st + fbytes, n * sizeof(long long), cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(ctx->d_queue, st + fbytes + n * sizeof(long long), sizeof(QueueState), cudaMemcpyHostToDevice,
+                       stream));
+    CK(cudaEventRecord(ctx->stage_free, stream));
+    CK(cudaMemsetAsync(done, 0, static_cast<size_t>(nb) * sizeof(unsigned int), stream));
+    CK(cudaMemsetAsync(ctx->fstats.p, 0, n * sizeof(FrameStats), stream));
+    CK(cudaMemsetAsync(ctx->partials.p, 0, flux * sizeof(double), stream));
+    CK(cudaEventRecord(ctx->ev[0], stream));
+    for (cudaStream_t bs : ctx->batch_stream) CK(cudaStreamWaitEvent(bs, ctx->ev[0], 0));
+    if (p.rays > 0) CK(launch_trace(p.tl, stream));
+    CK(cudaEventRecord(ctx->ev[1], stream));
+    int piece = 0;
+    for (int f = 0; f < n; ++f) {
+        const FrameParams& F = frames[f];
+        const long long rows = piece_rows(F);
+        const int SS = F.S * F.S;
+        for (long long y = 0, k = 0; y < F.height; y += rows, ++k, ++piece) {
+            cudaStream_t bs = ctx->batch_stream[piece % kStreams];
+            const long long lo = y * F.width, hi = std::min<long long>(F.height, y + rows) * F.width;
+            for (long long b = (F.ray_begin + lo * SS) / band; b <= (F.ray_begin + hi * SS - 1) / band; ++b) {
+                const long long rays = std::min(p.rays, (b + 1) * band) - b * band;
+                if (ctx->wait_value32(bs, reinterpret_cast<CUdeviceptr>(done + b), static_cast<cuuint32_t>(rays),
+                                      CU_STREAM_WAIT_VALUE_GEQ) != CUDA_SUCCESS)
+                    return fail(ctx, BH_ERR_CUDA, "stream wait on a batch's rays failed");
+            }
+            ShadeLaunch sl = p.sl;
+            sl.frames += f;
+            sl.nframes = 1;
+            sl.stats += f;
+            sl.pixel_lo = lo;
+            sl.pixel_hi = hi;
+            sl.blocks = grid;
+            sl.flux = static_cast<double*>(ctx->partials.p) + (static_cast<size_t>(f) * most + k) * grid;
+            CK(launch_shade(sl, bs));
+            CK(cudaMemcpyAsync(outs[f] + lo, static_cast<bh_xyz*>(ctx->pixels.p) + F.pixel_begin + lo,
+                               static_cast<size_t>(hi - lo) * sizeof(bh_xyz), cudaMemcpyDeviceToHost, bs));
+            ctx->d2h += (hi - lo) * static_cast<long long>(sizeof(bh_xyz));
+        }
+    }
+    for (int i = 0; i < kStreams; ++i) {
+        CK(cudaEventRecord(ctx->band_join[i], ctx->batch_stream[i]));
+        CK(cudaStreamWaitEvent(stream, ctx->band_join[i], 0));
+    }
+    CK(cudaEventRecord(ctx->ev[2], stream));
+    CK(launch_reduce(p.rl, stream));
     return BH_OK;
 }
 
@@ -690,6 +810,8 @@ void bh_gpu_destroy(bh_ctx* ctx) {
     cudaFree(ctx->d_queue);
     if (ctx->h_one) cudaFreeHost(ctx->h_one);
     if (ctx->h_readback) cudaFreeHost(ctx->h_readback);
+    for (cudaStream_t st : ctx->batch_stream)
+        if (st) cudaStreamDestroy(st);
     for (cudaStream_t st : ctx->band_stream)
         if (st) cudaStreamDestroy(st);
     for (cudaEvent_t ev : ctx->band_join)
@@ -815,15 +937,21 @@ int bh_gpu_render_batch(bh_ctx* ctx, const bh_render_config* cfgs, int n, bh_xyz
     size_t npx = 0;
     for (int i = 0; i < n; ++i) npx += static_cast<size_t>(cfgs[i].width) * cfgs[i].height;
     if ((rc = ensure(ctx, ctx->pixels, npx * sizeof(bh_xyz))) != BH_OK) return rc;
-    // The whole batch is one CUDA graph: staging copies, the persistent trace
-    // launch over every frame's rays (plus the binary64 pass), shading and the
-    // stats.  It is captured once per batch shape and replayed while the shape
-    // (frame count, sizes, buffers, launch shape) stays the same; the frame
-    // constants change freely, they are read from the pinned staging buffer.
     Plan p;
     if ((rc = plan_launch(ctx, frames, static_cast<bh_xyz*>(ctx->pixels.p), nullptr, false, p)) != BH_OK)
         return rc;
     ctx->h2d += static_cast<long long>(p.stage_bytes);
+    if (batch_goes_out_early(ctx, p, npx)) {
+        if ((rc = record_batch(ctx, p, frames, outs, ctx->stream)) != BH_OK) return rc;
+        CK(cudaStreamSynchronize(ctx->stream));
+        const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+        return finish(ctx, n, stats, nullptr, true, secs);
+    }
+    // Otherwise the whole batch is one CUDA graph: staging copies, the persistent trace
+    // launch over every frame's rays (plus the binary64 pass), shading and the
+    // stats.  It is captured once per batch shape and replayed while the shape
+    // (frame count, sizes, buffers, launch shape) stays the same; the frame
+    // constants change freely, they are read from the pinned staging buffer.
     std::vector<unsigned char> key(sizeof p.tl + sizeof p.sl + sizeof p.rl + sizeof(void*) + sizeof(size_t));
     {
         unsigned char* k = key.data();

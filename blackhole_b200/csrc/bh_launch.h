@@ -20,6 +20,8 @@ struct TraceLaunch {
     int precision;                   // BH_PRECISION_*
     int block_size;
     int grid;                        // blocks
+    int draws;                       // batches of rays a warp takes before it ends, with refill 32 and a
+                                     // grid to match (0: until none is left)
     int rays_per_thread;
     int refill;
     unsigned long long budget;       // step-attempt budget of the launch, 0 = none

@@ -581,6 +581,7 @@ struct TraceArgs {
     HitRecord* hits;
     QueueState* queue;
     Deferred* deferred;      // mixed: append target; resume: source
+    int draws;               // batches a warp takes before it ends (0: as many as there are)
     int rays_per_thread;
     int refill;
     unsigned long long budget;
@@ -1372,6 +1373,7 @@ __global__ void __maxnreg__(MAXREG) trace_kernel(TraceArgs A) {
     bool active = false, done = false;
     long long q_next = 0;
     int q_left = 0, q_stride = 0;
+    int draws = A.draws;
     while (true) {
         const unsigned want = __ballot_sync(kFull, !active && !done && q_left == 0);
         if (want) {
@@ -1382,11 +1384,12 @@ __global__ void __maxnreg__(MAXREG) trace_kernel(TraceArgs A) {
                 unsigned long long base = 0;
                 int stop = 0;
                 if (lane == leader) {
-                    stop = *(volatile int*)&A.queue->abort;
+                    stop = *(volatile int*)&A.queue->abort | (draws < 0);
                     if (!stop) base = atomicAdd(counter, (unsigned long long)n * A.rays_per_thread);
                 }
                 base = __shfl_sync(kFull, base, leader);
                 stop = __shfl_sync(kFull, stop, leader);
+                if (draws > 0 && --draws == 0) draws = -1;
                 if (want & (1u << lane)) {
                     if (stop) {
                         done = true;
@@ -1497,6 +1500,7 @@ cudaError_t launch_t(const TraceLaunch& L, int grid, int block, cudaStream_t s, 
     A.hits = L.hits;
     A.queue = L.queue;
     A.deferred = static_cast<Deferred*>(L.deferred);
+    A.draws = (select == 1 || RESUME) ? 0 : L.draws;
     A.rays_per_thread = L.rays_per_thread < 1 ? 1 : L.rays_per_thread;
     A.refill = L.refill < 1 ? 1 : (L.refill > 32 ? 32 : L.refill);
     A.select = select;

@@ -32,7 +32,7 @@ sys.path.insert(0, HERE)
 from cases import CASES, RENDER_CASE, kerr_a09_i60  # noqa: E402
 from parity import compare, q, summary, window_of  # noqa: E402
 
-from blackhole_b200 import BHError, RenderConfig, RenderStats, abi  # noqa: E402
+from blackhole_b200 import BHError, RenderConfig, Renderer, RenderStats, abi  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -426,3 +426,52 @@ def test_invariant_diagnostics_of_a_full_frame(renderer):
     sm = RenderStats()
     renderer.render(cfg, sm)
     assert sm.max_norm_error < 1e-2 and sm.max_carter_drift < 1e-1
+
+
+@pytest.mark.parametrize("sizes", [
+    [(256, 256), (256, 256)],                       # the smallest that goes out frame by frame
+    [(512, 515), (70, 67), (263, 1030), (1, 200)],  # pieces of one frame, ragged rows, a frame of one column
+    [(600, 300)] * 3 + [(3, 3)],
+])
+def test_batch_copied_while_it_is_traced_equals_single_frames(sizes):
+    """A binary32 batch is shaded and copied in pieces as its rays finish; each
+    frame equals its own render bit for bit, the counts too, the flux to the
+    order of its sum (2^-52 per term of a tree over 1e5 pixels: 1e-12)."""
+    renderer = Renderer(0)        # no launch shape set: a set one takes the graph
+    cfgs = []
+    for i, (w, h) in enumerate(sizes):
+        c = kerr_a09_i60(width=w, height=h)
+        c.precision = abi.PRECISION_MIXED
+        c.cam.phi += 0.1 * i
+        cfgs.append(c)
+    stats = []
+    frames = renderer.render_batch(cfgs, stats)
+    for c, px, st in zip(cfgs, frames, stats):
+        one = RenderStats()
+        assert np.array_equal(px, renderer.render(c, one))
+        assert (st.rays, st.steps, st.captured, st.disc_hits, st.escaped, st.exhausted) == \
+            (one.rays, one.steps, one.captured, one.disc_hits, one.escaped, one.exhausted)
+        assert st.total_flux == pytest.approx(one.total_flux, rel=1e-12)
+
+
+@pytest.mark.parametrize("stop", ["budget", "abort"])
+def test_batch_copied_while_it_is_traced_ends_when_stopped(stop):
+    renderer = Renderer(0)
+    cfgs = []
+    for i in range(3):
+        c = kerr_a09_i60(width=320, height=256)
+        c.precision = abi.PRECISION_MIXED
+        cfgs.append(c)
+    if stop == "budget":
+        renderer.set_step_budget(5000)
+    else:
+        renderer.request_abort()
+    try:
+        with pytest.raises(BHError) as e:
+            renderer.render_batch(cfgs)
+        assert e.value.code == (abi.ERR_BUDGET if stop == "budget" else abi.ERR_ABORTED)
+    finally:
+        renderer.set_step_budget(0)
+        renderer.clear_abort()
+    a, b, c = renderer.render_batch(cfgs)
+    assert np.array_equal(a, b) and np.array_equal(a, c) and np.isfinite(a).all()
