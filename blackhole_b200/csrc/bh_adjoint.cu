@@ -287,9 +287,9 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjBlocksPerSm) adjoint_kernel(con
 // record, then each step backwards from its record.  The lanes of a warp walk
 // the same step numbers, from the longest ray's last, so that their loads
 // coalesce (56 bytes a ray and step, 2.3 GB at 512^2: 0.35 ms of the kernel's
-// 4.4).  Bound by the latency of a step's chain of binary64 operations; 10
-// warps per SM with 200 registers: 8.3 ms per 512^2 gradient, 8 warps 8.8, 12
-// warps 8.4.
+// 4.4).  Bound by the latency of a step's chain of binary64 operations.  At
+// least 5 blocks per SM: 168 registers, with which 6 fit (12 warps), 8.3 ms per
+// 512^2 gradient; at least 4 (8 warps) 8.8.
 constexpr int kReverseBlocksPerSm = 5;
 __global__ void __launch_bounds__(kAdjBlock, kReverseBlocksPerSm)
 reverse_kernel(const __grid_constant__ AdjointLaunch L) {

@@ -63,7 +63,11 @@ struct bh_ctx {
     CUresult (*wait_value32)(CUstream, CUdeviceptr, cuuint32_t, unsigned int) = nullptr;
     cudaStream_t band_stream[8] = {};
     cudaEvent_t band_join[8] = {};
-    cudaStream_t batch_stream[2] = {};      // a batch's frames are shaded and copied on these
+    // A batch's pipeline: its frames are shaded and copied on the first two, its
+    // finished-ray counters read on the third into pinned memory.
+    cudaStream_t batch_stream[2] = {};
+    cudaStream_t poll_stream = nullptr;
+    unsigned int* h_bands = nullptr;
 
     std::vector<double> h_table;
     double* d_table = nullptr;
@@ -455,13 +459,6 @@ void setup_band_pipeline(bh_ctx* ctx) {
             cudaGetLastError();
             return;
         }
-    int least = 0, most_urgent = 0;
-    if (cudaDeviceGetStreamPriorityRange(&least, &most_urgent) != cudaSuccess) most_urgent = 0;
-    for (cudaStream_t& bs : ctx->batch_stream)
-        if (cudaStreamCreateWithPriority(&bs, cudaStreamNonBlocking, most_urgent) != cudaSuccess) {
-            cudaGetLastError();
-            return;
-        }
     // The wait must work here: one on a word this stream has just zeroed
     // (the queue's first counter, zero anyway) returns at once.
     auto wait = reinterpret_cast<CUresult (*)(CUstream, CUdeviceptr, cuuint32_t, unsigned int)>(fn);
@@ -548,8 +545,11 @@ int record_banded(bh_ctx* ctx, Plan& p, const bh_render_config* cfg, bh_xyz* out
 // frames of 256^2 to 1024^2 14.9 ms with the shading inside -> 16.2, but the
 // call 18.1 -> 16.6; 4 of 1024^2 10.1 -> 8.8; 2 of 512^2 2.71 -> 2.35; 6 of 256^2 2.27 -> 2.20.
 // Blocks of 128 threads 16.9, two batches per warp 17.1; one to five streams
-// the same (on eight, some share a hardware queue with the trace's own and
-// wait for its end: 17.2).
+// the same.  The host, which has to wait for the call's end anyway, reads the
+// counters and launches a piece when its rays are done: with stream waits on
+// the counters, as in the row-band pipeline, a call in four ran with none of
+// them served before the trace's end (64 frames 225 instead of 194 ms; the
+// graph 217).
 // A binary64 trace takes 4.5 times as long per pixel and the slots' cost with
 // it (6 of 512^2 13.5 -> 14.1 ms), and so does one with a jet or with several
 // samples a pixel; a launch shape set by the user stays as it was set.  Those,
@@ -562,8 +562,23 @@ constexpr int kBatchBlock = 64;
 constexpr size_t kBatchFramePixels = 1 << 16;
 
 bool batch_goes_out_early(const bh_ctx* ctx, const Plan& p, size_t npx) {
-    return ctx->wait_value32 && p.mixed && !p.tl.jet && !ctx->launch_set[1] &&
+    return p.mixed && !p.tl.jet && !ctx->launch_set[1] &&
            p.rays < 2 * static_cast<long long>(npx) && npx >= kBatchFramePixels * std::max(p.n, 2);
+}
+
+// False: not set up, and the batch takes the graph.
+bool setup_batch_pipeline(bh_ctx* ctx) {
+    if (ctx->h_bands) return true;
+    int least = 0, most_urgent = 0;
+    bool ok = cudaDeviceGetStreamPriorityRange(&least, &most_urgent) == cudaSuccess;
+    for (cudaStream_t& bs : ctx->batch_stream)
+        ok = ok && (bs || cudaStreamCreateWithPriority(&bs, cudaStreamNonBlocking, most_urgent) == cudaSuccess);
+    ok = ok && (ctx->poll_stream ||
+                cudaStreamCreateWithFlags(&ctx->poll_stream, cudaStreamNonBlocking) == cudaSuccess);
+    ok = ok && cudaHostAlloc(reinterpret_cast<void**>(&ctx->h_bands), kBatchBands * sizeof(unsigned int),
+                             cudaHostAllocDefault) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok;
 }
 
 // The launch of plan `p` (frames of a batch, d_pixels on the device) with each
@@ -610,35 +625,55 @@ int record_batch(bh_ctx* ctx, Plan& p, const std::vector<FrameParams>& frames, b
     CK(cudaMemsetAsync(ctx->partials.p, 0, flux * sizeof(double), stream));
     CK(cudaEventRecord(ctx->ev[0], stream));
     for (cudaStream_t bs : ctx->batch_stream) CK(cudaStreamWaitEvent(bs, ctx->ev[0], 0));
+    CK(cudaStreamWaitEvent(ctx->poll_stream, ctx->ev[0], 0));
     if (p.rays > 0) CK(launch_trace(p.tl, stream));
     CK(cudaEventRecord(ctx->ev[1], stream));
-    int piece = 0;
+    struct Piece {
+        int frame, k;
+        long long lo, hi, band_lo, band_hi;
+    };
+    std::vector<Piece> pieces;
     for (int f = 0; f < n; ++f) {
         const FrameParams& F = frames[f];
-        const long long rows = piece_rows(F);
-        const int SS = F.S * F.S;
-        for (long long y = 0, k = 0; y < F.height; y += rows, ++k, ++piece) {
-            cudaStream_t bs = ctx->batch_stream[piece % kStreams];
+        const long long rows = piece_rows(F), SS = static_cast<long long>(F.S) * F.S;
+        for (long long y = 0; y < F.height; y += rows) {
             const long long lo = y * F.width, hi = std::min<long long>(F.height, y + rows) * F.width;
-            for (long long b = (F.ray_begin + lo * SS) / band; b <= (F.ray_begin + hi * SS - 1) / band; ++b) {
-                const long long rays = std::min(p.rays, (b + 1) * band) - b * band;
-                if (ctx->wait_value32(bs, reinterpret_cast<CUdeviceptr>(done + b), static_cast<cuuint32_t>(rays),
-                                      CU_STREAM_WAIT_VALUE_GEQ) != CUDA_SUCCESS)
-                    return fail(ctx, BH_ERR_CUDA, "stream wait on a batch's rays failed");
-            }
-            ShadeLaunch sl = p.sl;
-            sl.frames += f;
-            sl.nframes = 1;
-            sl.stats += f;
-            sl.pixel_lo = lo;
-            sl.pixel_hi = hi;
-            sl.blocks = grid;
-            sl.flux = static_cast<double*>(ctx->partials.p) + (static_cast<size_t>(f) * most + k) * grid;
-            CK(launch_shade(sl, bs));
-            CK(cudaMemcpyAsync(outs[f] + lo, static_cast<bh_xyz*>(ctx->pixels.p) + F.pixel_begin + lo,
-                               static_cast<size_t>(hi - lo) * sizeof(bh_xyz), cudaMemcpyDeviceToHost, bs));
-            ctx->d2h += (hi - lo) * static_cast<long long>(sizeof(bh_xyz));
+            pieces.push_back({f, static_cast<int>(y / rows), lo, hi, (F.ray_begin + lo * SS) / band,
+                              (F.ray_begin + hi * SS - 1) / band});
         }
+    }
+    // The counters only grow, and are raised to their bands' sizes when the
+    // trace ends, however it ends.
+    const unsigned int* seen = ctx->h_bands;
+    for (int launched = 0; !pieces.empty();) {
+        CK(cudaMemcpyAsync(ctx->h_bands, done, static_cast<size_t>(nb) * sizeof(unsigned int), cudaMemcpyDeviceToHost,
+                           ctx->poll_stream));
+        CK(cudaStreamSynchronize(ctx->poll_stream));
+        size_t left = 0;
+        for (const Piece& q : pieces) {
+            bool ready = true;
+            for (long long b = q.band_lo; b <= q.band_hi && ready; ++b)
+                ready = seen[b] >= std::min(p.rays, (b + 1) * band) - b * band;
+            if (!ready) {
+                pieces[left++] = q;
+                continue;
+            }
+            cudaStream_t bs = ctx->batch_stream[launched++ % kStreams];
+            ShadeLaunch sl = p.sl;
+            sl.frames += q.frame;
+            sl.nframes = 1;
+            sl.stats += q.frame;
+            sl.pixel_lo = q.lo;
+            sl.pixel_hi = q.hi;
+            sl.blocks = grid;
+            sl.flux = static_cast<double*>(ctx->partials.p) + (static_cast<size_t>(q.frame) * most + q.k) * grid;
+            CK(launch_shade(sl, bs));
+            CK(cudaMemcpyAsync(outs[q.frame] + q.lo,
+                               static_cast<bh_xyz*>(ctx->pixels.p) + frames[q.frame].pixel_begin + q.lo,
+                               static_cast<size_t>(q.hi - q.lo) * sizeof(bh_xyz), cudaMemcpyDeviceToHost, bs));
+            ctx->d2h += (q.hi - q.lo) * static_cast<long long>(sizeof(bh_xyz));
+        }
+        pieces.resize(left);
     }
     for (int i = 0; i < kStreams; ++i) {
         CK(cudaEventRecord(ctx->band_join[i], ctx->batch_stream[i]));
@@ -810,8 +845,9 @@ void bh_gpu_destroy(bh_ctx* ctx) {
     cudaFree(ctx->d_queue);
     if (ctx->h_one) cudaFreeHost(ctx->h_one);
     if (ctx->h_readback) cudaFreeHost(ctx->h_readback);
-    for (cudaStream_t st : ctx->batch_stream)
+    for (cudaStream_t st : {ctx->batch_stream[0], ctx->batch_stream[1], ctx->poll_stream})
         if (st) cudaStreamDestroy(st);
+    if (ctx->h_bands) cudaFreeHost(ctx->h_bands);
     for (cudaStream_t st : ctx->band_stream)
         if (st) cudaStreamDestroy(st);
     for (cudaEvent_t ev : ctx->band_join)
@@ -941,7 +977,7 @@ int bh_gpu_render_batch(bh_ctx* ctx, const bh_render_config* cfgs, int n, bh_xyz
     if ((rc = plan_launch(ctx, frames, static_cast<bh_xyz*>(ctx->pixels.p), nullptr, false, p)) != BH_OK)
         return rc;
     ctx->h2d += static_cast<long long>(p.stage_bytes);
-    if (batch_goes_out_early(ctx, p, npx)) {
+    if (batch_goes_out_early(ctx, p, npx) && setup_batch_pipeline(ctx)) {
         if ((rc = record_batch(ctx, p, frames, outs, ctx->stream)) != BH_OK) return rc;
         CK(cudaStreamSynchronize(ctx->stream));
         const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();

@@ -307,10 +307,14 @@ int  bh_gpu_render_device(bh_ctx* ctx, const bh_render_config* cfg,
 int  bh_gpu_trace_rays(bh_ctx* ctx, const bh_render_config* cfg,
                        bh_ray_result* out, bh_render_stats* stats);
 
-/* Many frames of any size in one persistent launch (replaces the serial frame
+/* Many frames of any size in one launch (replaces the serial frame
    loop of main.cpp:952-989).  outs[i] receives frame i's pixels; stats[i]
    (optional array) receives frame i's counters.  All frames must share the
-   precision, sky and star settings of cfgs[0].  The batch runs as one CUDA
+   precision, sky and star settings of cfgs[0].  A mixed-precision batch
+   without jets at one sample a pixel, of 256^2 pixels a frame or more on
+   average, with no launch shape set, is shaded and copied out while the rest
+   is traced: kernel_ms is the device time of the trace with the shading beside
+   it and shade_ms what follows it.  Any other batch runs as one CUDA
    graph (staging copies, trace, shade, stats), captured on the first call and
    replayed while the batch shape (frame count and sizes, launch parameters,
    buffers) is unchanged; kernel_ms is then the device time of the whole graph
