@@ -84,6 +84,14 @@ __host__ __device__ __forceinline__ void pixel_xy(int W, int H, long long p, int
     *y = y0 + rel % bh;
 }
 
+// Whether the window [base - half, base + half] of `n` bins in a circle lies
+// within one turn, for any `base`: no sum that could overflow, since the bin of
+// a direction that is not finite (the record of a ray that a stop left
+// untraced) is the most negative int.  half <= n / 2.
+__host__ __device__ __forceinline__ bool whole_window(int base, int half, int n) {
+    return base >= half && base < n - half;
+}
+
 // The inverse of pixel_xy: the frame-local pixel index of pixel (x, y).
 __host__ __device__ __forceinline__ long long pixel_index(int W, int H, int x, int y) {
     const int band = y >> 2;

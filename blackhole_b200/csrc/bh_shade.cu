@@ -140,20 +140,21 @@ __device__ void sky_radiance(const SkyData& sky, const FrameParams& F, const dou
                 o[2] += w * c.y * c.z;
             }
         };
-        const int lo = pbase - sp, hi = pbase + sp;
-        if (lo >= 0 && hi < kLon) {
+        if (whole_window(pbase, sp, kLon)) {
             // the window's bins of a row are neighbours, and so are their stars:
             // one run per row
             for (int a = -F.span_t; a <= F.span_t; ++a) {
                 const int ti = it + a;
                 if (ti < 0 || ti >= kLat) continue;
-                stars(__ldg(&sky.bin_start[ti * kLon + lo]), __ldg(&sky.bin_start[ti * kLon + hi + 1]));
+                const int bin = ti * kLon + pbase;
+                stars(__ldg(&sky.bin_start[bin - sp]), __ldg(&sky.bin_start[bin + sp + 1]));
             }
         } else {
+            const int base = ((pbase % kLon) + kLon) % kLon;
             for (int a = -F.span_t; a <= F.span_t; ++a) {
                 const int ti = it + a;
                 if (ti < 0 || ti >= kLat) continue;
-                for (int b = lo; b <= hi; ++b) {
+                for (int b = base - sp; b <= base + sp; ++b) {
                     const int pi = ((b % kLon) + kLon) % kLon;
                     const int bin = ti * kLon + pi;
                     stars(__ldg(&sky.bin_start[bin]), __ldg(&sky.bin_start[bin + 1]));

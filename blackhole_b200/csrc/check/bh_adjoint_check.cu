@@ -207,6 +207,9 @@ int bhx_edge_mask(const bh_render_config* cfg, double rc, double dmax, int* mask
     return BH_OK;
 }
 
+// whole_window of the star bins around column `base`.
+int bhx_star_window(int base, int half) { return whole_window(base, half, kLon) ? 1 : 0; }
+
 // The image-plane position (su, sv, x, y in pixels) of sample k of pixel (px, py).
 int bhx_sample_position(const bh_render_config* cfg, int px, int py, int k, double out[4]) {
     std::lock_guard<std::mutex> lock(g_mu);
