@@ -66,6 +66,7 @@ struct bh_ctx {
     // A batch's pipeline: its frames are shaded and copied on the first two, its
     // finished-ray counters read on the third into pinned memory.
     cudaStream_t batch_stream[2] = {};
+    cudaEvent_t batch_join[2] = {};
     cudaStream_t poll_stream = nullptr;
     unsigned int* h_bands = nullptr;
 
@@ -573,6 +574,8 @@ bool setup_batch_pipeline(bh_ctx* ctx) {
     bool ok = cudaDeviceGetStreamPriorityRange(&least, &most_urgent) == cudaSuccess;
     for (cudaStream_t& bs : ctx->batch_stream)
         ok = ok && (bs || cudaStreamCreateWithPriority(&bs, cudaStreamNonBlocking, most_urgent) == cudaSuccess);
+    for (cudaEvent_t& ev : ctx->batch_join)
+        ok = ok && (ev || cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess);
     ok = ok && (ctx->poll_stream ||
                 cudaStreamCreateWithFlags(&ctx->poll_stream, cudaStreamNonBlocking) == cudaSuccess);
     ok = ok && cudaHostAlloc(reinterpret_cast<void**>(&ctx->h_bands), kBatchBands * sizeof(unsigned int),
@@ -676,8 +679,8 @@ int record_batch(bh_ctx* ctx, Plan& p, const std::vector<FrameParams>& frames, b
         pieces.resize(left);
     }
     for (int i = 0; i < kStreams; ++i) {
-        CK(cudaEventRecord(ctx->band_join[i], ctx->batch_stream[i]));
-        CK(cudaStreamWaitEvent(stream, ctx->band_join[i], 0));
+        CK(cudaEventRecord(ctx->batch_join[i], ctx->batch_stream[i]));
+        CK(cudaStreamWaitEvent(stream, ctx->batch_join[i], 0));
     }
     CK(cudaEventRecord(ctx->ev[2], stream));
     CK(launch_reduce(p.rl, stream));
@@ -847,6 +850,8 @@ void bh_gpu_destroy(bh_ctx* ctx) {
     if (ctx->h_readback) cudaFreeHost(ctx->h_readback);
     for (cudaStream_t st : {ctx->batch_stream[0], ctx->batch_stream[1], ctx->poll_stream})
         if (st) cudaStreamDestroy(st);
+    for (cudaEvent_t ev : ctx->batch_join)
+        if (ev) cudaEventDestroy(ev);
     if (ctx->h_bands) cudaFreeHost(ctx->h_bands);
     for (cudaStream_t st : ctx->band_stream)
         if (st) cudaStreamDestroy(st);
