@@ -142,6 +142,17 @@ int cuda_fail(bh_ctx* ctx, cudaError_t e, const char* what) {
         if (e_ != cudaSuccess) return cuda_fail(ctx, e_, #call); \
     } while (0)
 
+// Held by a call that copies into its caller's memory (or its own frame):
+// unless the call has waited for its copies itself (`waited`), its return waits
+// for all of the context's streams, so that a call that fails half-way leaves
+// nothing under way into memory that may be gone.
+struct CopiesEnd {
+    bh_ctx* ctx;
+    bool waited = false;
+    explicit CopiesEnd(bh_ctx* c) : ctx(c) {}
+    ~CopiesEnd();
+};
+
 int ensure(bh_ctx* ctx, DevBuf& b, size_t bytes) {
     if (bytes <= b.cap) return BH_OK;
     if (b.p) {
@@ -242,6 +253,15 @@ void stats_add(bh_render_stats* s, const FrameStats& f) {
     s->max_norm_error = std::max(s->max_norm_error, mn);
     s->max_carter_drift = std::max(s->max_carter_drift, mq);
     s->total_flux += f.total_flux;
+}
+
+CopiesEnd::~CopiesEnd() {
+    if (waited) return;
+    for (cudaStream_t st : {ctx->stream, ctx->side_stream, ctx->copy_stream, ctx->poll_stream, ctx->batch_stream[0],
+                            ctx->batch_stream[1]})
+        if (st) cudaStreamSynchronize(st);
+    for (cudaStream_t st : ctx->band_stream)
+        if (st) cudaStreamSynchronize(st);
 }
 
 // One launch of the pipeline, planned on the host.
@@ -885,6 +905,7 @@ int bh_gpu_render(bh_ctx* ctx, const bh_render_config* cfg, bh_xyz* out_pixels, 
     if (rc != BH_OK) return rc;
     const size_t npx = static_cast<size_t>(cfg->width) * cfg->height;
     if ((rc = ensure(ctx, ctx->pixels, npx * sizeof(bh_xyz))) != BH_OK) return rc;
+    CopiesEnd copies(ctx);
     if (ctx->wait_value32 && cfg->height >= 2 * kBandRows) {
         // rows shaded and copied out band by band while the frame is traced
         Plan p;
@@ -900,6 +921,7 @@ int bh_gpu_render(bh_ctx* ctx, const bh_render_config* cfg, bh_xyz* out_pixels, 
     }
     if ((rc = enqueue_readback(ctx, ctx->stream)) != BH_OK) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
+    copies.waited = true;
     const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     bh_render_stats local;
     std::memset(&local, 0, sizeof local);
@@ -953,6 +975,7 @@ int bh_gpu_trace_rays(bh_ctx* ctx, const bh_render_config* cfg, bh_ray_result* o
     const size_t nr = static_cast<size_t>(frames[0].n_rays);
     if ((rc = ensure(ctx, ctx->pixels, npx * sizeof(bh_xyz))) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->rays, nr * sizeof(bh_ray_result))) != BH_OK) return rc;
+    CopiesEnd copies(ctx);
     rc = enqueue(ctx, frames, static_cast<bh_xyz*>(ctx->pixels.p), static_cast<bh_ray_result*>(ctx->rays.p),
                  ctx->stream, true);
     if (rc != BH_OK) return rc;
@@ -960,6 +983,7 @@ int bh_gpu_trace_rays(bh_ctx* ctx, const bh_render_config* cfg, bh_ray_result* o
     ctx->d2h += static_cast<long long>(nr * sizeof(bh_ray_result));
     if ((rc = enqueue_readback(ctx, ctx->stream)) != BH_OK) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
+    copies.waited = true;
     const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return finish(ctx, 1, stats, nullptr, true, secs, true);
 }
@@ -982,9 +1006,11 @@ int bh_gpu_render_batch(bh_ctx* ctx, const bh_render_config* cfgs, int n, bh_xyz
     if ((rc = plan_launch(ctx, frames, static_cast<bh_xyz*>(ctx->pixels.p), nullptr, false, p)) != BH_OK)
         return rc;
     ctx->h2d += static_cast<long long>(p.stage_bytes);
+    CopiesEnd copies(ctx);
     if (batch_goes_out_early(ctx, p, npx) && setup_batch_pipeline(ctx)) {
         if ((rc = record_batch(ctx, p, frames, outs, ctx->stream)) != BH_OK) return rc;
         CK(cudaStreamSynchronize(ctx->stream));
+        copies.waited = true;
         const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         return finish(ctx, n, stats, nullptr, true, secs);
     }
@@ -1035,6 +1061,7 @@ int bh_gpu_render_batch(bh_ctx* ctx, const bh_render_config* cfgs, int n, bh_xyz
         ctx->d2h += static_cast<long long>(m * sizeof(bh_xyz));
     }
     CK(cudaStreamSynchronize(ctx->stream));
+    copies.waited = true;
     const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return finish(ctx, n, stats, nullptr, true, secs);
 }
@@ -1097,6 +1124,7 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
         record = false;
     }
 
+    CopiesEnd copies(ctx);
     CK(cudaMemcpyAsync(ctx->adj_target.p, target, npx * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     ctx->h2d += static_cast<long long>(npx * sizeof(float));
     CK(cudaMemsetAsync(ctx->adj_xr.p, 0, n_slots * sizeof(double), ctx->stream));
@@ -1160,6 +1188,7 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
         CK(cudaMemcpyAsync(ray_Y, ctx->adj_Y.p, static_cast<size_t>(n_rays) * sizeof(double),
                            cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    copies.waited = true;
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]));
     const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -1381,11 +1410,13 @@ int bh_gpu_develop(bh_ctx* ctx, const bh_xyz* pixels, int width, int height, con
     const size_t npx = static_cast<size_t>(width) * height;
     int rc;
     if ((rc = ensure(ctx, ctx->pixels, npx * sizeof(bh_xyz))) != BH_OK) return rc;
+    double e = 0.0;
+    CopiesEnd copies(ctx);
     CK(cudaMemcpyAsync(ctx->pixels.p, pixels, npx * sizeof(bh_xyz), cudaMemcpyHostToDevice, ctx->stream));
     ctx->h2d += static_cast<long long>(npx * sizeof(bh_xyz));
     const DisplayJob job{static_cast<bh_xyz*>(ctx->pixels.p), width, height, out_rgb};
-    double e = 0.0;
     if ((rc = display_impl(ctx, d, &job, 1, &e)) != BH_OK) return rc;
+    copies.waited = true;
     if (exposure_used) *exposure_used = e;
     return BH_OK;
 }
@@ -1405,7 +1436,9 @@ int bh_gpu_render_rgb(bh_ctx* ctx, const bh_render_config* cfg, const bh_display
         return rc;
     const DisplayJob job{static_cast<bh_xyz*>(ctx->pixels.p), cfg->width, cfg->height, out_rgb};
     double e = 0.0;
+    CopiesEnd copies(ctx);
     if ((rc = display_impl(ctx, d, &job, 1, &e)) != BH_OK) return rc;
+    copies.waited = true;
     if (exposure_used) *exposure_used = e;
     const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return finish(ctx, 1, stats, nullptr, true, secs);
@@ -1432,7 +1465,9 @@ int bh_gpu_render_batch_rgb(bh_ctx* ctx, const bh_render_config* cfgs, int n, co
         jobs[i] = DisplayJob{static_cast<bh_xyz*>(ctx->pixels.p) + off, cfgs[i].width, cfgs[i].height, outs_rgb[i]};
         off += static_cast<size_t>(cfgs[i].width) * cfgs[i].height;
     }
+    CopiesEnd copies(ctx);
     if ((rc = display_impl(ctx, d, jobs.data(), n, used.data())) != BH_OK) return rc;
+    copies.waited = true;
     if (exposure_used) std::copy(used.begin(), used.end(), exposure_used);
     const double secs = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return finish(ctx, n, stats, nullptr, true, secs);
@@ -1468,6 +1503,7 @@ int bh_gpu_eval(bh_ctx* ctx, const bh_render_config* cfg, int what, const double
     if ((rc = ensure(ctx, ctx->eval_in, n_in * sizeof(double))) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->eval_out, n_out * sizeof(double))) != BH_OK) return rc;
     if (what == BH_EVAL_BLACKBODY && (rc = ensure_table(ctx)) != BH_OK) return rc;
+    CopiesEnd copies(ctx);
     CK(cudaMemcpyAsync(ctx->frames.p, &F, sizeof(FrameParams), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->eval_in.p, in, n_in * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     const FrameParams* dF = static_cast<const FrameParams*>(ctx->frames.p);
@@ -1477,6 +1513,7 @@ int bh_gpu_eval(bh_ctx* ctx, const bh_render_config* cfg, int what, const double
     else CK(launch_eval_shade(what == BH_EVAL_DISC_TEMPERATURE ? 0 : 1, dF, ctx->d_table, din, n, dout, ctx->stream));
     CK(cudaMemcpyAsync(out, dout, n_out * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    copies.waited = true;
     return BH_OK;
 }
 

@@ -36,6 +36,16 @@ def lib(tmp_path_factory):
     lib.bh_gpu_last_error.argtypes = [C.c_void_p]
     lib.bh_gpu_last_error.restype = C.c_char_p
     lib.bh_gpu_render_batch.argtypes = [C.c_void_p, CFG, C.c_int, C.POINTER(XYZ), C.POINTER(abi.bh_render_stats)]
+    S, U8, D = C.POINTER(abi.bh_render_stats), C.POINTER(C.c_uint8), C.POINTER(C.c_double)
+    lib.bh_gpu_render.argtypes = [C.c_void_p, CFG, XYZ, S]
+    lib.bh_gpu_trace_rays.argtypes = [C.c_void_p, CFG, C.POINTER(abi.bh_ray_result), S]
+    lib.bh_gpu_render_rgb.argtypes = [C.c_void_p, CFG, C.POINTER(abi.bh_display), U8, D, S]
+    lib.bh_gpu_render_batch_rgb.argtypes = [C.c_void_p, CFG, C.c_int, C.POINTER(abi.bh_display), C.POINTER(U8), D, S]
+    lib.bh_gpu_develop.argtypes = [C.c_void_p, XYZ, C.c_int, C.c_int, C.POINTER(abi.bh_display), U8, D]
+    lib.bh_gpu_adjoint_rays.argtypes = [C.c_void_p, CFG, C.POINTER(C.c_float), C.POINTER(abi.bh_grad4), D, D]
+    lib.bh_gpu_eval.argtypes = [C.c_void_p, CFG, C.c_int, D, C.c_longlong, D]
+    lib.bh_display_default.argtypes = [C.POINTER(abi.bh_display)]
+    lib.bh_display_default.restype = None
     lib.fake_fail.argtypes = [C.c_char_p, C.c_int]
     lib.fake_memory.argtypes = [C.c_longlong]
     lib.fake_memory_used.restype = C.c_longlong
@@ -103,3 +113,64 @@ def test_batch_without_what_the_row_bands_need(lib, ctx, missing):
     assert b.whole()
     assert lib.fake_count(b"cudaGraphLaunch") == (missing == "event")
     assert lib.fake_outstanding_copies() == 0
+
+
+def _calls(lib):
+    """Every entry that copies into the caller's memory, as a function of the context."""
+    d = abi.bh_display()
+    lib.bh_display_default(C.byref(d))
+    d.glare = 0.3
+    u8, dp = C.POINTER(C.c_uint8), C.POINTER(C.c_double)
+    small, tall, adj = _cfg(40, 30).to_c(), _cfg(60, 300).to_c(), _cfg(24, 20, abi.PRECISION_FP64).to_c()
+    px = np.zeros((300, 60, 3))
+    rays = np.zeros(40 * 30, dtype=abi.ray_result_dtype())
+    rgb = [np.zeros((30, 40, 3), np.uint8) for _ in range(9)]
+    developed = np.zeros((300, 60, 3), np.uint8)
+    film = (abi.bh_render_config * 9)(*[small] * 9)
+    films = (u8 * 9)(*[a.ctypes.data_as(u8) for a in rgb])
+    ex, grad, lum, rhs = np.zeros(9), np.zeros((480, 4)), np.zeros(480), np.ones((5, 8))
+    target, g = np.zeros((20, 24), np.float32), abi.bh_grad4()
+    early, graph = Batch(EARLY), Batch([(30, 40), (20, 25)])
+    p = lambda a, t: a.ctypes.data_as(t)  # noqa: E731
+    return {
+        "render": lambda h: lib.bh_gpu_render(h, C.byref(small), p(px, XYZ), None),
+        "render in row bands": lambda h: lib.bh_gpu_render(h, C.byref(tall), p(px, XYZ), None),
+        "trace_rays": lambda h: lib.bh_gpu_trace_rays(h, C.byref(small), p(rays, C.POINTER(abi.bh_ray_result)), None),
+        "batch": lambda h: early.render(lib, h),
+        "batch as a graph": lambda h: graph.render(lib, h),
+        "develop": lambda h: lib.bh_gpu_develop(h, p(px, XYZ), 60, 300, C.byref(d), p(developed, u8), p(ex, dp)),
+        "render_rgb": lambda h: lib.bh_gpu_render_rgb(h, C.byref(small), C.byref(d), p(rgb[0], u8), p(ex, dp), None),
+        "film": lambda h, alive=rgb: lib.bh_gpu_render_batch_rgb(h, film, 9, C.byref(d), films, p(ex, dp), None),
+        "adjoint": lambda h: lib.bh_gpu_adjoint_rays(h, C.byref(adj), p(target, C.POINTER(C.c_float)), C.byref(g),
+                                                     p(grad, dp), p(lum, dp)),
+        "eval": lambda h: lib.bh_gpu_eval(h, C.byref(small), abi.EVAL_RHS, p(rhs, dp), 5, p(rhs, dp)),
+    }
+
+
+FAILING = ["cudaMemcpyAsync", "cudaMemcpy2DAsync", "cudaMemsetAsync", "cudaEventRecord", "cudaStreamWaitEvent",
+           "cudaStreamSynchronize", "cuStreamWaitValue32", "cudaGraphLaunch", "launch_trace", "launch_shade",
+           "launch_reduce", "launch_display", "launch_adjoint"]
+
+
+@pytest.mark.parametrize("call", ["render", "render in row bands", "trace_rays", "batch", "batch as a graph", "develop",
+                                  "render_rgb", "film", "adjoint", "eval"])
+def test_no_copy_into_the_callers_memory_outlives_a_failed_call(lib, ctx, call):
+    """Whichever runtime call fails, an entry returns an error with nothing under way
+    into memory that the caller may free, and the next call is whole."""
+    h = ctx()
+    run = _calls(lib)[call]
+    assert run(h) == abi.OK, lib.bh_gpu_last_error(h)
+    assert lib.fake_outstanding_copies() == 0
+    failed = 0
+    for name in FAILING:
+        for nth in range(1, 200):
+            lib.fake_reset()
+            lib.fake_fail(name.encode(), nth)
+            rc = run(h)
+            assert lib.fake_outstanding_copies() == 0, (name, nth)
+            lib.fake_reset()
+            if rc == abi.OK:
+                break
+            failed += 1
+        assert run(h) == abi.OK, (name, lib.bh_gpu_last_error(h))
+    assert failed > 3
