@@ -352,8 +352,6 @@ reverse_kernel(const __grid_constant__ AdjointLaunch L) {
     }
 }
 
-__global__ void after_kernel() {}
-
 __global__ void __launch_bounds__(kReduceThreads)
 adjoint_reduce_kernel(const double* __restrict__ grad, const double* __restrict__ edge,
                       const unsigned char* __restrict__ high, long long n_rays, const bh_xyz* __restrict__ pixels,
@@ -409,9 +407,9 @@ cudaError_t launch_adjoint(const AdjointLaunch& L, cudaStream_t stream) {
         edge_candidates_kernel<<<(unsigned)((L.n_rays + 255) / 256), 256, 0, stream>>>(L);
         adjoint_select_kernel<<<(unsigned)((L.n_rays + 255) / 256), 256, 0, stream>>>(L);
         // The edge terms and the rays without records beside the recorded rays:
-        // long chains both, that share no output.  The empty kernel lets the
-        // few long chains be placed first; the other way round they wait for
-        // the persistent reverse_kernel's blocks to end (512^2 9.7 against 8.4 ms).
+        // long chains both, that share no output.  reverse_kernel waits until the
+        // few long chains have begun; the other way round they wait for its
+        // persistent blocks to end (512^2 9.7 against 8.4 ms).
         cudaError_t e;
         const bool side = L.traj && L.side_stream;
         cudaStream_t s2 = side ? L.side_stream : stream;
@@ -419,8 +417,10 @@ cudaError_t launch_adjoint(const AdjointLaunch& L, cudaStream_t stream) {
             if ((e = cudaEventRecord(L.fork_event, stream)) != cudaSuccess) return e;
             if ((e = cudaStreamWaitEvent(s2, L.fork_event, 0)) != cudaSuccess) return e;
         }
-        adjoint_kernel<<<L.grid, L.block, kAdjShared, stream>>>(L);
-        if (side) after_kernel<<<1, 32, 0, s2>>>();
+        if ((e = launch_started(adjoint_kernel, L.grid, L.block, kAdjShared, stream, side ? L.start_event : nullptr,
+                                L)) != cudaSuccess)
+            return e;
+        if (side && (e = cudaStreamWaitEvent(s2, L.start_event, 0)) != cudaSuccess) return e;
         if (L.traj) reverse_kernel<<<L.grid_reverse, kAdjBlock, kAdjShared, s2>>>(L);
         if (side) {
             if ((e = cudaEventRecord(L.join_event, s2)) != cudaSuccess) return e;

@@ -43,7 +43,7 @@ struct bh_ctx {
     cudaStream_t stream = nullptr;
     cudaStream_t abort_stream = nullptr;
     cudaStream_t side_stream = nullptr;     // the binary32 kernel's, beside the near-critical binary64 one
-    cudaEvent_t fork_event = nullptr, join_event = nullptr;
+    cudaEvent_t fork_event = nullptr, start_event = nullptr, join_event = nullptr;
     std::string err;
     // Launch shapes of the FP64 [0] and mixed [1] trace kernels (measured
     // best on the 1024^2 edge-on frame: the tight register caps, blocks of
@@ -396,6 +396,7 @@ int plan_launch(bh_ctx* ctx, std::vector<FrameParams>& frames, bh_xyz* d_pixels,
         tl.frames_side = static_cast<const FrameParams*>(ctx->frames.p) + n;
         tl.side_stream = ctx->side_stream;
         tl.fork_event = ctx->fork_event;
+        tl.start_event = ctx->start_event;
         tl.join_event = ctx->join_event;
         tl.sel_flag = static_cast<unsigned char*>(ctx->sel_flag.p);
         tl.sel_list = static_cast<int*>(ctx->sel_list.p);
@@ -834,6 +835,7 @@ int bh_gpu_create(int device, bh_ctx** out) {
     for (auto& ev : ctx->disp_done)
         if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) return bail(e);
     if ((e = cudaEventCreateWithFlags(&ctx->fork_event, cudaEventDisableTiming)) != cudaSuccess) return bail(e);
+    if ((e = cudaEventCreateWithFlags(&ctx->start_event, cudaEventDisableTiming)) != cudaSuccess) return bail(e);
     if ((e = cudaEventCreateWithFlags(&ctx->join_event, cudaEventDisableTiming)) != cudaSuccess) return bail(e);
     if ((e = cudaMalloc(&ctx->d_queue, sizeof(QueueState))) != cudaSuccess) return bail(e);
     if ((e = cudaMemset(ctx->d_queue, 0, sizeof(QueueState))) != cudaSuccess) return bail(e);
@@ -889,6 +891,7 @@ void bh_gpu_destroy(bh_ctx* ctx) {
     for (auto& ev : ctx->disp_done)
         if (ev) cudaEventDestroy(ev);
     if (ctx->fork_event) cudaEventDestroy(ctx->fork_event);
+    if (ctx->start_event) cudaEventDestroy(ctx->start_event);
     if (ctx->join_event) cudaEventDestroy(ctx->join_event);
     delete ctx;
 }
@@ -1165,6 +1168,7 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
                                                           (n_rays + block - 1) / block));
     L.side_stream = ctx->side_stream;
     L.fork_event = ctx->fork_event;
+    L.start_event = ctx->start_event;
     L.join_event = ctx->join_event;
     L.xing_r = static_cast<double*>(ctx->adj_xr.p);
     L.cand = static_cast<unsigned long long*>(ctx->adj_cand.p);

@@ -100,6 +100,26 @@ __host__ __device__ __forceinline__ long long pixel_index(int W, int H, int x, i
     return (long long)band * 4 * W + (long long)x * bh + (y - y0);
 }
 
+#if defined(__CUDACC__)
+// kernel<<<grid, block, shared, stream>>>(args); `started` (may be null)
+// fires once all of its blocks have begun.
+template <class... Params, class... Args>
+inline cudaError_t launch_started(void (*kernel)(Params...), int grid, int block, size_t shared, cudaStream_t stream,
+                                  cudaEvent_t started, const Args&... args) {
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeLaunchCompletionEvent;
+    attr.val.launchCompletionEvent.event = started;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3((unsigned)block);
+    c.dynamicSmemBytes = shared;
+    c.stream = stream;
+    c.attrs = &attr;
+    c.numAttrs = started ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, args...);
+}
+#endif
+
 // Index of the frame whose cumulative end exceeds `id` (ends ascending).
 __device__ __forceinline__ int find_frame(const long long* __restrict__ ends, int n, long long id) {
     int lo = 0, hi = n - 1;

@@ -51,9 +51,9 @@ struct TraceLaunch {
     int surfaces;                    // 1 when a frame of the launch has the Sun or a neutron star
     // Mixed precision: near-critical rays (escaping rays that circle close to
     // the photon shell) traced by a binary64 kernel of grid_side blocks of 64
-    // on `stream`, beside the binary32 kernel on side_stream (fork_event /
-    // join_event order it against `stream`), or before it on `stream` when
-    // side_stream is null.
+    // on `stream`, beside the binary32 kernel on side_stream (fork_event and
+    // join_event order it against `stream`, start_event fires once the binary64
+    // blocks have begun), or before it on `stream` when side_stream is null.
     int near_critical;
     int grid_side;
     const FrameParams* frames_side;  // device: the frames under binary64_treatment
@@ -61,7 +61,7 @@ struct TraceLaunch {
                                      // pass), or null: then both kernels test each ray themselves
     int* sel_list;                   // device, total_rays: the near-critical rays' ids
     cudaStream_t side_stream;
-    cudaEvent_t fork_event, join_event;
+    cudaEvent_t fork_event, start_event, join_event;
     // Row bands of a single-frame launch whose pixels are shaded and copied
     // out while the rest of the frame is traced: each finished ray adds one
     // to band_done[gid / rays_per_band]; after the last trace kernel every

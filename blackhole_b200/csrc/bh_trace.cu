@@ -1489,7 +1489,8 @@ __global__ void eval_rhs_kernel(const FrameParams* __restrict__ Fp, const double
 }
 
 template <class P, int MAXREG, bool JET, int SURF, bool RESUME = false>
-cudaError_t launch_t(const TraceLaunch& L, int grid, int block, cudaStream_t s, int select = 0) {
+cudaError_t launch_t(const TraceLaunch& L, int grid, int block, cudaStream_t s, int select = 0,
+                     cudaEvent_t started = nullptr) {
     TraceArgs A;
     A.frames = (select == 1) ? L.frames_side : L.frames;
     A.sel_flag = select ? L.sel_flag : nullptr;
@@ -1520,12 +1521,8 @@ cudaError_t launch_t(const TraceLaunch& L, int grid, int block, cudaStream_t s, 
     A.disc_end = L.disc_end;
     A.band_done = L.band_done;
     A.rays_per_band = L.rays_per_band > 0 ? L.rays_per_band : 1;
-    trace_kernel<P, MAXREG, JET, SURF, RESUME><<<grid, block, 0, s>>>(A);
-    return cudaGetLastError();
+    return launch_started(trace_kernel<P, MAXREG, JET, SURF, RESUME>, grid, block, 0, s, started, A);
 }
-
-// Does nothing (it orders two launches, see launch_trace_t).
-__global__ void gate_kernel() {}
 
 // Raises each band counter to its band's ray count (after the trace kernels).
 __global__ void band_release_kernel(unsigned int* band_done, int nbands, long long total, long long per_band) {
@@ -1675,7 +1672,7 @@ template <bool JET, int SURF>
 cudaError_t launch_trace_t(const TraceLaunch& L, cudaStream_t stream) {
     if (L.precision == BH_PRECISION_MIXED) {
         cudaError_t e;
-        const bool side = L.near_critical && L.side_stream && L.fork_event && L.join_event;
+        const bool side = L.near_critical && L.side_stream && L.fork_event && L.start_event && L.join_event;
         if (L.near_critical) {
             // The near-critical rays in binary64 (the binary64 path's
             // arithmetic) beside the binary32 launch (the two share no data
@@ -1691,8 +1688,8 @@ cudaError_t launch_trace_t(const TraceLaunch& L, cudaStream_t stream) {
                 if ((e = cudaGetLastError()) != cudaSuccess) return e;
             }
         }
-        // Beside: the binary32 kernel on the side stream from the fork on.  The
-        // binary64 kernel's grid could fill the GPU, a lane per listed ray in
+        // Beside: the binary32 kernel on the side stream from the binary64
+        // kernel's start on.  That kernel's grid could fill the GPU, a lane per listed ray in
         // flight; its blocks that find no ray left end at once, and the
         // binary32 kernel's blocks take the slots they leave.  So the long
         // serial chains start first and end in the shadow of the binary32
@@ -1708,17 +1705,16 @@ cudaError_t launch_trace_t(const TraceLaunch& L, cudaStream_t stream) {
             if ((e = cudaEventRecord(L.fork_event, stream)) != cudaSuccess) return e;
             if ((e = cudaStreamWaitEvent(L.side_stream, L.fork_event, 0)) != cudaSuccess) return e;
         }
-        if (L.near_critical &&
-            (e = launch_t<Fp64, kRegFp64Wide, JET, SURF>(L, L.grid_side, kSideBlock, stream, 1)) != cudaSuccess)
+        if (L.near_critical && (e = launch_t<Fp64, kRegFp64Wide, JET, SURF>(L, L.grid_side, kSideBlock, stream, 1,
+                                                                            side ? L.start_event : nullptr)) !=
+                                   cudaSuccess)
             return e;
-        if (side) {
-            // An empty kernel before the binary32 one: both kernels are ready
-            // at the fork, and the binary64 blocks are to be placed first (the
-            // other way round they wait for the persistent binary32 blocks to
-            // end: 3.3 against 2.7 ms per 1024^2 frame).
-            gate_kernel<<<1, 32, 0, s32>>>();
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        }
+        // The binary32 kernel waits until all binary64 blocks have begun: the
+        // other way round they wait for the persistent binary32 blocks to end.
+        // An empty kernel before the binary32 one made this order likely and
+        // not certain: on a process's first context and stream the 1024^2 frame
+        // took 3.2 ms, on the others 2.6; now 2.6 on all.
+        if (side && (e = cudaStreamWaitEvent(L.side_stream, L.start_event, 0)) != cudaSuccess) return e;
         e = L.reg_variant ? launch_t<Mixed, kRegMixedWide, JET, SURF>(L, L.grid, L.block_size, s32, sel)
                           : launch_t<Mixed, kRegMixed, JET, SURF>(L, L.grid, L.block_size, s32, sel);
         if (e != cudaSuccess) return e;
