@@ -142,7 +142,8 @@ __global__ void __launch_bounds__(256) adjoint_select_kernel(const __grid_consta
             double d[3], gY[3];
             if (adj::escape_direction_value(y6, -h.y[4], h.y[7], L.frame.a, d)) {
                 Y = adj::sky_luminance(L.sky, L.frame, d, gY);
-                listed = w != 0.0 && (gY[0] != 0.0 || gY[1] != 0.0 || gY[2] != 0.0);
+                // (a weight that is not finite has a gradient on any sky)
+                listed = w != 0.0 && (!isfinite(w) || gY[0] != 0.0 || gY[1] != 0.0 || gY[2] != 0.0);
             }
         }
         L.high_order[o] = high ? 1 : 0;

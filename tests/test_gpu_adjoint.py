@@ -382,3 +382,27 @@ def test_stopped_adjoint_is_an_error_and_the_next_is_whole(renderer, c4):
     finally:
         renderer.set_step_budget(0)
     assert renderer.adjoint(cfg, target)["d_spin"] == g["d_spin"]
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_a_target_that_is_not_finite_shows_in_the_gradient(renderer, bad):
+    """A pixel without a finite target has no finite weight: the loss is not finite, and
+    neither is the gradient of a ray of that pixel that met the sky, uniform or not.  The
+    other rays keep theirs."""
+    lib = _check_lib()
+    cfg = _scene(24, 0.7, 50.0)
+    cfg.stars_enabled, cfg.sky_mode = False, abi.SKY_UNIFORM
+    target = np.zeros((24, 24), dtype=np.float32)
+    _, whole, _ = renderer.adjoint(cfg, target, per_ray=True)
+    what = renderer.trace_rays(cfg)["what"]
+    idx = int(np.flatnonzero(what == abi.HIT_SKY)[5])
+    assert not whole[idx].any()                      # a uniform sky: no gradient of its own
+    target.reshape(-1)[idx] = bad
+    g, per_ray, _ = renderer.adjoint(cfg, target, per_ray=True)
+    out = np.zeros(9)
+    rid = int(np.flatnonzero(np.asarray(abi.work_order(24, 24, 1)) == idx)[0])
+    assert lib.bhx_ray(C.byref(cfg.to_c()), rid, -bad, 0, 0, out.ctypes.data_as(C.POINTER(C.c_double))) == abi.OK
+    assert np.isnan(out[1:3]).all() and np.isnan(per_ray[idx, :2]).all()
+    assert not np.isfinite(g["loss"]) and np.isnan(g["d_spin"]) and np.isnan(g["d_inclination"])
+    rest = np.arange(24 * 24) != idx
+    assert np.array_equal(per_ray[rest], whole[rest])
