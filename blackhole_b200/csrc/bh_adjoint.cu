@@ -13,8 +13,10 @@
 // adjoint_kernel: the edge terms, and the listed rays without records (more
 // steps than the record holds, or a frame too large for one), which are
 // integrated again.  A lane that does so owns `checkpoint_slots` stored states
-// in global memory, interleaved over the warp, for the job it is working on
-// (bh_adjoint.cuh has the per-ray algorithm).
+// (45 KB) in global memory, interleaved over the warp, for the job it is
+// working on (bh_adjoint.cuh has the per-ray algorithm).  Beside a record of 512
+// steps per ray few jobs need them (15 rays at 512^2), so an eighth of the
+// warps own states; every warp does elsewhere.
 //
 // In both a warp takes 32 jobs at a time from a global atomic counter.  A
 // ray's loss weight is 2 (Y_pixel - target) / S^2 for Loss = sum over pixels
@@ -96,8 +98,9 @@ __global__ void __launch_bounds__(256) edge_candidates_kernel(const __grid_const
         }
         const int m = adj::edge_mask(L.frame, rc, dmax);
         if (m) {
-            const unsigned long long at = atomicAdd(&L.counters[6], 1ull);
-            L.cand[at] = ((unsigned long long)(2 * id + j) << 2) | (unsigned long long)m;
+            const unsigned long long c = ((unsigned long long)(2 * id + j) << 2) | (unsigned long long)m;
+            if (L.traj && L.xing_step[2 * id + j] <= L.traj_cap) L.cand[atomicAdd(&L.counters[6], 1ull)] = c;
+            else L.cand[2 * L.n_rays - 1 - (long long)atomicAdd(&L.counters[13], 1ull)] = c;
         }
     }
 }
@@ -227,43 +230,50 @@ __device__ __noinline__ long long edge_recorded(const AdjointLaunch& L, long lon
     return work;
 }
 
-// One queue of jobs: first the listed rays without recorded steps (a forward
-// pass and a reverse sweep: the longest jobs), then the edge candidates.  Results go to per-ray and
-// per-crossing slots, so the sums do not depend on which lane took which job.
+// Two queues of jobs.  First the listed rays and the edge candidates without
+// recorded steps (a forward pass and a reverse sweep: the longest jobs), for the
+// warps that own stored states; then, for every warp, the candidates with
+// recorded steps.  Results go to per-ray and per-crossing slots, so the sums do
+// not depend on which lane took which job.
 __global__ void __launch_bounds__(kAdjBlock, kAdjBlocksPerSm) adjoint_kernel(const __grid_constant__ AdjointLaunch L) {
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int slots = L.X.checkpoint_slots;
     double* ck = L.ckpt + warp * slots * adj::kCkWords * 32 + lane;
     const int SS = L.frame.S * L.frame.S;
-    // each part starts on a warp of its own
+    // rays and candidates start on a warp of their own
     const unsigned long long n_rays = L.counters[11], first_cand = (n_rays + 31) & ~31ull,
-                             n_jobs = first_cand + L.counters[6];
+                             n_stored = first_cand + L.counters[13], n_recorded = L.counters[6];
     unsigned long long replay = 0, max_int = 0, edge_steps = 0, edge_cells = 0;
+    bool stored = warp < L.ckpt_warps;       // which queue the warp takes from
     for (;;) {
         unsigned long long job = 0;
-        if (lane == 0) job = atomicAdd(&L.counters[0], 32ull);
+        if (lane == 0) job = atomicAdd(&L.counters[stored ? 14 : 0], 32ull);
         job = __shfl_sync(kFull, job, 0);
-        if (job >= n_jobs) break;
+        if (job >= (stored ? n_stored : n_recorded)) {
+            if (!stored) break;
+            stored = false;
+            continue;
+        }
         job += lane;
         int px, py, k;
-        if (job >= first_cand && job < n_jobs) {
-            const unsigned long long c = L.cand[job - first_cand];
+        if (stored ? (job >= first_cand && job < n_stored) : job < n_recorded) {
+            const unsigned long long c = L.cand[stored ? 2 * L.n_rays - 1 - (long long)(job - first_cand)
+                                                       : (long long)job];
             const long long xs = (long long)(c >> 2);     // 2 * ray + crossing
             const long long pix = ray_pixel(L, xs >> 1, &px, &py, &k);
             const double w = 2.0 * (L.pixels[pix].y - (double)L.target[pix]);
             double out[3];
             int n_cells = 0;
-            const bool recorded = L.traj && L.xing_step[xs] <= L.traj_cap;
             edge_steps += (unsigned long long)(
-                recorded ? edge_recorded(L, xs >> 1, px, py, k, (int)(xs & 1), (int)(c & 3ull), w, out, &n_cells)
-                         : adj::edge_sample(L.frame, L.X, L.sky, px, py, k, (int)(xs & 1) + 1, (int)(c & 3ull), w, ck,
-                                            slots, 32, out, &n_cells));
+                stored ? adj::edge_sample(L.frame, L.X, L.sky, px, py, k, (int)(xs & 1) + 1, (int)(c & 3ull), w, ck,
+                                          slots, 32, out, &n_cells)
+                       : edge_recorded(L, xs >> 1, px, py, k, (int)(xs & 1), (int)(c & 3ull), w, out, &n_cells));
             edge_cells += (unsigned long long)n_cells;
             L.edge_out[3 * xs] = out[0];
             L.edge_out[3 * xs + 1] = out[1];
             L.edge_out[3 * xs + 2] = out[2];
-        } else if (job < n_rays) {
+        } else if (stored && job < n_rays) {
             const long long id = L.rays[L.n_rays - 1 - (long long)job];
             const long long pix = ray_pixel(L, id, &px, &py, &k);
             const double w = 2.0 * (L.pixels[pix].y - (double)L.target[pix]) / (double)SS;

@@ -51,7 +51,9 @@ struct AdjointLaunch {
     const float* target;             // target luminance, row-major W x H (device)
     double* ray_grad;                // 4 per ray, pixel-major then sample (device)
     double* ray_Y;                   // luminance per ray in the same order, or nullptr
-    double* ckpt;                    // grid * block * checkpoint_slots * kAdjSlotWords doubles
+    double* ckpt;                    // ckpt_warps * 32 * checkpoint_slots * kAdjSlotWords doubles: the stored
+                                     // states of the first ckpt_warps warps
+    int ckpt_warps;
     const HitRecord* hits;           // the render's hit records, work order (device)
     // The rays that have a gradient (work order ids; n_rays entries): those whose
     // steps the render recorded from the front, the others from the back.
@@ -64,18 +66,20 @@ struct AdjointLaunch {
     // The edge pass: per crossing slot (2 per ray, slot = 2 * ray + crossing,
     // rays in work order) the radius of the ray's first two equatorial
     // crossings as the render found them (0: none; zeroed before the
-    // render; the second one's sign is set when a third followed), the candidate list ((slot << 2) | kEdge* bits) and 3 edge
-    // contributions per slot.
+    // render; the second one's sign is set when a third followed), the
+    // candidate list ((slot << 2) | kEdge* bits; those in recorded steps from the
+    // front, the others from the back) and 3 edge contributions per slot.
     double* xing_r;
     unsigned long long* cand;
     double* edge_out;
     // 1 for a ray whose event came after its third or later equatorial
     // crossing (an image of order three or higher), in ray_grad order
     unsigned char* high_order;
-    // next job, accepted, replayed, disc rays, sky rays, max interval, edge
-    // candidates, edge-pass steps, edge cells, high-order rays, rays with a gradient and recorded steps, other rays with a
-    // gradient, next recorded ray and recorded steps, other rays with a
-    // gradient, next job of the recorded rays
+    // By index: 0 next recorded candidate, 1 accepted steps, 2 replayed steps, 3 disc
+    // rays, 4 sky rays, 5 largest interval, 6 recorded candidates, 7 steps of the
+    // edge pass, 8 edge cells, 9 high-order rays, 10 recorded rays with a
+    // gradient, 11 other rays with a gradient, 12 next recorded ray, 13 other
+    // candidates, 14 next job without records.
     unsigned long long* counters;
     // loss; the four per-ray gradient sums (spin and inclination over the
     // rays of image order one and two); the three edge sums; the spin and
@@ -84,18 +88,19 @@ struct AdjointLaunch {
     long long n_rays;
     int grid, block;
     int grid_reverse;                // blocks of the kernel over the recorded rays
-    cudaStream_t side_stream;        // the edge terms and the rays without records run here, beside it
+    cudaStream_t side_stream;        // that kernel runs here, beside the edge terms and the rays without records
     cudaEvent_t fork_event, start_event, join_event;
 };
 
-constexpr int kAdjCounters = 13;
+constexpr int kAdjCounters = 15;
 constexpr int kAdjSlotWords = 11;         // doubles per stored state
 constexpr int kAdjSums = 10;
 
 // Enqueues the edge pass's candidate selection over the sample grid, the
-// adjoint kernel (edge terms, then the rays) and the deterministic reduction
-// of the per-ray gradients, the edge contributions and the loss; `counters`
-// and `edge_out` must be zeroed before.
+// adjoint kernel (rays without records, then edge terms), the sweeps over the
+// recorded rays beside it and the deterministic reduction of the per-ray
+// gradients, the edge contributions and the loss; `counters` and `edge_out`
+// must be zeroed before.
 cudaError_t launch_adjoint(const AdjointLaunch& L, cudaStream_t stream);
 // Threads per block of the adjoint kernel, and its resident blocks per SM at
 // `block_size` threads.

@@ -153,17 +153,51 @@ struct CopiesEnd {
     ~CopiesEnd();
 };
 
+void release(DevBuf& b) {
+    if (b.p) cudaFree(b.p);
+    b.p = nullptr;
+    b.cap = 0;
+}
+
+// At least `bytes` in buffer b.  Where the device has no room, what an earlier
+// gradient left behind (its step record and stored states, gigabytes that every
+// gradient sizes anew) is given back first.
 int ensure(bh_ctx* ctx, DevBuf& b, size_t bytes) {
     if (bytes <= b.cap) return BH_OK;
-    if (b.p) {
-        cudaFree(b.p);
-        b.p = nullptr;
-        b.cap = 0;
-    }
+    release(b);
     const size_t want = std::max<size_t>(bytes, 256);
-    CK(cudaMalloc(&b.p, want));
+    cudaError_t e = cudaMalloc(&b.p, want);
+    if (e == cudaErrorMemoryAllocation && (ctx->adj_traj.p || ctx->adj_ckpt.p)) {
+        cudaGetLastError();
+        release(ctx->adj_traj);
+        release(ctx->adj_ckpt);
+        e = cudaMalloc(&b.p, want);
+    }
+    if (e != cudaSuccess) {
+        b.p = nullptr;
+        return cuda_fail(ctx, e, "cudaMalloc(&b.p, want)");
+    }
     b.cap = want;
     return BH_OK;
+}
+
+// The same for memory a call can do without: no error is kept, and nothing is
+// given back for it.  At most a quarter of the device memory that is free.
+bool ensure_optional(DevBuf& b, size_t bytes) {
+    if (bytes <= b.cap) return true;
+    size_t free_bytes = 0, all_bytes = 0;
+    if (cudaMemGetInfo(&free_bytes, &all_bytes) != cudaSuccess || bytes > (free_bytes + b.cap) / 4) {
+        cudaGetLastError();
+        return false;
+    }
+    release(b);
+    if (cudaMalloc(&b.p, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        b.p = nullptr;
+        return false;
+    }
+    b.cap = bytes;
+    return true;
 }
 
 int check_cfg_header(bh_ctx* ctx, const bh_render_config* cfg) {
@@ -1093,14 +1127,12 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
     if (bps < 1) bps = 1;
     const size_t npx = static_cast<size_t>(c.width) * c.height;
     const long long n_rays = frames[0].n_rays;
-    // no more blocks than jobs (a ray, and an edge term for each of its two crossings)
-    const int grid = static_cast<int>(std::min<long long>(ctx->sm_count * bps, (3 * n_rays + block - 1) / block));
     if ((rc = ensure(ctx, ctx->pixels, npx * sizeof(bh_xyz))) != BH_OK) return rc;
+    Plan p;
+    if ((rc = plan_launch(ctx, frames, static_cast<bh_xyz*>(ctx->pixels.p), nullptr, false, p)) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->adj_target, npx * sizeof(float))) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->adj_grad, static_cast<size_t>(n_rays) * 4 * sizeof(double))) != BH_OK) return rc;
     if (ray_Y && (rc = ensure(ctx, ctx->adj_Y, static_cast<size_t>(n_rays) * sizeof(double))) != BH_OK) return rc;
-    const size_t ck_bytes = static_cast<size_t>(grid) * block * X.checkpoint_slots * kAdjSlotWords * sizeof(double);
-    if ((rc = ensure(ctx, ctx->adj_ckpt, ck_bytes)) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->adj_counters, kAdjCounters * sizeof(unsigned long long))) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->adj_sums, kAdjSums * sizeof(double))) != BH_OK) return rc;
     const size_t n_slots = static_cast<size_t>(n_rays) * 2;     // two equatorial crossings per ray
@@ -1110,22 +1142,27 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
     if ((rc = ensure(ctx, ctx->adj_high, static_cast<size_t>(n_rays))) != BH_OK) return rc;
     if ((rc = ensure(ctx, ctx->adj_rays, static_cast<size_t>(n_rays) * sizeof(int))) != BH_OK) return rc;
 
-    // The render records its rays' steps where they fit; a ray with more steps
-    // than the cap, and every ray of a larger frame, is integrated again.
+    // After everything the call cannot do without: the render records its rays'
+    // steps where they fit; a ray with more steps than the cap, and every ray of a
+    // larger frame, is integrated again.
     const size_t step_bytes = static_cast<size_t>(n_rays) * kTrajWords * sizeof(double);
     const int traj_cap = static_cast<int>(std::min<size_t>(kTrajCap, kTrajMostBytes / step_bytes));
-    bool record = traj_cap >= kTrajCapLeast;
-    if (record && step_bytes * traj_cap > ctx->adj_traj.cap) {
-        size_t free_bytes = 0, all_bytes = 0;
-        CK(cudaMemGetInfo(&free_bytes, &all_bytes));
-        record = step_bytes * traj_cap <= (free_bytes + ctx->adj_traj.cap) / 4;
-    }
-    if (record && (ensure(ctx, ctx->adj_traj, step_bytes * traj_cap) != BH_OK ||
-                   ensure(ctx, ctx->adj_xstep, n_slots * sizeof(int)) != BH_OK ||
-                   ensure(ctx, ctx->adj_end, static_cast<size_t>(n_rays) * kEndWords * sizeof(double)) != BH_OK)) {
-        cudaGetLastError();            // no room: without records
-        record = false;
-    }
+    const bool record = traj_cap >= kTrajCapLeast && ensure_optional(ctx->adj_xstep, n_slots * sizeof(int)) &&
+                        ensure_optional(ctx->adj_end, static_cast<size_t>(n_rays) * kEndWords * sizeof(double)) &&
+                        ensure_optional(ctx->adj_traj, step_bytes * traj_cap);
+    // no more blocks than jobs (a ray, and an edge term for each of its two crossings)
+    int grid = static_cast<int>(std::min<long long>(ctx->sm_count * bps, (3 * n_rays + block - 1) / block));
+    // The stored states of the rays that are integrated again: for every warp,
+    // or beside a full record for an eighth of them (1.7 and 0.2 GB on 148 SMs); for
+    // fewer where the device has no room for those, down to one block's.
+    const int block_warps = block / 32;
+    const size_t warp_bytes = static_cast<size_t>(32) * X.checkpoint_slots * kAdjSlotWords * sizeof(double);
+    int stored = (record && traj_cap == kTrajCap) ? (grid + 7) / 8 : grid;
+    auto room = [&] { return ensure_optional(ctx->adj_ckpt, stored * block_warps * warp_bytes); };
+    if (!record && !room()) release(ctx->adj_traj);      // an earlier call's record
+    while (stored > 1 && !room()) stored /= 2;
+    if (stored <= 1 && (rc = ensure(ctx, ctx->adj_ckpt, block_warps * warp_bytes)) != BH_OK) return rc;
+    if (!record) grid = stored;
 
     CopiesEnd copies(ctx);
     CK(cudaMemcpyAsync(ctx->adj_target.p, target, npx * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
@@ -1134,9 +1171,6 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     {
         // the render, recording each ray's first two equatorial crossings
-        Plan p;
-        if ((rc = plan_launch(ctx, frames, static_cast<bh_xyz*>(ctx->pixels.p), nullptr, false, p)) != BH_OK)
-            return rc;
         p.tl.xing = static_cast<double*>(ctx->adj_xr.p);
         p.tl.traj = record ? static_cast<double*>(ctx->adj_traj.p) : nullptr;
         p.tl.traj_cap = traj_cap;
@@ -1157,6 +1191,7 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
     L.ray_grad = static_cast<double*>(ctx->adj_grad.p);
     L.ray_Y = ray_Y ? static_cast<double*>(ctx->adj_Y.p) : nullptr;
     L.ckpt = static_cast<double*>(ctx->adj_ckpt.p);
+    L.ckpt_warps = stored * block_warps;
     L.hits = static_cast<const HitRecord*>(ctx->hits.p);
     L.rays = static_cast<int*>(ctx->adj_rays.p);
     L.traj = record ? static_cast<const double*>(ctx->adj_traj.p) : nullptr;
@@ -1205,7 +1240,7 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
     out->d_r_out = sums[4] + sums[5];
     out->edge_spin = sums[6];
     out->edge_inclination = sums[7];
-    out->edge_candidates = static_cast<long long>(cnt[6]);
+    out->edge_candidates = static_cast<long long>(cnt[6] + cnt[13]);
     out->edge_steps = static_cast<long long>(cnt[7]);
     out->edge_cells = static_cast<long long>(cnt[8]);
     out->held_spin = sums[8];

@@ -434,9 +434,7 @@ typedef struct bh_grad4 {
    spin, the camera inclination, the Eddington ratio and the disc's outer
    radius.  The frame is rendered in binary64 (whatever cfg->precision says);
    the gradient is the discrete adjoint of that render: each ray's accepted
-   DP5 step sequence is taken backwards from its stored states (one per
-   accepted step, 512 per ray in flight; for longer rays every second, fourth
-   .. state is kept and the steps between are replayed), with
+   DP5 step sequence is taken backwards, with
    the step sizes and each ray's termination class held fixed.  To that the
    edge term is added: the motion of the disc's outer edge (r_out) and inner
    edge (the ISCO) across the image, which a point-sampled frame shows only
@@ -455,7 +453,19 @@ typedef struct bh_grad4 {
    part of the cell, so their per-ray spin and inclination terms are
    reported apart (held_spin, held_inclination) and their edges are left
    out.  Scenes with the Sun, a neutron star, a hot spot or a jet return
-   BH_ERR_UNSUPPORTED.  No counterpart in the reference. */
+   BH_ERR_UNSUPPORTED.  No counterpart in the reference.
+
+   Device memory.  The render records its rays' steps, 56 bytes each, for up to
+   512 steps a ray and 8 GiB in all (512 x 512 rays: 7.5 GB; frames of more than
+   684,784 rays: none), if that is no more than a quarter of the free memory.
+   A ray without a record, or with more steps than it holds, is integrated
+   again with 512 stored states (for longer rays every second, fourth .. state is
+   kept and the steps between are replayed): 1.7 GB without a record, 0.2 GB beside a
+   full one, less with fewer rays at a time where there is no room.  Both stay
+   with the context for the next gradient; any other call of the context that
+   finds no room gives them back.  So the free memory decides between two
+   ways to the same sums, which differ in rounding: by 1e-12 of a ray's gradient
+   as a rule, by up to 1e-6 for a ray that circles the photon shell. */
 int  bh_gpu_adjoint(bh_ctx* ctx, const bh_render_config* cfg, const float* target, bh_grad4* out);
 
 /* bh_gpu_adjoint plus, when not NULL, each ray's gradient contribution

@@ -14,6 +14,7 @@
 // cuStreamWaitValue32 away.
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 
 #include <cstdint>
 #include <cstdio>
@@ -147,8 +148,9 @@ cudaError_t cudaGetDriverEntryPoint(const char*, void** fn, unsigned long long, 
 
 cudaError_t cudaMalloc(void** p, size_t n) {
     if (fails("cudaMalloc") || g_used + n > g_limit) return cudaErrorMemoryAllocation;
-    *p = std::calloc(n, 1);
-    if (!*p) return cudaErrorMemoryAllocation;
+    // zero pages that take no memory until they are written
+    *p = mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
+    if (*p == MAP_FAILED) return cudaErrorMemoryAllocation;
     g_blocks[*p] = n;
     g_used += n;
     return cudaSuccess;
@@ -157,8 +159,8 @@ cudaError_t cudaFree(void* p) {
     if (!p) return cudaSuccess;
     for (Stream* s : g_streams) run_to(s, s->ops.size());      // cudaFree waits for the device
     g_used -= g_blocks[p];
+    munmap(p, g_blocks[p]);
     g_blocks.erase(p);
-    std::free(p);
     return cudaSuccess;
 }
 cudaError_t cudaMemGetInfo(size_t* free_bytes, size_t* total) {

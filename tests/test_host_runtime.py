@@ -174,3 +174,48 @@ def test_no_copy_into_the_callers_memory_outlives_a_failed_call(lib, ctx, call):
             failed += 1
         assert run(h) == abi.OK, (name, lib.bh_gpu_last_error(h))
     assert failed > 3
+
+
+MB = 1 << 20
+
+
+def _gradient(lib, h, n):
+    """bh_gpu_adjoint_rays of an n x n frame."""
+    c, g = _cfg(n, n, abi.PRECISION_FP64).to_c(), abi.bh_grad4()
+    target, d = np.zeros(n * n, np.float32), np.zeros(4 * n * n)
+    dp = d.ctypes.data_as(C.POINTER(C.c_double))
+    return lib.bh_gpu_adjoint_rays(h, C.byref(c), target.ctypes.data_as(C.POINTER(C.c_float)), C.byref(g), dp, None)
+
+
+def test_a_gradient_needs_no_more_than_its_rays(lib, ctx):
+    """Records and stored states shrink to the memory there is: a gradient of 128^2 rays
+    needs about 200 bytes a ray, whatever it takes on an empty device."""
+    h = ctx()
+    assert _gradient(lib, h, 8) == abi.OK            # the sky's tables
+    lib.fake_memory(lib.fake_memory_used() + 16 * MB)
+    assert _gradient(lib, h, 128) == abi.OK, lib.bh_gpu_last_error(h)
+
+
+def test_what_a_gradient_keeps_is_given_back(lib, ctx):
+    """A context that holds a gradient's record (0.94 GB at 128^2 x 512 steps) takes it
+    back before another call fails for want of memory."""
+    h = ctx()
+    assert _gradient(lib, h, 128) == abi.OK
+    held = lib.fake_memory_used()
+    assert held > 400 * MB
+    lib.fake_memory(held + MB)
+    b = Batch([(600, 700), (500, 400)], abi.PRECISION_FP64)
+    assert b.render(lib, h) == abi.OK, lib.bh_gpu_last_error(h)
+    assert b.whole()
+    lib.fake_memory(-1)
+    assert _gradient(lib, h, 128) == abi.OK
+
+
+def test_memory_of_a_gradient(lib, ctx):
+    """The figures of bh_gpu.h: 7.5 GB of records and 0.2 GB of stored states at 512^2."""
+    h = ctx()
+    assert _gradient(lib, h, 8) == abi.OK
+    before = lib.fake_memory_used()
+    assert _gradient(lib, h, 512) == abi.OK
+    used = (lib.fake_memory_used() - before) / 1e9
+    assert 7.5 < used < 7.9
