@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../bh_adjoint.cuh"
+#include "../bh_critical.cuh"
 #include "../bh_scene.h"
 
 using namespace bhg;
@@ -204,6 +205,37 @@ int bhx_edge_mask(const bh_render_config* cfg, double rc, double dmax, int* mask
     const int rc2 = prepare(cfg, F, X, sd);
     if (rc2 != BH_OK) return rc2;
     *mask = adj::edge_mask(F, rc, dmax);
+    return BH_OK;
+}
+
+// The near-critical class of sample k[i] of n pixels: quick[i] as the binary32 test
+// decides it (-1: it does not), rn[i] the value the class is a band of, R_min / r*^4
+// (+1 where there is no near miss), from the ray's photon in long double.
+int bhx_near_critical(const bh_render_config* cfg, int n, const int* px, const int* py, const int* k, int* quick,
+                      double* rn) {
+    std::lock_guard<std::mutex> lock(g_mu);
+    FrameParams F;
+    AdjointFrame X;
+    SkyData sd;
+    const int rc = prepare(cfg, F, X, sd);
+    if (rc != BH_OK) return rc;
+    using Q = long double;
+    for (int i = 0; i < n; ++i) {
+        const long long id = pixel_index(F.width, F.height, px[i], py[i]) * F.S * F.S + k[i];
+        quick[i] = near_critical_quick(F, id);
+        double y[6], E, Lz, dy[2][6], dE[2], dLz[2];
+        adj::ray_start(F, X, id, y, &E, &Lz, dy, dE, dLz);
+        rn[i] = 1.0;
+        if (!(E != 0.0) || !(y[4] < 0.0)) continue;
+        const Q a = F.a, b = Q(Lz) / E, pth = Q(y[5]) / E;
+        const Q q = pth * pth + Q(F.cam_cs2) * (b * b / Q(F.cam_sn2) - a * a);
+        const Q c2 = a * a - b * b - q, c1 = 2 * (q + (b - a) * (b - a)), c0 = -a * a * q;
+        if (!(c2 < 0)) continue;
+        Q r = std::sqrt(-c2);
+        for (int it = 0; it < 200; ++it) r -= (4 * r * r * r + 2 * c2 * r + c1) / (12 * r * r + 2 * c2);
+        if (!(r > F.r_plus) || !(r < y[1])) continue;
+        rn[i] = static_cast<double>((((r * r + c2) * r + c1) * r + c0) / (r * r * r * r));
+    }
     return BH_OK;
 }
 
