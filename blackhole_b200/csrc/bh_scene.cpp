@@ -303,7 +303,6 @@ void set_binary32_copies(FrameParams& F) {
     F.f_r_stop = static_cast<float>(F.r_stop);
     F.f_r_escape = static_cast<float>(F.r_escape);
     F.f_r_promote = static_cast<float>(F.r_promote);
-    F.f_pad = 0.f;
 }
 }  // namespace
 
@@ -515,6 +514,7 @@ int make_frame(const bh_render_config& c, FrameParams& F, std::string& err) {
     for (int i = 0; i < 3; ++i) F.sun_c[i] = c.sun.centre[i];
     F.sun_R = c.sun.radius;
     F.sun_R2 = c.sun.radius * c.sun.radius;
+    F.f_sun_margin = static_cast<float>(1e-4 + 2.4e-7 * std::fabs(c.cam.phi));
     F.sun_T_eff = c.sun.T_eff;
     F.sun_redshift_div = 1.0 + kG * kMsun / (kRsun * kC * kC);   // scene.h:239-240
     F.ns_enabled = c.star.enabled ? 1 : 0;

@@ -206,7 +206,8 @@ __device__ __forceinline__ void cartesian32(const Lane<P>& L, float r, float sn,
 // Whether a step between two points may meet render.cpp's condition for probing
 // it against the Sun (its start within the step's length and 1.5 radii of the
 // centre); false only where it certainly does not: the margin is a hundred
-// times binary32's error in these positions.  Taken every step, the six sin/cos
+// times binary32's error in these positions, with four times the rounding of the
+// camera's azimuth, which may be any number.  Taken every step, the six sin/cos
 // and three square roots of the binary64 test were a quarter of the kernel's
 // time (333 x 217 pixels of 4 samples, binary64, 5.7 -> 4.3 ms per frame).
 __device__ __forceinline__ bool sun_may_touch(const FrameParams& F, const float p0[3], const float p1[3]) {
@@ -218,7 +219,7 @@ __device__ __forceinline__ bool sun_may_touch(const FrameParams& F, const float 
         dc = fmaf(d, d, dc);
         size += fabsf(p0[i]) + fabsf(p1[i]) + fabsf(c);
     }
-    return !(sqrtf(dc) > sqrtf(seg) + 1.5f * (float)F.sun_R + 1e-4f * (size + (float)F.sun_R));
+    return !(sqrtf(dc) > sqrtf(seg) + 1.5f * (float)F.sun_R + F.f_sun_margin * (size + (float)F.sun_R));
 }
 
 template <class P>

@@ -146,3 +146,22 @@ def test_no_step_misses_the_sun(renderer, orc, centre, radius, fov, precision):
     both = sun & (got["what"] == abi.HIT_SUN)
     tol = 1e-6 if precision == abi.PRECISION_FP64 else 1e-3
     assert np.quantile(np.abs(got["y"][both, 1] / chk["y"][both, 1] - 1.0), 0.95) <= tol
+
+
+@pytest.mark.parametrize("turns", [1, -1000, 20000, 10 ** 6])
+def test_no_step_misses_the_sun_after_many_turns(renderer, turns):
+    """The camera's azimuth may be any number: with whole turns added to it the frame
+    is the same but for the azimuth's own rounding (10^6 turns: 10^-9 rad), and so
+    are its rays that end on a small Sun close to the camera, to two rays as above."""
+    from blackhole_b200.config import SunBody
+
+    def frame(phi):
+        return renderer.trace_rays(RenderConfig(
+            M_kg=4.3e6 * M_SUN, spin=0.6, cam=Camera(r=60.0, theta=math.radians(80.0), phi=phi, fov=0.6, yaw=0.15),
+            width=161, height=121, sqrt_spp=1, disc_r_out=20.0, sun_enabled=True,
+            sun=SunBody(centre=(45.0, 5.0, 8.0), radius=0.3), rtol=1e-9, atol=1e-11, r_escape=600.0, star_count=0,
+            quiet=True))["what"]
+
+    want, got = frame(0.0) == abi.HIT_SUN, frame(2.0 * math.pi * turns) == abi.HIT_SUN
+    assert want.sum() > 50
+    assert (want != got).sum() <= 2
