@@ -564,13 +564,14 @@ int make_frame(const bh_render_config& c, FrameParams& F, std::string& err) {
         F.jet_ck = std::pow(maxd(j.z_base, 1e-6) / j.z_sat, j.k) / std::pow(maxd(j.z_base, 1e-6) / j.z_base, j.k);
         F.jet_inv_gb = 1.0 / jet_gamma_at(j, j.z_base);
         // The profile exp(-((u - u_peak) / u_wid)^2) + spine exp(-(u / spine_wid)^2) is cut at 1e-9: both
-        // terms are below half of that (and a margin) beyond u_cut.
+        // terms are below half of that (and a margin) beyond u_cut.  Not known where the product with z^k
+        // could leave binary32's range on the way (a radius that grows like z^65 or faster).
         F.jet_f_cut = -1.f;
         if (j.k >= 0.0 && j.spine >= 0.0) {
             const double u1 = j.u_peak + j.u_wid * std::sqrt(std::log(2.2e9));
             const double u2 = j.spine_wid * std::sqrt(std::log(maxd(1.0, 2.2e9 * j.spine)));
             const double cut = 1.01 * maxd(maxd(u1, u2), 0.0) * j.R_base / std::pow(j.z_base, j.k);
-            if (std::isfinite(cut) && cut < 1e30) F.jet_f_cut = static_cast<float>(cut);
+            if (std::isfinite(cut) && cut > 1e-30 && cut < 1e30) F.jet_f_cut = static_cast<float>(cut);
         }
         powerlaw_xyz(j.alpha, F.jet_col);   // render.cpp:417
     }

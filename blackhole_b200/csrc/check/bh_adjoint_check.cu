@@ -239,6 +239,16 @@ int bhx_near_critical(const bh_render_config* cfg, int n, const int* px, const i
     return BH_OK;
 }
 
+// The frame's jet_f_cut: times |z|^k, the radius beyond which the jet's profile is
+// below its cut-off (negative: not known).
+int bhx_jet_cut(const bh_render_config* cfg, float* cut) {
+    FrameParams F;
+    std::string err;
+    const int rc = make_frame(*cfg, F, err);
+    if (rc == BH_OK) *cut = F.jet_f_cut;
+    return rc;
+}
+
 // whole_window of the star bins around column `base`.
 int bhx_star_window(int base, int half) { return whole_window(base, half, kLon) ? 1 : 0; }
 
