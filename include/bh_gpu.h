@@ -332,17 +332,20 @@ int  bh_gpu_get_launch(const bh_ctx* ctx, int precision, bh_launch_params* p);
 
 /* Autotuner: render `cfg` twice per launch shape of the search space (block
    size 64..512, rays per thread 1..8, refill threshold 8..32 idle lanes,
-   both register caps), keep the shape with the shortest trace-kernel time for
-   cfg->precision, and return it in *best (and its time in *best_ms).  Extension;
-   no counterpart in the reference. */
+   both register caps) and compare the shape with the shortest trace-kernel time
+   with no shape set, by the time of the whole call.  If the shape is faster it is
+   kept for cfg->precision; otherwise the library's own choice is (the default
+   shape, as though none had been set or tuned).  *best is the shape then in force
+   (bh_gpu_get_launch), *best_ms its trace time.  Extension; no counterpart in the
+   reference. */
 int  bh_gpu_autotune(bh_ctx* ctx, const bh_render_config* cfg, bh_launch_params* best, double* best_ms);
 
 /* The same search on a batch of frames through bh_gpu_render_batch (each
-   shape timed on the captured batch graph; *best_ms is its device time).
-   The search space: block size 64..512, rays per thread 1..8, refill
-   threshold 8..32 idle lanes (a refill claims n_idle x rays_per_thread rays,
-   8 to 256, in one atomic), both register caps.  Extension; no counterpart
-   in the reference. */
+   shape timed on the captured batch graph; *best_ms is what kernel_ms of a
+   batch is).  The search space: block size 64..512, rays per thread 1..8,
+   refill threshold 8..32 idle lanes (a refill claims n_idle x rays_per_thread
+   rays, 8 to 256, in one atomic), both register caps.  Extension; no
+   counterpart in the reference. */
 int  bh_gpu_autotune_batch(bh_ctx* ctx, const bh_render_config* cfgs, int n, bh_launch_params* best,
                            double* best_ms);
 
