@@ -31,10 +31,10 @@
 // against the spread of the neighbouring samples' same crossing; the render
 // records the crossings), and the adjoint kernel takes their edge terms
 // (weight 2 (Y_pixel - target)): edge_recorded where the render recorded the
-// steps up to the crossing, adj::edge_sample elsewhere.  It runs beside
-// reverse_kernel on a stream of its own, since both are long chains that leave
-// issue slots free: 512^2 takes 8.3 ms so and 10.9 ms with the edge terms after
-// the rays (the frame before the records: 12.2 ms; 128^2 5.6 -> 3.5 ms).
+// steps up to the crossing, adj::edge_sample elsewhere.  reverse_kernel runs
+// beside it on a second stream, since both are long chains that leave issue
+// slots free: 512^2 takes 8.3 ms so and 10.9 ms with the edge terms after the
+// rays (the frame before the records: 12.2 ms; 128^2 5.6 -> 3.5 ms).
 //
 // The edge pass covers the edges of the first two equatorial crossings (the
 // direct image of the disc and its first lensed image).  Images of order

@@ -603,7 +603,8 @@ int record_banded(bh_ctx* ctx, Plan& p, const bh_render_config* cfg, bh_xyz* out
 // frames of 256^2 to 1024^2 14.9 ms with the shading inside -> 16.2, but the
 // call 18.1 -> 16.6; 4 of 1024^2 10.1 -> 8.8; 2 of 512^2 2.71 -> 2.35; 6 of 256^2 2.27 -> 2.20.
 // Blocks of 128 threads 16.9, two batches per warp 17.1; one to five streams
-// the same.  The host, which has to wait for the call's end anyway, reads the
+// the same (on eight, some share a hardware queue with the trace's own and
+// wait for its end: 17.2).  The host, which has to wait for the call's end anyway, reads the
 // counters and launches a piece when its rays are done: with stream waits on
 // the counters, as in the row-band pipeline, a call in four ran with none of
 // them served before the trace's end (64 frames 225 instead of 194 ms; the

@@ -175,8 +175,9 @@ extern "C" int bh_gpu_trace_noalloc(int device, const bh_render_config* cfg, bh_
     const int bps = trace_blocks_per_sm(cfg->precision, tl.block_size, tl.reg_variant);
     tl.grid = sms * (bps < 1 ? 1 : bps);
     tl.deferred = mixed ? static_cast<void*>(base + kDeferredOff) : nullptr;
+    // The binary64 kernels of a mixed call run blocks of 64 under the wide cap.
     tl.block_resume = 64;
-    const int bps64 = trace_blocks_per_sm(BH_PRECISION_FP64, 128, 0);
+    const int bps64 = trace_blocks_per_sm(BH_PRECISION_FP64, 64, 1);
     tl.grid_resume = sms * (bps64 < 1 ? 1 : bps64);
     tl.resume_event = nullptr;
     tl.surfaces = (F.sun_enabled || F.ns_enabled) ? 1 : 0;

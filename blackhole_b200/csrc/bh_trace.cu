@@ -1,9 +1,8 @@
 // bh_trace.cu - The persistent trace kernels of the render path (sm_100a).
 //
 //   trace_kernel<Fp64>   every operation in binary64.
-//   trace_kernel<Mixed>  binary32 ray state, stages and right-hand side;
-//                        binary64 for the step size, the error-norm sum and
-//                        the accept/reject test, event root refinement and the
+//   trace_kernel<Mixed>  binary32 ray state, stages, right-hand side and step
+//                        control; binary64 for event root refinement and the
 //                        invariant diagnostics.  A ray that is provably falling
 //                        into the hole (moving inwards inside the innermost
 //                        photon orbit) is handed to binary64 for the plunge,
@@ -1504,9 +1503,9 @@ cudaError_t launch_t(const TraceLaunch& L, int grid, int block, cudaStream_t s, 
     A.refill = L.refill < 1 ? 1 : (L.refill > 32 ? 32 : L.refill);
     A.select = select;
     if (select == 1) {
-        // Without a list few rays are found among many looked at: refill a
-        // lane as soon as it is idle, one id at a time, so a lane tracing a ray
-        // does not hold up the search of the other 31.
+        // Without a list (the no-allocation entry) few rays are found among many
+        // looked at, one id at a time: idle lanes look on whenever a ray of their
+        // warp ends, and until the warp has one.
         A.rays_per_thread = 1;
         A.refill = L.sel_list ? 32 : 1;
     }

@@ -314,7 +314,8 @@ int  bh_gpu_trace_rays(bh_ctx* ctx, const bh_render_config* cfg,
    without jets at one sample a pixel, of 256^2 pixels a frame or more on
    average, with no launch shape set, is shaded and copied out while the rest
    is traced: kernel_ms is the device time of the trace with the shading beside
-   it and shade_ms what follows it.  Any other batch runs as one CUDA
+   it and shade_ms what follows it; the calling thread reads the rays' counters
+   over and over meanwhile, a full core for the length of the call.  Any other batch runs as one CUDA
    graph (staging copies, trace, shade, stats), captured on the first call and
    replayed while the batch shape (frame count and sizes, launch parameters,
    buffers) is unchanged; kernel_ms is then the device time of the whole graph
