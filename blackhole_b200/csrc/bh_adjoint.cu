@@ -239,13 +239,14 @@ __global__ void __launch_bounds__(kAdjBlock, kAdjBlocksPerSm) adjoint_kernel(con
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int slots = L.X.checkpoint_slots;
-    double* ck = L.ckpt + warp * slots * adj::kCkWords * 32 + lane;
+    const long long owner = warp - ((long long)gridDim.x * (kAdjBlock / 32) - L.ckpt_warps);
+    double* ck = L.ckpt + owner * slots * adj::kCkWords * 32 + lane;
     const int SS = L.frame.S * L.frame.S;
     // rays and candidates start on a warp of their own
     const unsigned long long n_rays = L.counters[11], first_cand = (n_rays + 31) & ~31ull,
                              n_stored = first_cand + L.counters[13], n_recorded = L.counters[6];
     unsigned long long replay = 0, max_int = 0, edge_steps = 0, edge_cells = 0;
-    bool stored = warp < L.ckpt_warps;       // which queue the warp takes from
+    bool stored = owner >= 0;                // which queue the warp takes from
     for (;;) {
         unsigned long long job = 0;
         if (lane == 0) job = atomicAdd(&L.counters[stored ? 14 : 0], 32ull);
@@ -363,6 +364,8 @@ reverse_kernel(const __grid_constant__ AdjointLaunch L) {
     }
 }
 
+__global__ void after_kernel() {}
+
 __global__ void __launch_bounds__(kReduceThreads)
 adjoint_reduce_kernel(const double* __restrict__ grad, const double* __restrict__ edge,
                       const unsigned char* __restrict__ high, long long n_rays, const bh_xyz* __restrict__ pixels,
@@ -418,9 +421,12 @@ cudaError_t launch_adjoint(const AdjointLaunch& L, cudaStream_t stream) {
         edge_candidates_kernel<<<(unsigned)((L.n_rays + 255) / 256), 256, 0, stream>>>(L);
         adjoint_select_kernel<<<(unsigned)((L.n_rays + 255) / 256), 256, 0, stream>>>(L);
         // The edge terms and the rays without records beside the recorded rays:
-        // long chains both, that share no output.  reverse_kernel waits until the
-        // few long chains have begun; the other way round they wait for its
-        // persistent blocks to end (512^2 9.7 against 8.4 ms).
+        // long chains both, that share no output.  The empty kernel lets the
+        // few long chains be placed first; the other way round they wait for
+        // the persistent reverse_kernel's blocks to end (512^2 9.7 against 8.4 ms).
+        // On the context's own streams that order held on each of 60 contexts;
+        // waiting for the chains' launch-completion event instead, as launch_trace
+        // does on a caller's stream, costs 1% (8.46 against 8.34 ms).
         cudaError_t e;
         const bool side = L.traj && L.side_stream;
         cudaStream_t s2 = side ? L.side_stream : stream;
@@ -428,10 +434,8 @@ cudaError_t launch_adjoint(const AdjointLaunch& L, cudaStream_t stream) {
             if ((e = cudaEventRecord(L.fork_event, stream)) != cudaSuccess) return e;
             if ((e = cudaStreamWaitEvent(s2, L.fork_event, 0)) != cudaSuccess) return e;
         }
-        if ((e = launch_started(adjoint_kernel, L.grid, L.block, kAdjShared, stream, side ? L.start_event : nullptr,
-                                L)) != cudaSuccess)
-            return e;
-        if (side && (e = cudaStreamWaitEvent(s2, L.start_event, 0)) != cudaSuccess) return e;
+        adjoint_kernel<<<L.grid, L.block, kAdjShared, stream>>>(L);
+        if (side) after_kernel<<<1, 32, 0, s2>>>();
         if (L.traj) reverse_kernel<<<L.grid_reverse, kAdjBlock, kAdjShared, s2>>>(L);
         if (side) {
             if ((e = cudaEventRecord(L.join_event, s2)) != cudaSuccess) return e;

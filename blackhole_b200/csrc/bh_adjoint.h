@@ -89,7 +89,7 @@ struct AdjointLaunch {
     int grid, block;
     int grid_reverse;                // blocks of the kernel over the recorded rays
     cudaStream_t side_stream;        // that kernel runs here, beside the edge terms and the rays without records
-    cudaEvent_t fork_event, start_event, join_event;
+    cudaEvent_t fork_event, join_event;
 };
 
 constexpr int kAdjCounters = 15;

@@ -1206,7 +1206,6 @@ static int adjoint_impl(bh_ctx* ctx, const bh_render_config* cfg, const float* t
                                                           (n_rays + block - 1) / block));
     L.side_stream = ctx->side_stream;
     L.fork_event = ctx->fork_event;
-    L.start_event = ctx->start_event;
     L.join_event = ctx->join_event;
     L.xing_r = static_cast<double*>(ctx->adj_xr.p);
     L.cand = static_cast<unsigned long long*>(ctx->adj_cand.p);
