@@ -568,7 +568,7 @@ def adjoint_leg(r, steps=3, warmup=1):
     wall = time.perf_counter() - t0
     ms = sum(dev_ms) / len(dev_ms)
     return {"workload": "adjoint_512: a=0.7, inclination 50 deg, 0.2 Eddington, r_out 25 M, 512x512, binary64; "
-                        "target rendered at a=0.75, 53 deg, 0.22, 27 M; checkpoints every 16 accepted steps",
+                        "target rendered at a=0.75, 53 deg, 0.22, 27 M; the steps the render recorded, backwards",
             "value": round(1e3 / ms, 2), "unit": "grads/s", "ms_per_grad": round(ms, 3),
             "timing": "device time of render + adjoint + reductions (CUDA events), mean of "
                       f"{steps} after {warmup} warm-up",

@@ -52,7 +52,7 @@ struct AdjointLaunch {
     double* ray_grad;                // 4 per ray, pixel-major then sample (device)
     double* ray_Y;                   // luminance per ray in the same order, or nullptr
     double* ckpt;                    // ckpt_warps * 32 * checkpoint_slots * kAdjSlotWords doubles: the stored
-                                     // states of the first ckpt_warps warps
+                                     // states of the grid's last ckpt_warps warps
     int ckpt_warps;
     const HitRecord* hits;           // the render's hit records, work order (device)
     // The rays that have a gradient (work order ids; n_rays entries): those whose
