@@ -417,11 +417,11 @@ typedef struct bh_grad4 {
     double d_r_out;          /* dLoss / d(disc_r_out): the edge term alone        */
     double kernel_ms;        /* device time of the render, adjoint, edge pass and reductions */
     long long rays;
-    long long steps;         /* accepted steps of the adjoint's forward pass      */
-    long long replayed_steps;/* accepted steps recomputed by the reverse pass     */
+    long long steps;         /* accepted steps of the rendered rays               */
+    long long replayed_steps;/* those replayed from stored states (0: each was kept) */
     long long disc_rays;
     long long sky_rays;
-    int32_t max_checkpoint_interval;
+    int32_t max_checkpoint_interval; /* most steps between stored states (0: every ray recorded) */
     int32_t reserved;
     double edge_spin;        /* the edge term's part of d_spin                    */
     double edge_inclination; /* the edge term's part of d_inclination             */
