@@ -340,11 +340,12 @@ int plan_launch(bh_ctx* ctx, std::vector<FrameParams>& frames, bh_xyz* d_pixels,
     if ((rc = ensure(ctx, ctx->partials, static_cast<size_t>(n) * shade_grid * sizeof(double))) != BH_OK)
         return rc;
     if ((rc = ensure(ctx, ctx->fstats, n * sizeof(FrameStats))) != BH_OK) return rc;
-    bool any_jet = false, any_surface = false, any_near_critical = false;
+    bool any_jet = false, any_surface = false, any_near_critical = false, any_expanded = false;
     for (int i = 0; i < n; ++i) {
         any_jet = any_jet || frames[i].jet_enabled;
         any_near_critical = any_near_critical || frames[i].fp64_near_critical;
         any_surface = any_surface || frames[i].sun_enabled || frames[i].ns_enabled;
+        any_expanded = any_expanded || !frames[i].factored_delta;
     }
     if (any_jet && (rc = ensure(ctx, ctx->jet, static_cast<size_t>(rays) * sizeof(double))) != BH_OK) return rc;
     if (p.mixed && (rc = ensure(ctx, ctx->deferred, static_cast<size_t>(rays) * deferred_record_bytes())) != BH_OK)
@@ -424,6 +425,7 @@ int plan_launch(bh_ctx* ctx, std::vector<FrameParams>& frames, bh_xyz* d_pixels,
     tl.resume_event = timed ? ctx->ev[3] : nullptr;
     tl.jet = any_jet ? static_cast<double*>(ctx->jet.p) : nullptr;
     tl.surfaces = any_surface ? 1 : 0;
+    tl.expanded = any_expanded ? 1 : 0;
     if (p.mixed && any_near_critical) {
         // Near-critical rays in binary64 beside the binary32 kernel, on as
         // many blocks as fit: those without a ray end at once.

@@ -49,6 +49,7 @@ struct TraceLaunch {
     int* xing_step;
     double* disc_end;
     int surfaces;                    // 1 when a frame of the launch has the Sun or a neutron star
+    int expanded;                    // 1 when a frame of the launch has a^2 >= 1 (Delta has no pair of roots)
     // Mixed precision: near-critical rays (escaping rays that circle close to
     // the photon shell) traced by a binary64 kernel of grid_side blocks of 64
     // on `stream`, beside the binary32 kernel on side_stream (fork_event and

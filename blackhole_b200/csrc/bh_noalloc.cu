@@ -181,6 +181,7 @@ extern "C" int bh_gpu_trace_noalloc(int device, const bh_render_config* cfg, bh_
     tl.grid_resume = sms * (bps64 < 1 ? 1 : bps64);
     tl.resume_event = nullptr;
     tl.surfaces = (F.sun_enabled || F.ns_enabled) ? 1 : 0;
+    tl.expanded = F.factored_delta ? 0 : 1;
     // Near-critical rays in binary64 as the context API traces them, here
     // before the binary32 kernel on the caller's stream (no stream of our own).
     tl.near_critical = F.fp64_near_critical;

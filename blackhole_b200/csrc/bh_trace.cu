@@ -159,8 +159,11 @@ struct Lane {
 };
 
 // The constants of Delta: binary32 lanes hold r_+ and r_- as exact two-term
-// sums (or use the expanded form where a^2 >= 1); binary64 ones
-// (r - rp_hi)(r - rm_hi) + rp_lo for every spin.
+// sums, binary64 ones (r - rp_hi)(r - rm_hi) + rp_lo with rp_lo = 0.  Where
+// a^2 >= 1 both use the expanded form; the binary64 kernels built without it
+// still hold (r - 1)^2 + (a^2 - 1) here and are not launched on such frames.
+// (Without rp_lo, edge_on 1024x1024 in binary64 takes 12.19 ms instead of
+// 12.27 and a 256x256 Kerr frame 1.635 instead of 1.620: left as it is.)
 template <class P>
 __device__ __forceinline__ void set_horizons(const FrameParams& F, Lane<P>& L) {
     using R = typename P::R;
@@ -270,8 +273,10 @@ __device__ __forceinline__ u64 mul2(u64 a, u64 b) {
 // fused is written out, so that every kernel and both forms of the stages
 // round alike; FIRST is a ray's first stage, where r^2 is rounded before it
 // enters Sigma and r^2 + a^2 (the choices the compiler made when they were
-// left to it: the frames keep their bits).
-template <class P, bool FIRST = false>
+// left to it: the frames keep their bits).  ROUND2: r^2 is rounded before it
+// enters the expanded Delta (a^2 >= 1): a ray's first stage, and the second of the
+// kernels without the jet.
+template <class P, bool FIRST = false, bool ROUND2 = FIRST>
 __device__ __forceinline__ void rhs_sc(const Lane<P>& L, float r, float sn, float cs, float pr, float pth, float* d,
                                        Aux<P>* aux) {
     static_assert(P::kMixed, "the binary64 right-hand side is rhs64");
@@ -280,7 +285,7 @@ __device__ __forceinline__ void rhs_sc(const Lane<P>& L, float r, float sn, floa
     const float r2 = __fmul_rn(r, r);
     const float S = FIRST ? __fmaf_rn(L.a2R, cs2, r2) : __fmaf_rn(r, r, __fmul_rn(L.a2R, cs2));
     const float D = L.factored ? __fmul_rn((r - L.rp_hi) - L.rp_lo, (r - L.rm_hi) - L.rm_lo)
-                               : __fadd_rn(FIRST ? __fmaf_rn(-2.f, r, r2) : __fmaf_rn(r, r, -2.f * r), L.a2R);
+                               : __fadd_rn(ROUND2 ? __fmaf_rn(-2.f, r, r2) : __fmaf_rn(r, r, -2.f * r), L.a2R);
     const float SD = __fmul_rn(S, D);
     const float inv = P::rcp(__fmul_rn(SD, sn2));
     const float iS = __fmul_rn(__fmul_rn(inv, D), sn2), iD = __fmul_rn(__fmul_rn(inv, S), sn2);
@@ -319,6 +324,15 @@ __device__ __noinline__ void stage_sincos_far(typename P::R th, typename P::R* s
     P::sc(th, sn, cs);
 }
 
+// Whether stage S (2..7) of a binary64 kernel rounds r^2 before it enters Sigma
+// and r^2 + a^2 (rhs64's SQUARE), and before it enters the expanded Delta (ROUND2).
+__host__ __device__ constexpr bool square64(int S, bool jet, bool resume) {
+    return (S == 2 && !jet) || (S < 7 && resume);
+}
+__host__ __device__ constexpr bool round64(int S, bool jet, bool resume) {
+    return S == 2 || (S == 3 && !jet) || (resume && (S < 7 || !jet));
+}
+
 // The binary64 right-hand side, the derivatives of rhs_sc, for |sn| >= 1e-9
 // (the caller's business).  The products that are fused are written out, here
 // and in the stage sums: a ray close to the photon shell amplifies the last
@@ -326,15 +340,19 @@ __device__ __noinline__ void stage_sincos_far(typename P::R th, typename P::R* s
 // SQUARE: r^2 is rounded before it enters Sigma and r^2 + a^2 (a ray's first
 // stage, the second stage of the kernels without the jet, and stages two to
 // six of the pass that finishes a mixed frame's rays: the choices the compiler
-// made when they were left to it).  Delta = (r - r_+)(r - r_-) + dD, dD = 0;
-// for a^2 >= 1, where there is no pair of horizons, (r - 1)^2 + (a^2 - 1).
-template <bool SQUARE>
+// made when they were left to it).  Delta = (r - r_+)(r - r_-); in EXPANDED
+// kernels, and there for a^2 >= 1 alone, r^2 - 2 r + a^2 in two roundings (three
+// with ROUND2), like the reference: at a^2 = 1 the rays that fall in creep to a
+// double root, and their steps and how they end follow the last bits of Delta.
+template <bool SQUARE, bool EXPANDED, bool ROUND2>
 __device__ __forceinline__ void rhs64(const Lane<Fp64>& L, double r, double sn, double cs, double pr, double pth,
                                       double* d, Aux<Fp64>* aux) {
     const double sn2 = __dmul_rn(sn, sn), cs2 = __dmul_rn(cs, cs);
     const double r2 = __dmul_rn(r, r);
     const double S = SQUARE ? __fma_rn(L.a2R, cs2, r2) : __fma_rn(r, r, __dmul_rn(L.a2R, cs2));
-    const double D = __fma_rn(r - L.rp_hi, r - L.rm_hi, L.rp_lo);
+    double D;
+    if (!EXPANDED || L.factored) D = __fma_rn(r - L.rp_hi, r - L.rm_hi, L.rp_lo);
+    else D = __dadd_rn(ROUND2 ? __fma_rn(-2.0, r, r2) : __fma_rn(r, r, -2.0 * r), L.a2R);
     const double SD = __dmul_rn(S, D);
     const double inv = rcp_nr(__dmul_rn(SD, sn2));
     const double iS = __dmul_rn(__dmul_rn(inv, D), sn2), iD = __dmul_rn(__dmul_rn(inv, S), sn2);
@@ -365,11 +383,11 @@ __device__ __forceinline__ void rhs64(const Lane<Fp64>& L, double r, double sn, 
 }
 
 // rhs64 with the metric's clamp of sin(th) (kerr.h:51).
-template <bool SQUARE>
+template <bool SQUARE, bool EXPANDED, bool ROUND2>
 __device__ __forceinline__ void rhs64_clamped(const Lane<Fp64>& L, double r, double sn, double cs, double pr,
                                               double pth, double* d, Aux<Fp64>* aux) {
     if (fabs(sn) < 1e-9) sn = (sn < 0.0) ? -1e-9 : 1e-9;
-    rhs64<SQUARE>(L, r, sn, cs, pr, pth, d, aux);
+    rhs64<SQUARE, EXPANDED, ROUND2>(L, r, sn, cs, pr, pth, d, aux);
 }
 
 // The RHS at a fresh angle (full sincos).
@@ -380,7 +398,7 @@ __device__ __forceinline__ void rhs(const Lane<P>& L, typename P::R r, typename 
     typename P::R sn, cs;
     P::sc(th, &sn, &cs);
     if constexpr (P::kMixed) rhs_sc<P, FIRST>(L, r, sn, cs, pr, pth, d, aux);
-    else rhs64_clamped<FIRST>(L, r, sn, cs, pr, pth, d, aux);
+    else rhs64_clamped<FIRST, true, FIRST>(L, r, sn, cs, pr, pth, d, aux);
 }
 
 // The binary64 attempt's stages k_2..k_7, the step's end yn and stage 7's
@@ -416,7 +434,7 @@ __device__ __forceinline__ double stage_sum64(const Lane<Fp64>& L, double h, int
 // clamped.  attempt() runs the stages in one straight line without either
 // and takes this form for the lanes that needed one (none in 10^5 attempts on
 // the measured scenes).
-template <int S, bool SQUARE2, bool SQUARE36>
+template <int S, bool JET, bool RESUME, bool EXPANDED>
 __device__ __forceinline__ void stage64_general(const Lane<Fp64>& L, Stages64* o) {
     double t[6];
     for (int i = 0; i < 6; ++i)
@@ -425,24 +443,25 @@ __device__ __forceinline__ void stage64_general(const Lane<Fp64>& L, Stages64* o
     double sn, cs;
     if (fabs(dth) <= kMaxShift) shift_sincos(L.sn0, L.c0, dth, &sn, &cs);
     else stage_sincos_far<Fp64>(t[2], &sn, &cs);
-    rhs64_clamped<(S == 2) ? SQUARE2 : (S < 7 && SQUARE36)>(L, t[1], sn, cs, t[4], t[5], o->k[S - 2], S < 7 ? nullptr : &o->ax7);
+    rhs64_clamped<square64(S, JET, RESUME), EXPANDED, round64(S, JET, RESUME)>(L, t[1], sn, cs, t[4], t[5], o->k[S - 2],
+                                                                              S < 7 ? nullptr : &o->ax7);
     if (S == 7)
         for (int i = 0; i < 6; ++i) o->yn[i] = t[i];
 }
-template <bool SQUARE2, bool SQUARE36>
+template <bool JET, bool RESUME, bool EXPANDED>
 __device__ __noinline__ void stages64_general(const Lane<Fp64>* L, Stages64* o) {
-    stage64_general<2, SQUARE2, SQUARE36>(*L, o);
-    stage64_general<3, SQUARE2, SQUARE36>(*L, o);
-    stage64_general<4, SQUARE2, SQUARE36>(*L, o);
-    stage64_general<5, SQUARE2, SQUARE36>(*L, o);
-    stage64_general<6, SQUARE2, SQUARE36>(*L, o);
-    stage64_general<7, SQUARE2, SQUARE36>(*L, o);
+    stage64_general<2, JET, RESUME, EXPANDED>(*L, o);
+    stage64_general<3, JET, RESUME, EXPANDED>(*L, o);
+    stage64_general<4, JET, RESUME, EXPANDED>(*L, o);
+    stage64_general<5, JET, RESUME, EXPANDED>(*L, o);
+    stage64_general<6, JET, RESUME, EXPANDED>(*L, o);
+    stage64_general<7, JET, RESUME, EXPANDED>(*L, o);
 }
 
 // The RHS at a stage angle th of a binary32 lane, from the sin/cos of the
 // step's base angle L.y[2] by angle addition (full sincos when the stage
 // moved th by more than kMaxShift).
-template <class P>
+template <class P, bool ROUND2 = false>
 __device__ __forceinline__ void rhs_stage(const Lane<P>& L, typename P::R r, typename P::R th,
                                           typename P::R pr, typename P::R pth, typename P::R* d) {
     using R = typename P::R;
@@ -450,7 +469,7 @@ __device__ __forceinline__ void rhs_stage(const Lane<P>& L, typename P::R r, typ
     R sn, cs;
     if (fabs(dth) <= R(kMaxShift)) shift_sincos(L.sn0, L.c0, dth, &sn, &cs);
     else stage_sincos_far<P>(th, &sn, &cs);
-    rhs_sc<P>(L, r, sn, cs, pr, pth, d, nullptr);
+    rhs_sc<P, false, ROUND2>(L, r, sn, cs, pr, pth, d, nullptr);
 }
 
 
@@ -523,12 +542,13 @@ __device__ __forceinline__ void stage_sum32(const Lane<P>& L, float h, const flo
 struct Stages32 {
     float k[5][6];
 };
+template <bool ROUND2>
 __device__ __noinline__ void stages32_general(const Lane<Mixed>* Lp, Stages32* o) {
     const Lane<Mixed>& L = *Lp;
     const float h = L.h;
     float t[6];
     stage_sum32<2>(L, h, nullptr, nullptr, nullptr, nullptr, t);
-    rhs_stage<Mixed>(L, t[1], t[2], t[4], t[5], o->k[0]);
+    rhs_stage<Mixed, ROUND2>(L, t[1], t[2], t[4], t[5], o->k[0]);
     stage_sum32<3>(L, h, o->k[0], nullptr, nullptr, nullptr, t);
     rhs_stage<Mixed>(L, t[1], t[2], t[4], t[5], o->k[1]);
     stage_sum32<4>(L, h, o->k[0], o->k[1], nullptr, nullptr, t);
@@ -712,9 +732,12 @@ __device__ __noinline__ int near_critical(const FrameParams& F, const double y8[
 // What a trace kernel is compiled with beyond the integration and the
 // horizon, disc and escape events: nothing; the Sun's and the neutron star's
 // surface tests and the record of equatorial crossings; the crossing record
-// alone (the discrete adjoint's render).
-enum { kSurfNone = 0, kSurfAll = 1, kSurfCrossings = 2 };
-constexpr int kFamily = 4;   // trace kernels of a precision and register cap
+// alone (the discrete adjoint's render); the surface tests and Delta's expanded
+// form (binary64 kernels of a launch with a frame of a^2 >= 1).
+enum { kSurfNone = 0, kSurfAll = 1, kSurfCrossings = 2, kSurfExpanded = 3 };
+template <int SURF>
+constexpr bool kSurfaces = SURF == kSurfAll || SURF == kSurfExpanded;
+constexpr int kFamily = 6;   // trace kernels of a precision and register cap
 
 // Lane set-up from an initial photon (fresh ray) or a deferred state.
 template <class P, bool JET, int SURF, bool RESUME>
@@ -814,12 +837,12 @@ __device__ bool start_ray(const TraceArgs& A, Lane<P>& L, long long id) {
     } else {
         double sn, cs;
         stage_sincos_far<P>(L.y[2], &sn, &cs);
-        rhs64_clamped<true>(L, L.y[1], sn, cs, L.y[4], L.y[5], L.k1, &ax);
+        rhs64_clamped<true, SURF == kSurfExpanded, true>(L, L.y[1], sn, cs, L.y[4], L.y[5], L.k1, &ax);
     }
     L.c0 = ax.cs;
     L.sn0 = ax.sn;
     if constexpr (JET) cylindrical(L, (float)L.y[1], (float)L.sn0, (float)L.c0, &L.jet_z, &L.jet_rho);
-    if constexpr (SURF == kSurfAll) {
+    if constexpr (kSurfaces<SURF>) {
         if (F.sun_enabled) cartesian32(L, (float)L.y[1], (float)L.sn0, (float)L.c0, (float)L.y[3], L.sun_at);
     }
     return true;
@@ -860,27 +883,28 @@ __device__ bool attempt(const TraceArgs& A, Lane<P>& L) {
         // frame 2.86 -> 2.62 ms with the loop of trace_kernel, bits unchanged.
         float t[6];
         bool far = false;
-        auto stage = [&](float* k) {
+        auto stage = [&](float* k, auto round2) {
             const float dth = t[2] - L.y[2];
             float sn, cs;
             shift_sincos(L.sn0, L.c0, dth, &sn, &cs);
             far = far || !(fabsf(dth) <= float(kMaxShift));
-            rhs_sc<P>(L, t[1], sn, cs, t[4], t[5], k, nullptr);
+            rhs_sc<P, false, decltype(round2)::value>(L, t[1], sn, cs, t[4], t[5], k, nullptr);
         };
+        constexpr std::integral_constant<bool, false> later{};
         stage_sum32<2>(L, h, k2, k3, k4, k5, t);
-        stage(k2);
+        stage(k2, std::integral_constant<bool, !JET>{});
         stage_sum32<3>(L, h, k2, k3, k4, k5, t);
-        stage(k3);
+        stage(k3, later);
         stage_sum32<4>(L, h, k2, k3, k4, k5, t);
-        stage(k4);
+        stage(k4, later);
         stage_sum32<5>(L, h, k2, k3, k4, k5, t);
-        stage(k5);
+        stage(k5, later);
         stage_sum32<6>(L, h, k2, k3, k4, k5, t);
-        stage(k6);
+        stage(k6, later);
         if (far) {
             const Lane<P> Lc = L;
             Stages32 o;
-            stages32_general(&Lc, &o);
+            stages32_general<!JET>(&Lc, &o);
             #pragma unroll
             for (int i = 0; i < 6; ++i) {
                 k2[i] = o.k[0][i]; k3[i] = o.k[1][i]; k4[i] = o.k[2][i];
@@ -900,30 +924,31 @@ __device__ bool attempt(const TraceArgs& A, Lane<P>& L) {
         // below.  1024^2 edge-on frame 13.6 -> 12.2 ms, with the loop of
         // trace_kernel and Delta's constant; bits unchanged.
         double t[6];
-        auto stage = [&](double* k, auto square) {
+        auto stage = [&](double* k, auto number) {
+            constexpr int S = decltype(number)::value;
             const double dth = t[2] - L.y[2];
             double sn, cs;
             shift_sincos(L.sn0, L.c0, dth, &sn, &cs);
             dth_hi = max(dth_hi, abs_hi(dth));
             sn_hi = min(sn_hi, abs_hi(sn));
-            rhs64<decltype(square)::value>(L, t[1], sn, cs, t[4], t[5], k, nullptr);
+            rhs64<square64(S, JET, RESUME), SURF == kSurfExpanded, round64(S, JET, RESUME)>(L, t[1], sn, cs, t[4], t[5],
+                                                                                         k, nullptr);
         };
-        constexpr std::integral_constant<bool, RESUME> later{};
         #pragma unroll
         for (int i = 0; i < 6; ++i) t[i] = stage_sum64<2>(L, h, i, k2, k3, k4, k5, k6);
-        stage(k2, std::integral_constant<bool, !JET || RESUME>{});
+        stage(k2, std::integral_constant<int, 2>{});
         #pragma unroll
         for (int i = 0; i < 6; ++i) t[i] = stage_sum64<3>(L, h, i, k2, k3, k4, k5, k6);
-        stage(k3, later);
+        stage(k3, std::integral_constant<int, 3>{});
         #pragma unroll
         for (int i = 0; i < 6; ++i) t[i] = stage_sum64<4>(L, h, i, k2, k3, k4, k5, k6);
-        stage(k4, later);
+        stage(k4, std::integral_constant<int, 4>{});
         #pragma unroll
         for (int i = 0; i < 6; ++i) t[i] = stage_sum64<5>(L, h, i, k2, k3, k4, k5, k6);
-        stage(k5, later);
+        stage(k5, std::integral_constant<int, 5>{});
         #pragma unroll
         for (int i = 0; i < 6; ++i) t[i] = stage_sum64<6>(L, h, i, k2, k3, k4, k5, k6);
-        stage(k6, later);
+        stage(k6, std::integral_constant<int, 6>{});
         #pragma unroll
         for (int i = 0; i < 6; ++i) yn[i] = stage_sum64<7>(L, h, i, k2, k3, k4, k5, k6);
     }
@@ -941,13 +966,14 @@ __device__ bool attempt(const TraceArgs& A, Lane<P>& L) {
         shift_sincos(L.sn0, L.c0, dth, &sn, &cs);
         dth_hi = max(dth_hi, abs_hi(dth));
         sn_hi = min(sn_hi, abs_hi(sn));
-        rhs64<false>(L, yn[1], sn, cs, yn[4], yn[5], k7, &ax7);
+        rhs64<square64(7, JET, RESUME), SURF == kSurfExpanded, round64(7, JET, RESUME)>(L, yn[1], sn, cs, yn[4], yn[5],
+                                                                                     k7, &ax7);
         if (dth_hi >= kMaxShiftHi || sn_hi <= kMinSinHi) {
             // the lane and the stages through stack copies, so that they
             // stay in registers on the common path
             const Lane<P> Lc = L;
             Stages64 o;
-            stages64_general<!JET || RESUME, RESUME>(&Lc, &o);
+            stages64_general<JET, RESUME, SURF == kSurfExpanded>(&Lc, &o);
             #pragma unroll
             for (int i = 0; i < 6; ++i) {
                 k2[i] = o.k[0][i]; k3[i] = o.k[1][i]; k4[i] = o.k[2][i];
@@ -1096,7 +1122,7 @@ __device__ bool attempt(const TraceArgs& A, Lane<P>& L) {
     // Fraction of the step the jet integral covers: up to an occluding
     // event, all of it otherwise; < 0: none (render.cpp:107-122, 165-244).
     double s_jet = 1.0;
-    if (SURF == kSurfAll && F.ns_enabled && rn <= F.ns_R) {
+    if (kSurfaces<SURF> && F.ns_enabled && rn <= F.ns_R) {
         // neutron-star surface (render.cpp:158-169)
         const DenseC cr = coef(1);
         what = BH_HIT_STAR;
@@ -1133,13 +1159,13 @@ __device__ bool attempt(const TraceArgs& A, Lane<P>& L) {
     }
     float sun1[3] = {0.f, 0.f, 0.f};
     bool sun_near = false;
-    if constexpr (SURF == kSurfAll) {
+    if constexpr (kSurfaces<SURF>) {
         if (F.sun_enabled) {
             cartesian32(L, (float)yn[1], (float)ax7.sn, (float)ax7.cs, (float)yn[3], sun1);
             sun_near = sun_may_touch(F, L.sun_at, sun1);
         }
     }
-    if (SURF == kSurfAll && what < 0 && sun_near) {
+    if (kSurfaces<SURF> && what < 0 && sun_near) {
         // The Sun (render.cpp:201-241): probe the dense geodesic, then bisect.
         const double a = F.a;
         auto cart = [&](double r, double th, double ph, double q[3]) {
@@ -1219,7 +1245,7 @@ __device__ bool attempt(const TraceArgs& A, Lane<P>& L) {
         L.jet_z = jet_z1;
         L.jet_rho = jet_rho1;
     }
-    if constexpr (SURF == kSurfAll) {
+    if constexpr (kSurfaces<SURF>) {
         #pragma unroll
         for (int i = 0; i < 3; ++i) L.sun_at[i] = sun1[i];
     }
@@ -1567,13 +1593,20 @@ __global__ void classify_kernel(const FrameParams* __restrict__ frames, const lo
 
 // The kernels of a precision and register cap: plain, with the surface tests
 // and the crossing record, with those and the jet's emission, with the
-// crossing record alone.
+// crossing record alone; in binary64 the second and third with Delta's
+// expanded form too.
 template <class P, int MAXREG>
 void family(const void* k[kFamily]) {
     k[0] = (const void*)trace_kernel<P, MAXREG, false, kSurfNone, false>;
     k[1] = (const void*)trace_kernel<P, MAXREG, false, kSurfAll, false>;
     k[2] = (const void*)trace_kernel<P, MAXREG, true, kSurfAll, false>;
     k[3] = (const void*)trace_kernel<P, MAXREG, false, kSurfCrossings, false>;
+    k[4] = k[1];
+    k[5] = k[2];
+    if constexpr (!P::kMixed) {
+        k[4] = (const void*)trace_kernel<P, MAXREG, false, kSurfExpanded, false>;
+        k[5] = (const void*)trace_kernel<P, MAXREG, true, kSurfExpanded, false>;
+    }
 }
 
 void kernels_of(int precision, int variant, const void* k[kFamily]) {
@@ -1590,7 +1623,9 @@ void kernels_of(int precision, int variant, const void* k[kFamily]) {
 // of launches with the Sun or a neutron star test for the surfaces and record
 // the crossings, those of the adjoint's render record the crossings alone
 // (without the surface tests' code: 1.3% per gradient); the others are
-// compiled without that code.
+// compiled without that code.  Launches with a frame of a^2 >= 1 run kernels
+// with Delta's expanded form and all the rest, so that the others' right-hand
+// side has no test of the frame.
 template <bool JET, int SURF>
 cudaError_t launch_fp64(const TraceLaunch& L, int grid, int block, int variant, cudaStream_t s) {
     return variant ? launch_t<Fp64, kRegFp64Wide, JET, SURF>(L, grid, block, s)
@@ -1644,8 +1679,15 @@ cudaError_t launch_trace_t(const TraceLaunch& L, cudaStream_t stream) {
         // not certain: on a process's first context and stream the 1024^2 frame
         // took 3.2 ms, on the others 2.6; now 2.6 on all.
         if (side && (e = cudaStreamWaitEvent(L.side_stream, L.start_event, 0)) != cudaSuccess) return e;
-        e = L.reg_variant ? launch_t<Mixed, kRegMixedWide, JET, SURF>(L, L.grid, L.block_size, s32, sel)
-                          : launch_t<Mixed, kRegMixed, JET, SURF>(L, L.grid, L.block_size, s32, sel);
+        // (binary32 kernels hold both forms of Delta)
+        auto launch32 = [&](auto surf) {
+            constexpr int kSurf = decltype(surf)::value;
+            return L.reg_variant ? launch_t<Mixed, kRegMixedWide, JET, kSurf>(L, L.grid, L.block_size, s32, sel)
+                                 : launch_t<Mixed, kRegMixed, JET, kSurf>(L, L.grid, L.block_size, s32, sel);
+        };
+        if constexpr (SURF != kSurfExpanded) e = launch32(std::integral_constant<int, SURF>{});
+        else if (JET || L.surfaces) e = launch32(std::integral_constant<int, kSurfAll>{});
+        else e = launch32(std::integral_constant<int, JET ? kSurfAll : kSurfNone>{});
         if (e != cudaSuccess) return e;
         if (side) {
             if ((e = cudaEventRecord(L.join_event, L.side_stream)) != cudaSuccess) return e;
@@ -1674,7 +1716,8 @@ cudaError_t launch_eval_rhs(int precision, const FrameParams* d_frame, const dou
 
 cudaError_t launch_trace(const TraceLaunch& L, cudaStream_t stream) {
     cudaError_t e;
-    if (L.jet) e = launch_trace_t<true, kSurfAll>(L, stream);
+    if (L.expanded) e = L.jet ? launch_trace_t<true, kSurfExpanded>(L, stream) : launch_trace_t<false, kSurfExpanded>(L, stream);
+    else if (L.jet) e = launch_trace_t<true, kSurfAll>(L, stream);
     else if (L.surfaces) e = launch_trace_t<false, kSurfAll>(L, stream);
     else if (L.xing) e = launch_trace_t<false, kSurfCrossings>(L, stream);
     else e = launch_trace_t<false, kSurfNone>(L, stream);

@@ -165,3 +165,46 @@ def test_no_step_misses_the_sun_after_many_turns(renderer, turns):
     want, got = frame(0.0) == abi.HIT_SUN, frame(2.0 * math.pi * turns) == abi.HIT_SUN
     assert want.sum() > 50
     assert (want != got).sum() <= 2
+
+
+@pytest.mark.parametrize("spin", [1.0, -1.0, 1.2])
+def test_expanded_delta_is_rounded_like_the_reference(renderer, spin):
+    """Without a pair of horizons Delta = r^2 - 2 r + a^2, in the reference's
+    rounded steps: close to r = 1 at a^2 = 1 what is left is the roundings, and the
+    rays that fall in follow it.  From dr / dlambda = Delta p_r / Sigma (a product of
+    six rounded factors): Delta is one of the two values that r^2, rounded or
+    exact, less 2 r, rounded, plus a^2, rounded, can have."""
+    from fractions import Fraction
+
+    rng = np.random.default_rng(5)
+    n = 200
+    y = np.zeros((n, 8))
+    y[:, 1] = 1.0 + np.exp(rng.uniform(math.log(1.5e-8), math.log(3.0), n))
+    y[:, 2] = 1.1
+    y[:, 4], y[:, 5], y[:, 6], y[:, 7] = -1.0, 1.0, 0.3, 0.5
+    cfg = RenderConfig(spin=spin, cam=Camera(r=50.0, theta=1.0), width=4, height=4, disc_enabled=False, star_count=0,
+                       quiet=True)
+    got = renderer.eval(cfg, abi.EVAL_RHS, y)[:, 1]
+    a2 = spin * spin
+    cs = math.cos(1.1)
+    for r, d in zip(y[:, 1], got):
+        exact = float(Fraction(r) ** 2 - 2 * Fraction(r)) + a2
+        rounded = float(Fraction(r * r) - 2 * Fraction(r)) + a2
+        want = [v / (r * r + a2 * cs * cs) for v in (exact, rounded) if v != 0.0]
+        assert not want or min(abs(d / w - 1.0) for w in want) <= 16 * 2.0 ** -53, (r, d, want)
+
+
+@pytest.mark.parametrize("precision", [abi.PRECISION_FP64, abi.PRECISION_MIXED])
+def test_a_batch_of_spins_on_both_sides_of_one_equals_its_frames(precision):
+    """A launch with a frame of a^2 >= 1 runs other binary64 kernels for all of its
+    frames: bit for bit the single frames."""
+    from blackhole_b200 import Renderer
+
+    with Renderer(0) as r:
+        cfgs = [RenderConfig(M_kg=4.3e6 * M_SUN, spin=s, cam=Camera(r=30.0, theta=th, fov=0.8), width=61, height=37,
+                             disc_r_out=20.0, r_escape=60.0, star_count=1000, max_steps=2000, quiet=True,
+                             precision=precision)
+                for s, th in ((0.9, 1.0), (1.0, 1.2), (0.0, 0.02), (1.2, 0.5), (-0.998, 1.5))]
+        batch = r.render_batch(cfgs)
+        for c, px in zip(cfgs, batch):
+            assert np.array_equal(px, r.render(c), equal_nan=True), c.spin
